@@ -51,7 +51,7 @@ def build_reference(ref: str | None = None) -> bool:
     """Compile the reference's own CPU models / evaluators (only where the
     reference sources exist)."""
     ref = ref or reference_dir()
-    if not os.path.isdir(ref):
+    if not os.path.isfile(os.path.join(ref, "CUDAKernel", "src", "GeliosphereModel.cu")):
         return False
     subprocess.run(["make", "-s", "-C", HERE, "ref", "REF=" + ref], check=True)
     return True
