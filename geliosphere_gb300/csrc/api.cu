@@ -157,22 +157,43 @@ __global__ void k_prepare(const gelio_sim_params *__restrict__ p, int n, SimDev 
     sims[i] = s;
   }
   __syncthreads();
-  if (threadIdx.x < 4) {
-    const int m = threadIdx.x;
-    int c = 0;
-    unsigned long long acc = 0;
+  // warp m groups model m: its simulations in order, then the prefix sums of
+  // their segments, 32 at a time
+  const int m = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (m < 4) {
     int *idx = g.sim_idx + (size_t)m * n;
-    unsigned long long *pre = g.prefix + (size_t)m * (n + 1);
-    for (int i = 0; i < n; ++i) {
-      if (p[i].model == m) {
-        idx[c] = i;
-        pre[c] = acc;
-        acc += (unsigned long long)(p[i].n_particles > 0 ? p[i].n_particles : 0);
-        ++c;
-      }
+    unsigned long long *pre = g.prefix + (size_t)m * ((size_t)n * g.segs + 1);
+    int c = 0;
+    for (int i0 = 0; i0 < n; i0 += 32) {
+      const bool mine = i0 + lane < n && p[i0 + lane].model == m;
+      const unsigned b = __ballot_sync(kFull, mine);
+      if (mine) idx[c + __popc(b & lanemask_lt())] = i0 + lane;
+      c += __popc(b);
     }
-    pre[c] = acc;
-    ctl->group_count[m] = (unsigned long long)c;
+    __syncwarp();
+    const int ne = c * g.segs;
+    unsigned long long acc = 0;
+    for (int e0 = 0; e0 < ne; e0 += 32) {
+      const int e = e0 + lane;
+      unsigned long long v = 0;
+      if (e < ne) {
+        const long long np = p[idx[e % c]].n_particles;
+        const unsigned long long cnt = np > 0 ? (unsigned long long)np : 0ull;
+        v = segment_first(cnt, e / c + 1, g.segs) - segment_first(cnt, e / c, g.segs);
+      }
+      unsigned long long inc = v;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long x = __shfl_up_sync(kFull, inc, d);
+        if (lane >= d) inc += x;
+      }
+      if (e < ne) pre[e] = acc + inc - v;
+      acc += __shfl_sync(kFull, inc, 31);
+    }
+    if (lane == 0) {
+      pre[ne] = acc;
+      ctl->group_count[m] = (unsigned long long)c;
+    }
   }
 }
 
@@ -457,7 +478,8 @@ static int ensure_sims(gelio_ctx *c, int n) {
   if (e == cudaSuccess) e = dev_malloc(&sims, sizeof(SimDev) * cap);
   if (e == cudaSuccess) e = dev_malloc(&tables, sizeof(float) * GELIO_GRID_MAX * cap);
   if (e == cudaSuccess) e = dev_malloc(&gsim, sizeof(int) * 4 * cap);
-  if (e == cudaSuccess) e = dev_malloc(&gpre, sizeof(unsigned long long) * 4 * (cap + 1));
+  if (e == cudaSuccess)
+    e = dev_malloc(&gpre, sizeof(unsigned long long) * 4 * ((cap > kMaxSegEntries ? cap : kMaxSegEntries) + 1));
   if (e != cudaSuccess) {
     cudaFree(params); cudaFree(sims); cudaFree(tables); cudaFree(gsim); cudaFree(gpre);
     return map_cuda(e);
@@ -645,7 +667,7 @@ static int enqueue_run(gelio_ctx *c, int n, const gelio_run_opts *o, double *d_o
   GELIO_TRY(grow(c->d_part, c->part_bytes, (size_t)n_slices * n * kSpecDoubles * 8));
   GELIO_TRY(cudaMemsetAsync(c->d_ctl, 0, sizeof(Control), st));
   GELIO_TRY(cudaMemsetAsync(c->d_part, 0, (size_t)n_slices * n * kSpecDoubles * 8, st));
-  Groups g{c->d_gsim, c->d_gpre};
+  Groups g{c->d_gsim, c->d_gpre, ticket_segments(n)};
   k_prepare<<<1, 256, 0, st>>>(c->d_params, n, c->d_sims, c->d_tables, g, c->d_ctl);
   GELIO_TRY(cudaGetLastError());
   KArgs a{};
@@ -694,6 +716,7 @@ static int enqueue_run(gelio_ctx *c, int n, const gelio_run_opts *o, double *d_o
     if (rc != GELIO_OK) return rc;
     a.smem_slots = s.smem_slots;
     a.refill = s.refill;
+    a.ctas_per_sm = s.blocks_per_sm;
     GELIO_TRY(launch_model(m, true, variant, s.grid, s.block, s.smem, st, a));
     if (!have_first) { first = s; have_first = true; }
   }
@@ -886,7 +909,7 @@ int32_t gelio_replay(gelio_ctx *c, const gelio_sim_params *sim, int64_t first, i
   GELIO_TRY(cudaMemcpyAsync(c->d_params, sim, sizeof(gelio_sim_params), cudaMemcpyHostToDevice, st));
   GELIO_TRY(cudaMemsetAsync(c->d_ctl, 0, sizeof(Control), st));
   GELIO_TRY(cudaMemsetAsync(c->d_part, 0, (size_t)kSpecDoubles * 8, st));
-  Groups g{c->d_gsim, c->d_gpre};
+  Groups g{c->d_gsim, c->d_gpre, 1};
   k_prepare<<<1, 256, 0, st>>>(c->d_params, 1, c->d_sims, c->d_tables, g, c->d_ctl);
   GELIO_TRY(cudaGetLastError());
   KArgs a{};

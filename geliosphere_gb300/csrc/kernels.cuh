@@ -5,8 +5,9 @@
 // warp level every `refill` steps: a ballot of idle lanes, one 64-bit
 // atomicAdd per warp on the model's ticket counter, and each idle lane takes
 // ticket base + rank.  Tickets run over all particles of all simulations of
-// the model in the launch (a whole batch CSV in one launch); the ticket ->
-// (simulation, particle) map is a binary search of the particle prefix sums.
+// the model in the launch (a whole batch CSV in one launch), a segment of each
+// simulation in turn; the ticket -> (simulation, particle) map is a binary
+// search of the segments' prefix sums.
 // This replaces the reference's host loop of 4,096-particle chunks with three
 // device synchronisations each (GeliosphereModel.cu:426-445), and its
 // warp-wide wait for the slowest particle.
@@ -43,10 +44,33 @@ struct Control {
 };
 
 // Simulation grouping by model, written by the prepare kernel.
+//
+// A simulation's tickets are cut into `segs` equal segments and the segments
+// of the model's simulations alternate: segment 0 of each simulation, then
+// segment 1 of each, ...  On a grid injection a simulation's first tickets are
+// its longest trajectories (ticket_particle below), so every simulation's
+// long trajectories start in the first 1 / segs of the run.  One simulation
+// after another, the last one's started when the others were done and the run
+// ended on them: 4 x 250,000 2D Geliosphere particles 75 ms, now 62 (the
+// kernel's full rate needs 51); a batch of 48 uneven rows, 3 M particles, 135 -> 117.
 struct Groups {
   int *sim_idx;                   // [4][n_sims]: simulation indices of model m
-  unsigned long long *prefix;     // [4][n_sims + 1]: particle prefix sums
+  unsigned long long *prefix;     // [4][n_sims * segs + 1]: entry (segment, simulation of the group)
+  int segs;
 };
+
+// 16 segments while the prefix sums stay at 4,096 entries (a 12-step search).
+constexpr int kMaxSegEntries = 4096;
+inline int ticket_segments(int n_sims) {
+  if (n_sims <= 1) return 1;
+  const int s = kMaxSegEntries / n_sims;
+  return s > 16 ? 16 : (s < 1 ? 1 : s);
+}
+// First ticket of segment s of a simulation of n particles.
+__host__ __device__ __forceinline__ unsigned long long segment_first(unsigned long long n, int s, int segs) {
+  const unsigned long long q = n / (unsigned)segs, r = n % (unsigned)segs;
+  return q * (unsigned)s + (((unsigned long long)s < r) ? (unsigned long long)s : r);
+}
 
 struct KArgs {
   const SimDev *sims;
@@ -62,6 +86,7 @@ struct KArgs {
   unsigned long long time_limit_ns; // 0 = no watchdog
   int smem_slots;                 // >0: histograms of the group's first smem_slots sims in shared memory
   int refill;                     // steps between refills (multiple of 4)
+  int ctas_per_sm;                // of this launch (placement of small runs)
   // plain / replay kernel
   int plain_sim;                  // simulation index of a plain launch
   unsigned long long plain_first, plain_count;
@@ -493,14 +518,39 @@ __device__ __forceinline__ unsigned long long grid_points(const SimDev &sd) {
 }
 
 __device__ __forceinline__ int find_group_index(const unsigned long long *prefix, int n,
-                                                unsigned long long t, int hint) {
-  if (hint >= 0 && hint < n && prefix[hint] <= t && t < prefix[hint + 1]) return hint;
+                                                unsigned long long t) {
   int lo = 0, hi = n - 1;          // largest g with prefix[g] <= t
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (prefix[mid] <= t) lo = mid; else hi = mid - 1;
   }
   return lo;
+}
+
+// Placement of a run of fewer trajectories than the launch has lanes.  Such a
+// run ends with its longest chains, and a chain is slowed by the warps it
+// shares its SM with and by the other lanes of its warp (their branches are
+// its own).  Handed out 32 to the warp that asks first, 4,096 trajectories sat
+// in 128 warps on 16 of the 152 SMs.  Instead each CTA opens only as many
+// warps as put kSpreadWarps on an SM (two a scheduler hide each other's
+// latency; FP64: one a scheduler, the SM's FP64 pipe takes 16 cycles an
+// instruction) and each warp as many lanes as the run needs.  A run that needs
+// more opens every warp, then every lane.  4,096 2D Geliosphere trajectories
+// 19.7 -> 16.3 ms; 4,001 1D B-p trajectories in FP64 steps 1,205 -> 849 ms.
+struct Spread {
+  unsigned warps, lanes;          // per CTA, per warp
+};
+template <class R>
+__device__ __forceinline__ Spread spread_lanes(unsigned long long total, unsigned ctas, unsigned ctas_per_sm,
+                                               unsigned warps_per_cta) {
+  constexpr unsigned kSpreadWarps = (sizeof(R) == 8) ? 4u : 8u;
+  Spread s;
+  s.warps = min(warps_per_cta, max(1u, kSpreadWarps / max(1u, ctas_per_sm)));
+  s.lanes = 32u;
+  if (total > (unsigned long long)ctas * s.warps * 32u) s.warps = warps_per_cta;
+  const unsigned long long w = (unsigned long long)ctas * s.warps;
+  if (total < w * 32u) s.lanes = (unsigned)((total + w - 1) / w);
+  return s;
 }
 
 // ---------------------------------------------------------------------------
@@ -514,8 +564,9 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   const int gn = (int)a.ctl->group_count[MODEL];
   if (gn == 0 || a.ctl->status != 0) return;
   const int *gsim = a.groups.sim_idx + (size_t)MODEL * a.n_sims;
-  const unsigned long long *gpre = a.groups.prefix + (size_t)MODEL * (a.n_sims + 1);
-  const unsigned long long total = gpre[gn];
+  const int segs = a.groups.segs, ne = gn * segs;
+  const unsigned long long *gpre = a.groups.prefix + (size_t)MODEL * ((size_t)a.n_sims * segs + 1);
+  const unsigned long long total = gpre[ne];
   const int slots = (gn <= a.smem_slots) ? gn : 0;
   constexpr int W = Window<MODEL>::size;
   for (int i = threadIdx.x; i < slots * W; i += blockDim.x) sh_hist[i] = 0.0;
@@ -535,11 +586,12 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   Lane<R> L;
   Consts<R> K;
   SimDev sd;
-  bool active = false, drained = false;
+  const Spread spread = spread_lanes<R>(total, gridDim.x, (unsigned)a.ctas_per_sm, blockDim.x >> 5);
+  bool active = false, drained = (unsigned)lane >= spread.lanes || (threadIdx.x >> 5) >= spread.warps;
   // 1D models, warp-uniform: every ticket is handed out, so no lane of this
   // warp will be refilled again and the window grows to cut the votes
   bool exhausted = false;
-  int slot = 0, g = -1;
+  int slot = 0;
   unsigned window = 0;
   R zq[4] = {R(0), R(0), R(0), R(0)};     // 1D models: normals of the lane's next step group
 
@@ -584,11 +636,14 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
       if (!active && !drained) {
         const unsigned long long t = base + __popc(need & lanemask_lt());
         if (t < total) {
-          g = find_group_index(gpre, gn, t, g);
-          const int sim = gsim[g];
+          const int g = find_group_index(gpre, ne, t);
+          const int seg = g / gn;
+          slot = g - seg * gn;
+          const int sim = gsim[slot];
           sd = a.sims[sim];
-          slot = g;
-          const unsigned long long pid = ticket_particle(t - gpre[g], gpre[g + 1] - gpre[g], grid_points(sd));
+          const unsigned long long n = (unsigned long long)sd.n_particles;
+          const unsigned long long pid =
+              ticket_particle(segment_first(n, seg, segs) + (t - gpre[g]), n, grid_points(sd));
           init_lane<MODEL, R>(L, K, sd, a.inj_tables + (size_t)sim * GELIO_GRID_MAX, sim, pid);
           if constexpr (Prefetch<MODEL>::value) draw_group<MODEL, R>(L, 0u, zq);
           sink.add(slot, sim, kOffNParticles, 1.0);
