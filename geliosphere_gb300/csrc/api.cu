@@ -525,8 +525,8 @@ static int shape_for(gelio_ctx *c, int model, int prec, int n_in_group_hint, con
   s.refill = (o && o->refill_interval > 0) ? o->refill_interval : (t.refill > 0 ? t.refill : default_refill(model));
   if (s.refill % 4 != 0 || s.refill > 4096) return GELIO_ERR_INVALID_ARGUMENT;
   const int win_doubles = (model >= kModelSolarProp) ? (kWinHi - kWin2DLo) : (kWinHi - kWin1DLo);
-  const size_t per_slot = (size_t)win_doubles * 8;
-  const size_t qbytes = (size_t)(s.block / 32) * (kQueue * sizeof(QEnt) + sizeof(int));
+  const size_t wbytes = (size_t)(s.block / 32) * warp_bytes(model, prec == 1 ? sizeof(double) : sizeof(float));
+  auto smem_of = [&](int slots_) { return hist_doubles(slots_, win_doubles) * 8 + wbytes; };
   // occupancy per (model, precision, block, smem slots), cached: no CUDA
   // call that a stream capture would reject happens while enqueueing
   const int bi = (int)s.block / 32 - 1;
@@ -536,7 +536,7 @@ static int shape_for(gelio_ctx *c, int model, int prec, int n_in_group_hint, con
     if (cached == 0) {
       int occ = 0;
       GELIO_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kfn, (int)s.block,
-                                                              (size_t)slots_ * per_slot + qbytes));
+                                                              smem_of(slots_)));
       cached = (occ < 1) ? -1 : occ;
     }
     occ_ = cached;
@@ -552,7 +552,7 @@ static int shape_for(gelio_ctx *c, int model, int prec, int n_in_group_hint, con
   const int max_slots = (model >= kModelSolarProp) ? 4 : 1;
   int slots = (n_in_group_hint >= 1 && n_in_group_hint <= max_slots) ? n_in_group_hint : 0;
   while (slots > 0) {
-    if ((size_t)slots * per_slot + qbytes <= (size_t)c->max_smem_optin) {
+    if (smem_of(slots) <= (size_t)c->max_smem_optin) {
       int occs = 0;
       rc0 = occupancy(slots, occs);
       if (rc0 != GELIO_OK) return rc0;
@@ -561,7 +561,7 @@ static int shape_for(gelio_ctx *c, int model, int prec, int n_in_group_hint, con
     slots = (slots == n_in_group_hint) ? 0 : slots - 1;   // all of the group's sims or none
   }
   s.smem_slots = slots;
-  s.smem = (size_t)slots * per_slot + qbytes;
+  s.smem = smem_of(slots);
   int occ = 0;
   rc0 = occupancy(slots, occ);
   if (rc0 != GELIO_OK) return rc0;
@@ -628,7 +628,7 @@ int32_t gelio_create(gelio_ctx **out, int32_t device) {
     for (int m = 0; m < 4 && rc == GELIO_OK; ++m)
       for (int p = 0; p < 3 && rc == GELIO_OK; ++p) {
         const int win = (m >= kModelSolarProp) ? 4 * (kWinHi - kWin2DLo) : (kWinHi - kWin1DLo);
-        const int need = win * 8 + 8 * (kQueue * (int)sizeof(QEnt) + (int)sizeof(int));
+        const int need = (int)(hist_doubles(1, win) * 8 + 8 * warp_bytes(m, p == 1 ? sizeof(double) : sizeof(float)));
         const int bytes = need <= c->max_smem_optin ? need : c->max_smem_optin;
         e = cudaFuncSetAttribute(model_kernel(m, true, p), cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
         if (e != cudaSuccess) rc = map_cuda(e);

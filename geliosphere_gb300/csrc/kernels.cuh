@@ -215,17 +215,17 @@ __device__ __forceinline__ void append_records(const KArgs &a, unsigned mask, co
 }
 
 // Append one exit record (any lane, no warp synchronisation).
-template <class R>
-__device__ __forceinline__ void append_record_one(const KArgs &a, const Lane<R> &L, int model) {
+template <int MODEL, class R>
+__device__ __forceinline__ void append_record_one(const KArgs &a, const Lane<R> &L) {
   const unsigned long long idx = atomicAdd(&a.ctl->rec_count, 1ull);
   if (idx < a.record_capacity) {
     gelio_exit_record rec;
     rec.particle = (int64_t)L.pid;
     rec.sim = L.sim;
     rec.t_injection = L.Tinj;
-    rec.t_exit = (float)L.T.v;
+    rec.t_exit = (float)lane_energy<MODEL>(L);
     rec.r = (float)L.r.v;
-    rec.theta = (model >= kModelSolarProp) ? (float)theta_full(L) : 0.0f;
+    rec.theta = (MODEL >= kModelSolarProp) ? (float)theta_full(L) : 0.0f;
     rec.sumac = 0.0f;
     a.records[idx] = rec;
   } else {
@@ -336,10 +336,20 @@ struct QEnt {
   unsigned slot_gbin;        // group slot (low 16 bits), grid bin + 1 (high 16 bits)
 };
 constexpr int kQueue = 64;   // entries per warp (<= 31 left + 32 pushed)
-// F-p: at most this many running trajectories in a warp whose tickets are
+// 1D: at most this many running trajectories in a warp whose tickets are
 // exhausted switch to normals drawn by the whole warp (>= 4 groups ahead each)
 constexpr int kCoopLanes = 8;
-static_assert(32 * 4 * sizeof(double) <= kQueue * sizeof(QEnt), "cooperative normals fit a warp's queue area");
+
+// Dynamic shared memory of a persistent CTA: histograms of `slots`
+// simulations (rounded up to 16 bytes), then per warp its exit queue, its
+// cooperative normals (1D: 32 groups of four) and its queue length.
+__host__ __device__ constexpr size_t hist_doubles(size_t slots, size_t window) { return (slots * window + 1) & ~(size_t)1; }
+__host__ __device__ constexpr size_t coop_bytes(int model, size_t real_bytes) {
+  return (model == kModelFp || model == kModelBp) ? 32 * 4 * real_bytes : 0;
+}
+__host__ __device__ constexpr size_t warp_bytes(int model, size_t real_bytes) {
+  return kQueue * sizeof(QEnt) + coop_bytes(model, real_bytes) + sizeof(int);
+}
 
 template <int MODEL>
 __device__ __forceinline__ void flush_queue(const KArgs &a, const Sink<MODEL> &sink, const QEnt *q,
@@ -364,28 +374,24 @@ __device__ __forceinline__ void flush_queue(const KArgs &a, const Sink<MODEL> &s
 // lengthening every step.
 struct FpCrossing {
   float Tinj, Texit, rrec, sumac;
-  int sim, slot, grid_bins;
+  int sim, slot;
   unsigned long long pid;
-  double grid_log_lo, grid_inv_dlog;
 };
 
 template <class R>
-__device__ __forceinline__ FpCrossing fp_crossing(const Lane<R> &L, const SimDev &sd, int slot) {
+__device__ __forceinline__ FpCrossing fp_crossing(const Lane<R> &L, int slot) {
   FpCrossing x;
   x.Tinj = L.Tinj;
-  x.Texit = (float)L.T.v;
+  x.Texit = (float)lane_energy<kModelFp>(L);
   x.rrec = L.rrec;
   x.sumac = (float)L.sumac.v;
   x.sim = L.sim;
   x.slot = slot;
-  x.grid_bins = sd.grid_bins;
   x.pid = L.pid;
-  x.grid_log_lo = sd.grid_log_lo;
-  x.grid_inv_dlog = sd.grid_inv_dlog;
   return x;
 }
 
-static __device__ __noinline__ void emit_fp(Control *ctl, gelio_exit_record *records,
+static __device__ __noinline__ void emit_fp(Control *ctl, const SimDev *sims, gelio_exit_record *records,
                                      unsigned long long record_capacity, Sink<kModelFp> sink,
                                      FpCrossing x) {
   const double p100 = round6(p_si((double)x.Tinj));
@@ -401,7 +407,8 @@ static __device__ __noinline__ void emit_fp(Control *ctl, gelio_exit_record *rec
   if (C.b_e2) { sink.add(slot, s, kOffE2W + C.b_e2 - 1, w); sink.add(slot, s, kOffE2W2 + C.b_e2 - 1, w2); sink.add(slot, s, kOffE2N + C.b_e2 - 1, 1.0); }
   if (C.b_e3) { sink.add(slot, s, kOffE3W + C.b_e3 - 1, w); sink.add(slot, s, kOffE3W2 + C.b_e3 - 1, w2); sink.add(slot, s, kOffE3N + C.b_e3 - 1, 1.0); }
   if (C.b_e4) { sink.add(slot, s, kOffE4W + C.b_e4 - 1, w); sink.add(slot, s, kOffE4W2 + C.b_e4 - 1, w2); sink.add(slot, s, kOffE4N + C.b_e4 - 1, 1.0); }
-  const int gb = grid_log_bin(T1, x.grid_log_lo, x.grid_inv_dlog, x.grid_bins);
+  const SimDev &sd = sims[s];
+  const int gb = grid_log_bin(T1, sd.grid_log_lo, sd.grid_inv_dlog, sd.grid_bins);
   if (gb >= 0) {
     sink.add(slot, s, kOffGridW + gb, w);
     sink.add(slot, s, kOffGridW2 + gb, w2);
@@ -479,11 +486,6 @@ __device__ __forceinline__ void draw(Lane<R> &L, R *z) {
 template <int MODEL> struct Prefetch {
   static constexpr bool value = (MODEL == kModelFp || MODEL == kModelBp);
 };
-
-template <int MODEL, class R>
-__device__ __forceinline__ void draw_group(const Lane<R> &L, uint32_t group, R *z) {
-  normals4<R>(L.key0, L.key1, group, kStreamSde, L.pid, z);
-}
 
 // Particle handed out by the u-th ticket of a simulation of n particles.
 // On a grid injection (particle i takes grid point i mod P, the energies
@@ -570,11 +572,13 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   const int slots = (gn <= a.smem_slots) ? gn : 0;
   constexpr int W = Window<MODEL>::size;
   for (int i = threadIdx.x; i < slots * W; i += blockDim.x) sh_hist[i] = 0.0;
-  // the exit queues and their lengths follow the histogram window (sized
-  // for a.smem_slots)
-  QEnt *qbase = reinterpret_cast<QEnt *>(sh_hist + (size_t)a.smem_slots * W);
-  QEnt *q = qbase + (threadIdx.x >> 5) * kQueue;
-  int *qlen = reinterpret_cast<int *>(qbase + (blockDim.x >> 5) * kQueue) + (threadIdx.x >> 5);
+  // what follows the histogram window (sized for a.smem_slots)
+  const unsigned warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
+  QEnt *qbase = reinterpret_cast<QEnt *>(sh_hist + hist_doubles(a.smem_slots, W));
+  QEnt *q = qbase + warp * kQueue;
+  unsigned char *coop_base = reinterpret_cast<unsigned char *>(qbase + warps * kQueue);
+  R *coop = reinterpret_cast<R *>(coop_base + warp * coop_bytes(MODEL, sizeof(R)));
+  int *qlen = reinterpret_cast<int *>(coop_base + warps * coop_bytes(MODEL, sizeof(R))) + warp;
   if ((threadIdx.x & 31) == 0) *qlen = 0;
   __syncthreads();
   Sink<MODEL> sink;
@@ -585,15 +589,15 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   const int lane = threadIdx.x & 31;
   Lane<R> L;
   Consts<R> K;
-  SimDev sd;
-  const Spread spread = spread_lanes<R>(total, gridDim.x, (unsigned)a.ctas_per_sm, blockDim.x >> 5);
-  bool active = false, drained = (unsigned)lane >= spread.lanes || (threadIdx.x >> 5) >= spread.warps;
+  const Spread spread = spread_lanes<R>(total, gridDim.x, (unsigned)a.ctas_per_sm, warps);
+  bool active = false, drained = (unsigned)lane >= spread.lanes || warp >= spread.warps;
   // 1D models, warp-uniform: every ticket is handed out, so no lane of this
   // warp will be refilled again and the window grows to cut the votes
   bool exhausted = false;
   int slot = 0;
   unsigned window = 0;
   R zq[4] = {R(0), R(0), R(0), R(0)};     // 1D models: normals of the lane's next step group
+  PhiloxLane rng;                          // 1D models
 
   for (;;) {
     // 1) evaluate and bin queued exits, 32 at a time with every lane busy
@@ -640,12 +644,15 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
           const int seg = g / gn;
           slot = g - seg * gn;
           const int sim = gsim[slot];
-          sd = a.sims[sim];
+          const SimDev sd = a.sims[sim];
           const unsigned long long n = (unsigned long long)sd.n_particles;
           const unsigned long long pid =
               ticket_particle(segment_first(n, seg, segs) + (t - gpre[g]), n, grid_points(sd));
           init_lane<MODEL, R>(L, K, sd, a.inj_tables + (size_t)sim * GELIO_GRID_MAX, sim, pid);
-          if constexpr (Prefetch<MODEL>::value) draw_group<MODEL, R>(L, 0u, zq);
+          if constexpr (Prefetch<MODEL>::value) {
+            rng = philox_lane(L.key0, L.key1, kStreamSde, pid);
+            normals_of<R>(philox_draw(rng, 0u), zq);
+          }
           sink.add(slot, sim, kOffNParticles, 1.0);
           active = true;
         } else {
@@ -664,47 +671,84 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
     constexpr int spc = StepsPerCall<MODEL>::value;
     const int win = (Prefetch<MODEL>::value && exhausted && a.refill < 64) ? 64 : a.refill;
     const uint32_t cap32 = (a.max_steps > 0xffffffffull) ? 0xffffffffu : (uint32_t)a.max_steps;
-    // F-p runs end on the latency of their longest chain: one test per step
-    // covers the rare events (a crossing record, a stop, the step cap), and a
-    // stopped lane leaves its group of four steps at once
-    auto fp_group = [&](const R *z) {
-      if constexpr (MODEL == kModelFp) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int res = step_fp(L, K, z[j]);
+    // the end of a lane's trajectory (2D, B-p) with the result of its last step
+    auto end_lane = [&](int res) {
+      active = false;
+      sink.add(slot, L.sim, kOffNSteps, (double)L.steps);
+      if (res == kRecordAndStop) {
+        // queue the exit (at most one per lane per window: <= 63 entries)
+        QEnt e;
+        e.Tinj = L.Tinj;
+        e.Texit = (float)lane_energy<MODEL>(L);
+        e.sim = L.sim;
+        e.slot_gbin = ((unsigned)(L.gbin + 1) << 16) | ((unsigned)slot & 0xffffu);
+        q[atomicAdd(qlen, 1)] = e;
+        if (a.records != nullptr) append_record_one<MODEL>(a, L);
+      } else if (res != kContinue) {
+        sink.add(slot, L.sim, kOffNLost, 1.0);
+      } else {
+        sink.add(slot, L.sim, kOffNCapped, 1.0);
+      }
+    };
+    // A 1D lane's next four steps: as one block if they meet no rare event,
+    // else one by one.  Both 1D kernels gain: B-p is bound by instruction
+    // issue (the event tests and selects of four steps become one test), F-p
+    // by the latency of its longest chain (four steps without a branch
+    // overlap).  A lane at an event repeats its group while its warp waits:
+    // rare, since events are (B-p: ~10^-4 of the steps).  With the energy
+    // formed only at a record, kept round keys and B-p's tail drawn by the
+    // warp: B-p 400,000 particles 227 -> 156 ms (258 -> 378 G steps/s), 4,001
+    // in FP64 steps 849 -> 440 ms, F-p 10^6 particles 116 -> 44 ms.
+    auto group_1d = [&](const R *z) {
+      if constexpr (Prefetch<MODEL>::value) {
+        if (L.steps + 4u < cap32 && four_quiet_steps<MODEL, R>(L, K, z)) {
+          L.steps += 4u;
+          return;
+        }
+        R z0 = z[0], z1 = z[1], z2 = z[2];
+        const R z3 = z[3];
+#pragma unroll 1
+        for (int j = 0; j < 4 && active; ++j) {
+          const int res = (MODEL == kModelFp) ? step_fp(L, K, z0) : step_bp(L, K, z0);
+          z0 = z1;
+          z1 = z2;
+          z2 = z3;
           ++L.steps;
+          // an exit on the capped step counts as an exit
           if (res != kContinue || L.steps >= cap32) {
-            if (res == kRecordAndContinue || res == kRecordAndStop)
-              emit_fp(a.ctl, a.records, a.record_capacity, sink, fp_crossing(L, sd, slot));
-            if (res == kRecordAndStop || res == kStop) {
+            if constexpr (MODEL == kModelFp) {
+              if (res == kRecordAndContinue || res == kRecordAndStop)
+                emit_fp(a.ctl, a.sims, a.records, a.record_capacity, sink, fp_crossing(L, slot));
+              if (res == kRecordAndContinue && L.steps < cap32) continue;
               active = false;
+              if (res == kContinue || res == kRecordAndContinue) sink.add(slot, L.sim, kOffNCapped, 1.0);
               sink.add(slot, L.sim, kOffNSteps, (double)L.steps);
-            } else if (L.steps >= cap32) {
-              active = false;
-              sink.add(slot, L.sim, kOffNSteps, (double)L.steps);
-              sink.add(slot, L.sim, kOffNCapped, 1.0);
+            } else {
+              end_lane(res);
             }
-            if (!active) break;
           }
         }
       }
     };
-    if constexpr (MODEL == kModelFp) {
-      // The tail of an F-p run: this warp's tickets are exhausted and at most
-      // kCoopLanes of its trajectories still run (often one chain of ~10^6
-      // steps).  A trajectory's normals depend only on (key, particle, group
-      // of four steps), so every lane of the warp draws one group for one of
-      // the running trajectories -- 32 / n groups ahead for each of n -- into
-      // the warp's exit-queue area (F-p queues no exits), and the running
-      // lanes then integrate those groups without drawing: a lone chain pays
-      // one warp-wide draw per 128 steps instead of one per 4 steps on its
-      // own instruction stream.  The normals are those of the per-lane draws
-      // (a lane at a window start is at a group boundary), so the results are
-      // identical.
+    if constexpr (Prefetch<MODEL>::value) {
+      // The tail of a 1D run: this warp's tickets are exhausted and at most
+      // kCoopLanes of its trajectories still run (F-p: often one chain of
+      // ~10^6 steps).  A trajectory's normals depend only on (key, particle,
+      // group of four steps), so every lane of the warp draws one group for
+      // one of the running trajectories -- 32 / n groups ahead for each of n
+      // -- into shared memory, and the running lanes then integrate those
+      // groups without drawing: a lone chain pays one warp-wide draw per 128
+      // steps instead of one per 4 steps on its own instruction stream.  The
+      // normals are those of the per-lane draws (a lane at a window start is
+      // at a group boundary), so the results are identical.
       const unsigned act = __ballot_sync(kFull, active);
       const int na = __popc(act);
+      if (!exhausted && spread.lanes < 32u) {     // a small run hands out its tickets at once
+        unsigned long long t = 0;
+        if (lane == 0) t = *(volatile unsigned long long *)&a.ctl->ticket[MODEL];
+        exhausted = __shfl_sync(kFull, t, 0) >= total;
+      }
       if (exhausted && na <= kCoopLanes) {
-        R *coop = reinterpret_cast<R *>(q);            // [na][G][4] normals, <= 128 entries
         const int G = 32 / na;
         const int jt = lane % na, gi = lane / na;     // this lane draws group gi of the jt-th running lane
         unsigned m = act;
@@ -721,32 +765,35 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
           for (int j = 0; j < 4; ++j) coop[(jt * G + gi) * 4 + j] = zz[j];
         }
         __syncwarp();
-        const int me = __popc(act & lanemask_lt());
-        for (int g = 0; g < G; ++g) {
-          if (active) {
-            R z[4];
+        if (active) {
+          const R *mine = coop + __popc(act & lanemask_lt()) * G * 4;
+          R z[4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) z[j] = coop[(me * G + g) * 4 + j];
-            fp_group(z);
+          for (int j = 0; j < 4; ++j) z[j] = mine[j];
+          for (int g = 1; g <= G && active; ++g) {
+            R zn[4];                                   // the next group's, loaded under this one's steps
+            const int gn = g < G ? g : 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) zn[j] = mine[gn * 4 + j];
+            group_1d(z);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) z[j] = zn[j];
           }
         }
         __syncwarp();                                  // the buffer is drawn again next window
         continue;
       }
     }
-    for (int k = 0; k < win; k += spc) {
+    for (int k = 0; k < win; k += (Prefetch<MODEL>::value ? 4 : spc)) {
       if (active) {
         R z[4];
         if constexpr (Prefetch<MODEL>::value) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) z[j] = zq[j];
-          draw_group<MODEL, R>(L, L.steps / spc + 1u, zq);
+          normals_of<R>(philox_draw(rng, L.steps / 4u + 1u), zq);
+          group_1d(z);
         } else {
           draw<MODEL, R>(L, z);
-        }
-        if constexpr (MODEL == kModelFp) {
-          fp_group(z);
-        } else {
 #pragma unroll
           for (int j = 0; j < spc; ++j) {
             if (active) {
@@ -754,24 +801,7 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
               ++L.steps;
               // one test per step covers the rare events: an exit, a stop,
               // the step cap (an exit on the capped step counts as an exit)
-              if (res != kContinue || L.steps >= cap32) {
-                active = false;
-                sink.add(slot, L.sim, kOffNSteps, (double)L.steps);
-                if (res == kRecordAndStop) {
-                  // queue the exit (at most one per lane per window: <= 63 entries)
-                  QEnt e;
-                  e.Tinj = L.Tinj;
-                  e.Texit = (float)L.T.v;
-                  e.sim = L.sim;
-                  e.slot_gbin = ((unsigned)(L.gbin + 1) << 16) | ((unsigned)slot & 0xffffu);
-                  q[atomicAdd(qlen, 1)] = e;
-                  if (a.records != nullptr) append_record_one(a, L, MODEL);
-                } else if (res != kContinue) {
-                  sink.add(slot, L.sim, kOffNLost, 1.0);
-                } else {
-                  sink.add(slot, L.sim, kOffNCapped, 1.0);
-                }
-              }
+              if (res != kContinue || L.steps >= cap32) end_lane(res);
             }
           }
         }
@@ -825,7 +855,7 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4) ? 2 : 1) k_plain(const K
         ++L.steps;
         if (res == kRecordAndContinue || res == kRecordAndStop) {
           if (nrec == 0) {
-            t_rec = (float)L.T.v;
+            t_rec = (float)lane_energy<MODEL>(L);
             r_rec = (MODEL == kModelFp) ? L.rrec : (float)L.r.v;
             aux_rec = (MODEL == kModelFp) ? (float)L.sumac.v : (float)theta_full(L);
           }
@@ -833,14 +863,14 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4) ? 2 : 1) k_plain(const K
         }
         if constexpr (MODEL == kModelFp) {
           if (res == kRecordAndContinue || res == kRecordAndStop)
-            emit_fp(a.ctl, a.records, a.record_capacity, sink, fp_crossing(L, sd, 1 << 30));
+            emit_fp(a.ctl, a.sims, a.records, a.record_capacity, sink, fp_crossing(L, 1 << 30));
           if (res != kContinue && res != kRecordAndContinue) { active = false; status = (nrec > 0) ? 0 : 1; }
         } else if (res != kContinue) {
           active = false;
           if (res == kRecordAndStop) {
             pending = true;
             status = 0;
-            pd.Tinj = L.Tinj; pd.Texit = (float)L.T.v; pd.r = (float)L.r.v; pd.aux = (float)theta_full(L);
+            pd.Tinj = L.Tinj; pd.Texit = (float)lane_energy<MODEL>(L); pd.r = (float)L.r.v; pd.aux = (float)theta_full(L);
             pd.sim = sim; pd.slot = 1 << 30; pd.gbin = L.gbin; pd.pid = L.pid;
           } else {
             status = 1;
@@ -869,7 +899,7 @@ __global__ void __launch_bounds__(256, (sizeof(R) == 4) ? 2 : 1) k_plain(const K
     t.steps = L.steps;
     t.n_records = nrec;
     t.t_injection = L.Tinj;
-    t.t_final = (float)L.T.v;
+    t.t_final = (float)lane_energy<MODEL>(L);
     t.r_final = (float)L.r.v;
     t.theta_final = (MODEL == kModelFp) ? (float)L.sumac.v : (float)theta_full(L);
     t.t_record = t_rec;

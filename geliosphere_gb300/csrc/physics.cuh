@@ -63,6 +63,12 @@ template <> struct Math<float> {
   __device__ static __forceinline__ float atan(float x) { return atanf(x); }
   __device__ static __forceinline__ float abs(float x) { return fabsf(x); }
   __device__ static __forceinline__ float copysign(float x, float y) { return copysignf(x, y); }
+  __device__ static __forceinline__ float min(float x, float y) { return fminf(x, y); }
+  __device__ static __forceinline__ float fma(float a, float b, float c) { return fmaf(a, b, c); }
+  // a b and a b + c with every operation rounded: never contracted into an fma
+  __device__ static __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+  __device__ static __forceinline__ float mul_add(float a, float b, float c) { return __fadd_rn(__fmul_rn(a, b), c); }
+  __device__ static __forceinline__ float max(float x, float y) { return fmaxf(x, y); }
 };
 
 template <> struct Math<double> {
@@ -77,6 +83,13 @@ template <> struct Math<double> {
   __device__ static __forceinline__ double atan(double x) { return ::atan(x); }
   __device__ static __forceinline__ double abs(double x) { return fabs(x); }
   __device__ static __forceinline__ double copysign(double x, double y) { return ::copysign(x, y); }
+  __device__ static __forceinline__ double min(double x, double y) { return fmin(x, y); }
+  __device__ static __forceinline__ double fma(double a, double b, double c) { return ::fma(a, b, c); }
+  __device__ static __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+  __device__ static __forceinline__ double mul_add(double a, double b, double c) {
+    return __dadd_rn(__dmul_rn(a, b), c);
+  }
+  __device__ static __forceinline__ double max(double x, double y) { return fmax(x, y); }
 };
 
 // Kahan-compensated scalar: value v, running compensation c (true ~ v - c).
@@ -91,6 +104,17 @@ template <class R> struct Acc {
       v = t;
     } else {
       v += d;
+    }
+  }
+  // add(a b), the product not rounded by itself
+  __device__ __forceinline__ void add_product(R a, R b) {
+    if constexpr (Math<R>::kCompensate) {
+      const R y = Math<R>::fma(a, b, -c);
+      const R t = v + y;
+      c = (t - v) - y;
+      v = t;
+    } else {
+      v = Math<R>::fma(a, b, v);
     }
   }
   __device__ __forceinline__ void negate() { v = -v; c = -c; }
@@ -493,6 +517,40 @@ __device__ __forceinline__ int step_solarprop(Lane<R> &L, const Consts<R> &k, R 
   return (L.r.v > R(100)) ? kRecordAndStop : ((L.r.v < R(100)) ? kContinue : kStop);
 }
 
+// Kinetic energy of a lane that has taken a step.  The 1D steps carry the
+// momentum Pt and q = 1 / sqrt(Pt^2 + T0^2) only: the energy itself,
+// P^2 / (sqrt(P^2 + T0^2) + T0), is formed where a record asks for it.
+template <int MODEL, class R>
+__device__ __forceinline__ R lane_energy(const Lane<R> &L) {
+  if constexpr (MODEL == kModelFp || MODEL == kModelBp) {
+    using M = Math<R>;
+    const R T0 = (R)kT0;
+    const R xn = M::mul_add(L.Pt, L.Pt, T0 * T0);
+    return M::mul(M::mul(L.Pt, L.Pt), M::rcp(M::fma(xn, L.q, T0)));
+  } else {
+    return L.T.v;
+  }
+}
+
+// The 1D steps are compiled into several loops; which products of a sum the
+// compiler would contract may differ from one to the next, so it is written
+// out: a trajectory's bits do not depend on the loop that integrates it.
+
+// B-p: dr of Eq. 13.
+template <class R>
+__device__ __forceinline__ R bp_dr(const Consts<R> &k, R Kdiff, R inv_r, R z) {
+  using M = Math<R>;
+  const R K2 = M::mul(R(2), Kdiff);
+  return M::fma(z, M::sqrt(M::mul(K2, k.dt)), M::mul(M::fma(K2, inv_r, k.V), k.dt));
+}
+// F-p: dr of Eq. 9; sqrt(2 Kdiff dt) = Pt sqrt(2 K0 dt) sqrt(q), Kdiff: Eq. 7.
+template <class R>
+__device__ __forceinline__ R fp_dr(const Consts<R> &k, R Pt, R q, R beta, R inv_r, R z) {
+  using M = Math<R>;
+  const R K2 = M::mul(R(2), M::mul(M::mul(k.K0, beta), Pt));
+  return M::fma(M::fma(K2, inv_r, k.V), k.dt, M::mul(z, M::mul(M::mul(Pt, k.sq2K0dt), M::sqrt(q))));
+}
+
 // ---------------------------------------------------------------------------
 // 1D B-p: OneDimensionBpModel.cu:69-140 (Eq. 5-7, 12-14).  V < 0.
 // ---------------------------------------------------------------------------
@@ -511,15 +569,12 @@ __device__ __forceinline__ int step_bp(Lane<R> &L, const Consts<R> &k, R z) {
   const Acc<R> Psave = L.P;
   const Acc<R> rsave = L.r;
   const R inv_r = M::rcp(r);
-  L.P.add(-k.adv * Rig * inv_r);                        // Eq. 14
-  const R Kdiff = k.K0 * beta0 * Rig;                   // Eq. 7
-  const R dr = (k.V + R(2) * Kdiff * inv_r) * k.dt + z * M::sqrt(R(2) * Kdiff * k.dt);   // Eq. 13
+  L.P.add_product(M::mul(-k.adv, Rig), inv_r);          // Eq. 14
+  const R dr = bp_dr(k, M::mul(M::mul(k.K0, beta0), Rig), inv_r, z);   // Kdiff: Eq. 7
   L.r.add(dr);
   const R Pn = L.P.v;
-  const R xn = Pn * Pn + T0 * T0;
+  const R xn = M::mul_add(Pn, Pn, T0 * T0);
   const R qn = M::rsqrt(xn);
-  const R Tn = Pn * Pn * M::rcp(xn * qn + T0);          // P^2 / (sqrt(P^2 + T0^2) + T0)
-  L.T.set(Tn);
   L.Pt = Pn;
   L.q = qn;
   const R beta = Pn * qn;                               // beta of Tn
@@ -554,20 +609,16 @@ __device__ __forceinline__ int step_fp(Lane<R> &L, const Consts<R> &k, R z) {
   const R Pt = L.Pt, q = L.q;
   const R beta = Pt * q;
   const R inv_r = M::rcp(r);
-  L.sumac.add(R(2) * k.adv * inv_r);                    // Eq. 11: 4 V dt / (3 r)
+  L.sumac.add_product(M::mul(R(2), k.adv), inv_r);      // Eq. 11: 4 V dt / (3 r)
   const Acc<R> Psave = L.P;
   const Acc<R> rsave = L.r;
-  L.P.add(-k.adv * L.P.v * inv_r);                      // Eq. 10
-  const R Kdiff = k.K0 * beta * Pt;                     // Eq. 7
-  // Eq. 9; sqrt(2 Kdiff dt) = Pt sqrt(2 K0 dt) sqrt(q)
-  const R dr = (k.V + R(2) * Kdiff * inv_r) * k.dt + z * (Pt * k.sq2K0dt * M::sqrt(q));
+  L.P.add_product(M::mul(-k.adv, L.P.v), inv_r);        // Eq. 10
+  const R dr = fp_dr(k, Pt, q, beta, inv_r, z);
   L.r.add(dr);
   const R Pn = L.P.v;
   const R Pn2 = Pn * Pn;
-  const R xn = Pn2 + T0 * T0;
+  const R xn = M::mul_add(Pn, Pn, T0 * T0);
   const R qn = M::rsqrt(xn);
-  const R Tn = Pn2 * M::rcp(xn * qn + T0);              // P^2 / (sqrt(P^2 + T0^2) + T0)
-  L.T.set(Tn);
   L.Pt = Pn;                     // T keeps the rejected step's value if the step is undone below
   L.q = qn;
   const R rn = L.r.v;
@@ -587,6 +638,63 @@ __device__ __forceinline__ int step_fp(Lane<R> &L, const Consts<R> &k, R z) {
   const int ended = cross ? kRecordAndStop : kStop;
   const int going = cross ? kRecordAndContinue : kContinue;
   return slow ? kStop : (out ? ended : going);
+}
+
+// ---------------------------------------------------------------------------
+// Four 1D steps at once, for the common case that none of them meets a rare
+// event (a record, a stop, an undone step): the same arithmetic as step_bp /
+// step_fp without their events, straight through, so that the four steps
+// schedule as one block.  Returns false, with the lane as it was, if an event
+// is possible; the caller then takes the four steps one by one.
+//
+// What makes an event impossible, B-p: r in [0.3, 100] and beta > 0.01 after
+// each step (exits and stops need r > 100 or beta < 0.01, undone steps
+// r < 0.3).  F-p: r in [1.5, 100] after each step and before the first (a
+// crossing has 1 AU between r - dr and r, and r - dr is the step's start to a
+// few units of rounding; undone steps need r < 0.1, the outer exit
+// r >= 100.0002), and beta > 0.01 at the start of each.
+// ---------------------------------------------------------------------------
+template <int MODEL, class R>
+__device__ __forceinline__ bool four_quiet_steps(Lane<R> &L, const Consts<R> &k, const R *z) {
+  using M = Math<R>;
+  static_assert(MODEL == kModelFp || MODEL == kModelBp, "1D models");
+  const R T0 = (R)kT0;
+  Acc<R> r = L.r, P = L.P, sumac = L.sumac;
+  R Pt = L.Pt, q = L.q;
+  R lo = r.v, hi = r.v, beta = Pt * q, beta_low = beta;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const R inv_r = M::rcp(r.v);
+    R dr;
+    if constexpr (MODEL == kModelBp) {
+      const R Rig = P.v;
+      P.add_product(M::mul(-k.adv, Rig), inv_r);
+      dr = bp_dr(k, M::mul(M::mul(k.K0, beta), Rig), inv_r, z[j]);
+    } else {
+      sumac.add_product(M::mul(R(2), k.adv), inv_r);
+      P.add_product(M::mul(-k.adv, P.v), inv_r);
+      dr = fp_dr(k, Pt, q, beta, inv_r, z[j]);
+    }
+    r.add(dr);
+    Pt = P.v;
+    q = M::rsqrt(M::mul_add(Pt, Pt, T0 * T0));
+    beta = Pt * q;
+    lo = M::min(lo, r.v);
+    hi = M::max(hi, r.v);
+    if (MODEL == kModelBp || j < 3) beta_low = M::min(beta_low, beta);
+  }
+  const R r_low = (MODEL == kModelBp) ? (R)0.3f : (R)1.5f;
+  // (a NaN passes through the minimum and maximum: in r it stays to the last
+  // step, in beta it is no event)
+  const bool quiet = lo >= r_low && hi <= R(100) && r.v <= R(100) && beta_low > (R)0.01f;
+  if (quiet) {
+    L.r = r;
+    L.P = P;
+    L.Pt = Pt;
+    L.q = q;
+    if constexpr (MODEL == kModelFp) L.sumac = sumac;
+  }
+  return quiet;
 }
 
 }  // namespace gelio
