@@ -568,7 +568,6 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   const int *gsim = a.groups.sim_idx + (size_t)MODEL * a.n_sims;
   const int segs = a.groups.segs, ne = gn * segs;
   const unsigned long long *gpre = a.groups.prefix + (size_t)MODEL * ((size_t)a.n_sims * segs + 1);
-  const unsigned long long total = gpre[ne];
   const int slots = (gn <= a.smem_slots) ? gn : 0;
   constexpr int W = Window<MODEL>::size;
   for (int i = threadIdx.x; i < slots * W; i += blockDim.x) sh_hist[i] = 0.0;
@@ -589,11 +588,19 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   const int lane = threadIdx.x & 31;
   Lane<R> L;
   Consts<R> K;
-  const Spread spread = spread_lanes<R>(total, gridDim.x, (unsigned)a.ctas_per_sm, warps);
-  bool active = false, drained = (unsigned)lane >= spread.lanes || warp >= spread.warps;
-  // 1D models, warp-uniform: every ticket is handed out, so no lane of this
-  // warp will be refilled again and the window grows to cut the votes
-  bool exhausted = false;
+  bool active = false, drained, exhausted;
+  // The first tickets are dealt, not asked for: chunk w * CTAs + b to warp w of
+  // CTA b, so that every SM starts with its share of each length of trajectory
+  // (asked for, the longest went to the CTAs that started first: 60,000 2D
+  // particles 28.3 ms, dealt 25.0).  The counter hands out those after.
+  //
+  // exhausted (1D models, warp-uniform): every ticket is handed out, so no lane
+  // of this warp will be refilled again and the window grows to cut the votes
+  {
+    const Spread spread = spread_lanes<R>(gpre[ne], gridDim.x, (unsigned)a.ctas_per_sm, warps);
+    drained = (unsigned)lane >= spread.lanes || warp >= spread.warps;
+    exhausted = gpre[ne] <= (unsigned long long)gridDim.x * spread.warps * spread.lanes;
+  }
   int slot = 0;
   unsigned window = 0;
   R zq[4] = {R(0), R(0), R(0), R(0)};     // 1D models: normals of the lane's next step group
@@ -633,9 +640,16 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
     const unsigned need = __ballot_sync(kFull, !active && !drained);
     if (need) {
       const int leader = __ffs(need) - 1;
-      unsigned long long base = 0;
-      if (lane == leader) base = atomicAdd(&a.ctl->ticket[MODEL], (unsigned long long)__popc(need));
-      base = __shfl_sync(kFull, base, leader);
+      const unsigned long long total = gpre[ne];
+      const Spread spread = spread_lanes<R>(total, gridDim.x, (unsigned)a.ctas_per_sm, warps);
+      unsigned long long base = ((unsigned long long)warp * gridDim.x + blockIdx.x) * spread.lanes;
+      if (window > 1u) {
+        if (lane == leader) {
+          const unsigned long long dealt = (unsigned long long)gridDim.x * spread.warps * spread.lanes;
+          base = dealt + atomicAdd(&a.ctl->ticket[MODEL], (unsigned long long)__popc(need));
+        }
+        base = __shfl_sync(kFull, base, leader);
+      }
       if (Prefetch<MODEL>::value && base + (unsigned long long)__popc(need) >= total) exhausted = true;
       if (!active && !drained) {
         const unsigned long long t = base + __popc(need & lanemask_lt());
@@ -743,11 +757,6 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
       // at a group boundary), so the results are identical.
       const unsigned act = __ballot_sync(kFull, active);
       const int na = __popc(act);
-      if (!exhausted && spread.lanes < 32u) {     // a small run hands out its tickets at once
-        unsigned long long t = 0;
-        if (lane == 0) t = *(volatile unsigned long long *)&a.ctl->ticket[MODEL];
-        exhausted = __shfl_sync(kFull, t, 0) >= total;
-      }
       if (exhausted && na <= kCoopLanes) {
         const int G = 32 / na;
         const int jt = lane % na, gi = lane / na;     // this lane draws group gi of the jt-th running lane
