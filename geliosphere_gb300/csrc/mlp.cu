@@ -13,11 +13,13 @@
 #include <cstring>
 #include <mutex>
 #include <random>
+#include <thread>
 #include <vector>
 
 #include "gelio.h"
 #include "alloc.cuh"
 #include "mlp_kernels.cuh"
+#include "mlp_train.cuh"
 
 int gelio_internal_device(const gelio_ctx *c);
 
@@ -60,6 +62,19 @@ bool make_map(CUtensorMap *m, const void *ptr, uint64_t inner, uint64_t outer, u
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// BF16 tensor [members][outer][inner], boxes of {64, box_outer, 1}.
+bool make_map3(CUtensorMap *m, const void *ptr, uint64_t inner, uint64_t outer, uint64_t members, uint32_t box_outer) {
+  EncodeFn f = encode_fn();
+  if (!f) return false;
+  const cuuint64_t dims[3] = {inner, outer, members};
+  const cuuint64_t strides[2] = {inner * 2, inner * outer * 2};
+  const cuuint32_t box[3] = {64, box_outer, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return f(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void *>(ptr), dims, strides, box, estr,
+           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // Local interstellar spectra of the evaluators (TwoDimensionBpResults.cpp:50-60),
 // for the training targets.
 double lis(int which, double T) {
@@ -93,10 +108,21 @@ uint64_t splitmix(uint64_t &x) {
 
 struct Member {
   float *P = nullptr, *M1 = nullptr, *M2 = nullptr;
-  bf16 *W1 = nullptr, *W[3] = {}, *WT[3] = {};
-  CUtensorMap mW1, mW[3], mWT[3];
+  bf16 *W1 = nullptr, *W[3] = {}, *WT[3] = {};       // in the ensemble's arrays
+  CUtensorMap mW1, mW[3];
   int adam_t = 0;
   bool trained = false;
+};
+
+// Activations and gradients of a group of G members training at once
+// (mlp_train.cuh), allocated by the first training step or gradient.
+struct TrainBuffers {
+  int G = 0;
+  bf16 *X0 = nullptr, *Z[4] = {}, *X[4] = {}, *dH[4] = {};
+  float *yhat = nullptr, *y = nullptr, *dy = nullptr, *partial = nullptr, *cls = nullptr, *cls5 = nullptr;
+  float *loss_part = nullptr;
+  CUtensorMap aX0, aX[3], adH[4];        // row tiles of 128 (K-major operands)
+  CUtensorMap bX0, bX[3], bdH[4];        // boxes of 64 rows (MN-major operands of dW)
 };
 
 }  // namespace
@@ -109,19 +135,22 @@ struct gelio_surrogate {
   gelio_ctx *ctx = nullptr;
   gelio_surrogate_opts o{};
   int device = 0, sm_count = 0, rows = 0;   // rows = batch rows
-  int k_split = 256, splits = 0;
   cudaStream_t stream = nullptr;
   std::vector<Member> mem;
-  // activations and gradients of one batch
-  bf16 *X0 = nullptr, *X0T = nullptr, *Z[4] = {}, *X[3] = {}, *XT[4] = {}, *dH[4] = {}, *dHT[4] = {};
-  float *yhat = nullptr, *y = nullptr, *dy = nullptr, *partial = nullptr, *grad = nullptr, *loss_part = nullptr;
+  // BF16 operand copies of every member's weights, [members][256][fan-in]
+  bf16 *W1 = nullptr, *W[3] = {}, *WT[3] = {};
+  CUtensorMap tW1, tW[3], tWT[3];
+  TrainBuffers tb;
+  float *grad = nullptr;     // gelio_surrogate_gradient's result
   float *step_loss = nullptr;
-  int step_loss_cap = 0;
+  size_t step_loss_cap = 0;
   int *ident = nullptr;      // 0, 1, ..., rows - 1
-  int *order = nullptr;      // this epoch's shuffled row order
+  int *order = nullptr;      // this epoch's shuffled row orders, [group][rows of the set]
   size_t order_cap = 0;
+  int *h_order = nullptr;    // pinned staging of two epochs' orders
+  size_t h_order_cap = 0;
+  cudaEvent_t ev_copy[2] = {nullptr, nullptr};   // an epoch's orders have left the staging
   unsigned *error = nullptr;
-  CUtensorMap mX0, mX[3], mdH[4], mdHT[4], mX0T, mXT[3];
   // training rows (host) and their device copy
   std::vector<float> feats, targ;
   float *d_feats = nullptr, *d_targ = nullptr;
@@ -143,7 +172,6 @@ struct gelio_surrogate {
   int qrows = 0;
   bf16 *Q0 = nullptr, *Q[2] = {};
   float *qy = nullptr;
-  int *qident = nullptr;
   CUtensorMap mQ0, mQ[2];
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;    // device time of the last inference
   double last_ms = 0.0, last_flop = 0.0;
@@ -170,9 +198,7 @@ template <int MODE>
 int launch_gemm(gelio_surrogate *s, const CUtensorMap &A, const CUtensorMap &B, GemmArgs a) {
   a.error = s->error;
   a.timeout_ns = 2000000000ull;
-  if (a.splits < 1) a.splits = 1;
-  if (a.k_per_split <= 0) a.k_per_split = a.K;
-  const int tiles = ((a.M + kTileM - 1) / kTileM) * a.splits;
+  const int tiles = (a.M + kTileM - 1) / kTileM;
   const int grid = std::max(1, std::min(tiles, s->sm_count));
   k_mlp_gemm<MODE><<<grid, kGemmThreads, kGemmSmem, s->stream>>>(A, B, a);
   return cuda_status(cudaGetLastError());
@@ -187,12 +213,12 @@ int set_smem_attrs() {
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
     };
-    set((const void *)k_mlp_gemm<FWD>);
-    set((const void *)k_mlp_gemm<FWD_LAST>);
     set((const void *)k_mlp_gemm<INFER>);
     set((const void *)k_mlp_gemm<INFER_LAST>);
-    set((const void *)k_mlp_gemm<DX>);
-    set((const void *)k_mlp_gemm<DW>);
+    set((const void *)k_train_gemm<FWD>);
+    set((const void *)k_train_gemm<FWD_LAST>);
+    set((const void *)k_train_gemm<DX>);
+    set((const void *)k_train_gemm<DW>);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute((const void *)k_mlp_infer_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kFusedSmem);
@@ -201,20 +227,27 @@ int set_smem_attrs() {
   return rc;
 }
 
+void free_train(TrainBuffers &t) {
+  auto f = [](void *p) { if (p) cudaFree(p); };
+  f(t.X0);
+  for (int i = 0; i < 4; ++i) { f(t.Z[i]); f(t.X[i]); f(t.dH[i]); }
+  f(t.yhat); f(t.y); f(t.dy); f(t.partial); f(t.cls); f(t.cls5); f(t.loss_part);
+  t = TrainBuffers();
+}
+
 void free_all(gelio_surrogate *s) {
   auto f = [](void *p) { if (p) cudaFree(p); };
-  for (auto &m : s->mem) {
-    f(m.P); f(m.M1); f(m.M2); f(m.W1);
-    for (int i = 0; i < 3; ++i) { f(m.W[i]); f(m.WT[i]); }
-  }
-  f(s->X0); f(s->X0T);
-  for (int i = 0; i < 4; ++i) { f(s->Z[i]); f(s->XT[i]); f(s->dH[i]); f(s->dHT[i]); }
-  for (int i = 0; i < 3; ++i) f(s->X[i]);
-  f(s->yhat); f(s->y); f(s->dy); f(s->partial); f(s->grad); f(s->loss_part); f(s->step_loss);
+  for (auto &m : s->mem) { f(m.P); f(m.M1); f(m.M2); }
+  f(s->W1);
+  for (int i = 0; i < 3; ++i) { f(s->W[i]); f(s->WT[i]); }
+  free_train(s->tb);
+  f(s->grad); f(s->step_loss);
   f(s->ident); f(s->order); f(s->error); f(s->d_feats); f(s->d_targ); f(s->d_query); f(s->d_yq);
-  f(s->Q0); f(s->Q[0]); f(s->Q[1]); f(s->qy); f(s->qident);
+  f(s->Q0); f(s->Q[0]); f(s->Q[1]); f(s->qy);
   f(s->d_pup); f(s->d_py); f(s->d_pstat);
   if (s->h_pstage) cudaFreeHost(s->h_pstage);
+  if (s->h_order) cudaFreeHost(s->h_order);
+  for (auto &e : s->ev_copy) if (e) cudaEventDestroy(e);
   if (s->ev0) cudaEventDestroy(s->ev0);
   if (s->ev1) cudaEventDestroy(s->ev1);
   if (s->stream) cudaStreamDestroy(s->stream);
@@ -238,64 +271,127 @@ int check_error(gelio_surrogate *s) {
   return GELIO_OK;
 }
 
-// Forward (training form) + backward of member m on the gathered batch;
-// gradient into s->grad, squared-error sum into *loss_slot (device).
-int forward_backward(gelio_surrogate *s, Member &m, int n_valid, float *loss_slot) {
+// Members that train at once: as many as keep the group's activations near
+// 2 GiB (16 members of 16,384 rows; past 2^18 rows one, as much as a member
+// always took), within the ensemble.
+int group_size(const gelio_surrogate *s) {
+  const size_t R = (size_t)s->rows;
+  const size_t per = R * kInPad * 2 + 12 * R * kWidth * 2 + (R / kSplitRows) * kWidth * kWidth * 4;
+  return (int)std::max<size_t>(1, std::min(s->mem.size(), ((size_t)2 << 30) / per));
+}
+
+// Training buffers for G members; a refused or failed allocation leaves those
+// there were.
+int ensure_train(gelio_surrogate *s, int G) {
+  if (G <= s->tb.G) return GELIO_OK;
+  const size_t R = (size_t)s->rows, g = (size_t)G;
+  TrainBuffers t;
+  cudaError_t e = cudaSuccess;
+  auto alloc = [&](auto **p, size_t n) {
+    if (e == cudaSuccess) e = gelio::dev_malloc(p, n * sizeof(**p));
+  };
+  alloc(&t.X0, g * R * kInPad);
+  for (int i = 0; i < 4; ++i) {
+    alloc(&t.Z[i], g * R * kWidth);
+    alloc(&t.X[i], g * R * kWidth);
+    alloc(&t.dH[i], g * R * kWidth);
+  }
+  alloc(&t.yhat, g * R);
+  alloc(&t.y, g * R);
+  alloc(&t.dy, g * R);
+  alloc(&t.partial, g * (R / kSplitRows) * kWidth * kWidth);
+  alloc(&t.cls, g * kClasses * kWidth);
+  alloc(&t.cls5, g * kClasses * kWidth);
+  alloc(&t.loss_part, g * (R / kHeadRows));
+  if (e == cudaSuccess) e = cudaMemsetAsync(t.X0, 0, g * R * kInPad * 2, s->stream);   // the padding columns
+  bool ok = e == cudaSuccess;
+  ok = ok && make_map3(&t.aX0, t.X0, kInPad, R, g, kTileM) && make_map3(&t.bX0, t.X0, kInPad, R, g, kChunk);
+  for (int i = 0; i < 4; ++i) {
+    if (i < 3)
+      ok = ok && make_map3(&t.aX[i], t.X[i], kWidth, R, g, kTileM) && make_map3(&t.bX[i], t.X[i], kWidth, R, g, kChunk);
+    ok = ok && make_map3(&t.adH[i], t.dH[i], kWidth, R, g, kTileM) && make_map3(&t.bdH[i], t.dH[i], kWidth, R, g, kChunk);
+  }
+  if (!ok) {
+    free_train(t);
+    return e != cudaSuccess ? cuda_status(e) : GELIO_ERR_CUDA;
+  }
+  t.G = G;
+  if (s->tb.G) SUR_TRY(cudaStreamSynchronize(s->stream));
+  free_train(s->tb);
+  s->tb = t;
+  return GELIO_OK;
+}
+
+template <int MODE>
+int launch_train(gelio_surrogate *s, const CUtensorMap &A, const CUtensorMap &B, const TrainArgs &a) {
+  int grid;
+  if (MODE == DW) grid = std::min(s->sm_count, a.G * (a.rows / kSplitRows) * 2);
+  else grid = a.G * std::max(1, std::min(s->sm_count / a.G, a.rows / kTileM));   // the same CTAs for each slot
+  k_train_gemm<MODE><<<grid, kGemmThreads, kGemmSmem, s->stream>>>(A, B, a);
+  return cuda_status(cudaGetLastError());
+}
+
+// One step of members [m0, m0 + G) on the gathered batches: forward, backward
+// and, layer by layer from the top, the update that u describes (Adam's step,
+// or the gradient of one member).  A layer's dX runs before its weights change.
+int train_step(gelio_surrogate *s, int m0, int G, int n_valid, UpdateArgs &u) {
+  TrainBuffers &t = s->tb;
   const int R = s->rows;
   int rc;
-  GemmArgs a{};
-  a.M = R; a.N = kWidth; a.ldt = R; a.splits = 1;
+  TrainArgs a{};
+  a.rows = R; a.G = G; a.m0 = m0; a.N = kWidth;
+  a.error = s->error; a.timeout_ns = 2000000000ull;
+  for (int g = 0; g < G; ++g) a.P[g] = s->mem[m0 + g].P;
   // forward
-  a.K = kInPad; a.bias = m.P + kOffB1; a.z_out = s->Z[0]; a.x_out = s->X[0]; a.xt_out = s->XT[0];
-  if ((rc = launch_gemm<FWD>(s, s->mX0, m.mW1, a)) != GELIO_OK) return rc;
-  a.K = kWidth; a.bias = m.P + kOffB2; a.z_out = s->Z[1]; a.x_out = s->X[1]; a.xt_out = s->XT[1];
-  if ((rc = launch_gemm<FWD>(s, s->mX[0], m.mW[0], a)) != GELIO_OK) return rc;
-  a.bias = m.P + kOffB3; a.z_out = s->Z[2]; a.x_out = s->X[2]; a.xt_out = s->XT[2];
-  if ((rc = launch_gemm<FWD>(s, s->mX[1], m.mW[1], a)) != GELIO_OK) return rc;
-  a.bias = m.P + kOffB4; a.z_out = s->Z[3]; a.x_out = nullptr; a.xt_out = s->XT[3];
-  a.w5 = m.P + kOffW5; a.b5 = m.P + kOffB5; a.y_out = s->yhat;
-  SUR_TRY(cudaMemsetAsync(s->yhat, 0, (size_t)R * 4, s->stream));
-  if ((rc = launch_gemm<FWD_LAST>(s, s->mX[2], m.mW[2], a)) != GELIO_OK) return rc;
+  a.K = kInPad; a.off_bias = kOffB1; a.z_out = t.Z[0]; a.x_out = t.X[0];
+  if ((rc = launch_train<FWD>(s, t.aX0, s->tW1, a)) != GELIO_OK) return rc;
+  a.K = kWidth; a.off_bias = kOffB2; a.z_out = t.Z[1]; a.x_out = t.X[1];
+  if ((rc = launch_train<FWD>(s, t.aX[0], s->tW[0], a)) != GELIO_OK) return rc;
+  a.off_bias = kOffB3; a.z_out = t.Z[2]; a.x_out = t.X[2];
+  if ((rc = launch_train<FWD>(s, t.aX[1], s->tW[1], a)) != GELIO_OK) return rc;
+  a.off_bias = kOffB4; a.z_out = t.Z[3]; a.x_out = t.X[3]; a.y_out = t.yhat;
+  if ((rc = launch_train<FWD_LAST>(s, t.aX[2], s->tW[2], a)) != GELIO_OK) return rc;
   // head
-  const int hb = (R + kThreads - 1) / kThreads;
-  k_head_backward<<<hb, kThreads, 0, s->stream>>>(s->yhat, s->y, n_valid, R, m.P + kOffW5, s->Z[3], s->dH[3],
-                                                   s->dHT[3], s->dy, s->loss_part);
-  k_sum_f32<<<1, 256, 0, s->stream>>>(s->loss_part, hb, loss_slot);
-  k_rowsum_bf16<<<kWidth, 256, 0, s->stream>>>(s->XT[3], R, s->dy, s->grad + kOffW5);
-  k_sum_f32<<<1, 256, 0, s->stream>>>(s->dy, R, s->grad + kOffB5);
+  k_head_backward<<<dim3(R / kHeadRows, G), 256, 0, s->stream>>>(t.yhat, t.y, n_valid, R, a, t.Z[3], t.dH[3], t.dy,
+                                                                 t.loss_part);
+  k_class_sums<<<dim3(kClasses / 32, kWidth / 64, G), 256, 0, s->stream>>>(t.X[3], t.dy, R, t.cls5);
   SUR_TRY(cudaGetLastError());
   // hidden layers, top down
   const int offW[4] = {kOffW1, kOffW2, kOffW3, kOffW4};
   const int offB[4] = {kOffB1, kOffB2, kOffB3, kOffB4};
-  for (int l = 4; l >= 1; --l) {
-    const int li = l - 1;
-    GemmArgs d{};
-    d.M = kWidth; d.K = R; d.k_per_split = s->k_split; d.splits = s->splits; d.partial = s->partial; d.ldt = R;
-    d.N = (l == 1) ? kInPad : kWidth;
-    const CUtensorMap &Bm = (l == 1) ? s->mX0T : s->mXT[l - 2];
-    if ((rc = launch_gemm<DW>(s, s->mdHT[li], Bm, d)) != GELIO_OK) return rc;
-    const int fan_in = (l == 1) ? kFeatures : kWidth;
-    k_reduce_dw<<<(kWidth * fan_in + 255) / 256, 256, 0, s->stream>>>(s->partial, s->splits, d.N, fan_in,
-                                                                      s->grad + offW[li]);
-    k_rowsum_bf16<<<kWidth, 256, 0, s->stream>>>(s->dHT[li], R, nullptr, s->grad + offB[li]);
+  u.rows = R; u.splits = R / kSplitRows; u.partial = t.partial; u.cls = t.cls; u.m0 = m0;
+  for (int li = 3; li >= 0; --li) {
+    k_class_sums<<<dim3(kClasses / 32, kWidth / 64, G), 256, 0, s->stream>>>(t.dH[li], nullptr, R, t.cls);
     SUR_TRY(cudaGetLastError());
-    if (l >= 2) {
-      GemmArgs x{};
-      x.M = R; x.N = kWidth; x.K = kWidth; x.splits = 1; x.ldt = R;
-      x.z_prev = s->Z[li - 1]; x.dh_out = s->dH[li - 1]; x.dht_out = s->dHT[li - 1];
-      if ((rc = launch_gemm<DX>(s, s->mdH[li], m.mWT[li - 1], x)) != GELIO_OK) return rc;
+    if (li > 0) {
+      a.K = kWidth; a.N = kWidth; a.z_prev = t.Z[li - 1]; a.dh_out = t.dH[li - 1];
+      if ((rc = launch_train<DX>(s, t.adH[li], s->tWT[li - 1], a)) != GELIO_OK) return rc;
     }
+    a.K = kSplitRows; a.N = (li == 0) ? kInPad : kWidth; a.partial = t.partial;
+    if ((rc = launch_train<DW>(s, t.bdH[li], li == 0 ? t.bX0 : t.bX[li - 1], a)) != GELIO_OK) return rc;
+    u.N = a.N;
+    u.fan_in = (li == 0) ? kFeatures : kWidth;
+    u.off_w = offW[li];
+    u.off_b = offB[li];
+    u.cls5 = (li == 3) ? t.cls5 : nullptr;
+    u.dy = t.dy;
+    u.loss_part = t.loss_part;
+    u.w = (li == 0) ? s->W1 : s->W[li - 1];
+    u.wt = (li == 0) ? nullptr : s->WT[li - 1];
+    u.w_ld = (li == 0) ? kInPad : kWidth;
+    const int blocks = 8 * ((u.fan_in + 31) / 32) + 8 + (li == 3 ? 9 : 0);
+    k_update<<<dim3(blocks, G), 256, 0, s->stream>>>(u);
+    SUR_TRY(cudaGetLastError());
   }
   return GELIO_OK;
 }
-
 
 // Inference of member m on the first `M` rows of the inference batch
 // (M a multiple of 128); outputs in s->qy.
 int forward_infer_q(gelio_surrogate *s, Member &m, int M) {
   int rc;
   GemmArgs a{};
-  a.M = M; a.N = kWidth; a.ldt = s->qrows; a.splits = 1;
+  a.M = M;
   a.K = kInPad; a.bias = m.P + kOffB1; a.x_out = s->Q[0];
   if ((rc = launch_gemm<INFER>(s, s->mQ0, m.mW1, a)) != GELIO_OK) return rc;
   a.K = kWidth; a.bias = m.P + kOffB2; a.x_out = s->Q[1];
@@ -305,13 +401,6 @@ int forward_infer_q(gelio_surrogate *s, Member &m, int M) {
   a.bias = m.P + kOffB4; a.x_out = nullptr; a.w5 = m.P + kOffW5; a.b5 = m.P + kOffB5; a.y_out = s->qy;
   SUR_TRY(cudaMemsetAsync(s->qy, 0, (size_t)M * 4, s->stream));
   return launch_gemm<INFER_LAST>(s, s->mQ[0], m.mW[2], a);
-}
-
-// Upload x rows [n][7] to the training-row buffer tail used as scratch and
-// gather them (identity order, padding to the batch).
-int stage_rows(gelio_surrogate *s, float *d_x, float *d_t, int n) {
-  k_gather<<<(s->rows + 127) / 128, 128, 0, s->stream>>>(d_x, d_t, s->ident, n, 0, s->rows, s->X0, s->X0T, s->y);
-  return cuda_status(cudaGetLastError());
 }
 
 bool valid_member(gelio_surrogate *s, int m) { return s && m >= 0 && m < (int)s->mem.size(); }
@@ -337,8 +426,7 @@ int infer_rows(gelio_surrogate *s, int m0, int m1, const float *x, size_t n, flo
     const int c = (int)std::min<size_t>((size_t)s->qrows, n - off);
     const int M = (c + kTileM - 1) / kTileM * kTileM;     // only the tiles this chunk needs
     padded += (size_t)M;
-    k_gather<<<(M + 127) / 128, 128, 0, s->stream>>>(s->d_query + off * kFeatures, nullptr, s->qident, c, 0, M,
-                                                     s->Q0, nullptr, nullptr);
+    k_query_rows<<<(M + 127) / 128, 128, 0, s->stream>>>(s->d_query + off * kFeatures, c, M, s->Q0);
     SUR_TRY(cudaGetLastError());
     for (size_t e = 0; e < E; ++e) {
       const int rc = forward_infer_q(s, s->mem[m0 + e], M);
@@ -358,6 +446,92 @@ int infer_rows(gelio_surrogate *s, int m0, int m1, const float *x, size_t n, flo
                    ((double)kInPad * kWidth + 3.0 * kWidth * kWidth + (double)kWidth);
   }
   return rc;
+}
+
+// The epochs of members [m0, m0 + g).  Each member has its own shuffles; the
+// host makes the next epoch's while the device runs this one's, a thread a
+// member (a shuffle of 200,000 rows takes 1.5 ms, as long as the device's
+// epoch).  Losses of the last epoch's steps: sl[member][step].
+int train_group(gelio_surrogate *s, int m0, int g, int epochs, int steps, long long total, size_t nrow, float *sl) {
+  const int R = s->rows;
+  std::vector<std::vector<int>> order(g, std::vector<int>(nrow));
+  std::vector<std::mt19937_64> rng;
+  for (int k = 0; k < g; ++k) {
+    rng.emplace_back(s->o.seed * 1000003ull + (unsigned)(m0 + k));
+    for (size_t i = 0; i < nrow; ++i) order[k][i] = (int)i;
+  }
+  auto shuffle = [&](int k, int ep) {
+    std::shuffle(order[k].begin(), order[k].end(), rng[k]);
+    std::memcpy(s->h_order + ((size_t)(ep & 1) * g + k) * nrow, order[k].data(), nrow * sizeof(int));
+  };
+  std::vector<std::thread> workers;
+  auto start_shuffles = [&](int ep) {
+    for (int k = 0; k < g; ++k) {
+      bool run = false;
+      try {
+        workers.emplace_back(shuffle, k, ep);
+        run = true;
+      } catch (...) {          // no thread to be had: shuffled here
+      }
+      if (!run) shuffle(k, ep);
+    }
+  };
+  auto join = [&] {
+    for (auto &w : workers) w.join();
+    workers.clear();
+  };
+  int rc = GELIO_OK;
+  UpdateArgs u{};
+  u.b1 = 0.9f; u.b2 = 0.999f; u.eps = 1e-8f;
+  for (int k = 0; k < g; ++k) {
+    u.P[k] = s->mem[m0 + k].P;
+    u.M1[k] = s->mem[m0 + k].M1;
+    u.M2[k] = s->mem[m0 + k].M2;
+  }
+  u.loss_stride = steps;
+  auto epoch = [&](int ep) -> int {
+    SUR_TRY(cudaMemcpyAsync(s->order, s->h_order + (size_t)(ep & 1) * g * nrow, (size_t)g * nrow * sizeof(int),
+                            cudaMemcpyHostToDevice, s->stream));
+    SUR_TRY(cudaEventRecord(s->ev_copy[ep & 1], s->stream));
+    if (ep + 1 < epochs) {
+      // the other half of the staging was copied an epoch ago
+      if (ep > 0) SUR_TRY(cudaEventSynchronize(s->ev_copy[(ep + 1) & 1]));
+      start_shuffles(ep + 1);
+    }
+    for (int st = 0; st < steps; ++st) {
+      const long long off = (long long)st * R;
+      const int nv = (int)std::min<long long>(R, (long long)nrow - off);
+      k_gather<<<dim3((R + 127) / 128, g), 128, 0, s->stream>>>(s->d_feats, s->d_targ, s->order, (long long)nrow, off,
+                                                                R, s->tb.X0, s->tb.y, s->tb.yhat);
+      SUR_TRY(cudaGetLastError());
+      const long long t = (long long)ep * steps + st;
+      const double frac = total > 1 ? (double)t / (double)(total - 1) : 1.0;
+      const float lr = (float)(s->o.lr_final + 0.5 * (s->o.lr - s->o.lr_final) * (1.0 + std::cos(M_PI * frac)));
+      for (int k = 0; k < g; ++k) {
+        Member &m = s->mem[m0 + k];
+        ++m.adam_t;
+        u.lr[k] = lr;
+        u.c1[k] = 1.0f - std::pow(0.9f, (float)m.adam_t);
+        u.c2[k] = 1.0f - std::pow(0.999f, (float)m.adam_t);
+      }
+      u.loss = s->step_loss + st;
+      const int r = train_step(s, m0, g, nv, u);
+      if (r != GELIO_OK) return r;
+    }
+    return GELIO_OK;
+  };
+  if (epochs > 0) start_shuffles(0);
+  for (int ep = 0; ep < epochs && rc == GELIO_OK; ++ep) {
+    join();
+    rc = epoch(ep);
+  }
+  join();
+  if (rc != GELIO_OK) {
+    cudaStreamSynchronize(s->stream);
+    return rc;
+  }
+  SUR_TRY(cudaMemcpyAsync(sl, s->step_loss, sizeof(float) * (size_t)g * steps, cudaMemcpyDeviceToHost, s->stream));
+  return check_error(s);
 }
 
 void default_opts(gelio_surrogate_opts &o) {
@@ -418,7 +592,6 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
   s->o = o;
   s->device = gelio_internal_device(ctx);
   s->rows = o.batch_rows;
-  s->splits = s->rows / s->k_split;
   int rc = GELIO_OK;
   auto fail = [&](int r) { free_all(s); delete s; return r; };
   if (cudaSetDevice(s->device) != cudaSuccess) return fail(GELIO_ERR_NO_DEVICE);
@@ -428,6 +601,8 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
   cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, s->device);
   if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(GELIO_ERR_CUDA);
   if (cudaEventCreate(&s->ev0) != cudaSuccess || cudaEventCreate(&s->ev1) != cudaSuccess) return fail(GELIO_ERR_CUDA);
+  for (auto &e : s->ev_copy)
+    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(GELIO_ERR_CUDA);
   const size_t R = (size_t)s->rows;
   auto alloc = [&](void **p, size_t bytes) {
     if (rc != GELIO_OK) return;
@@ -435,21 +610,7 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
     if (e == cudaSuccess) e = cudaMemset(*p, 0, bytes);
     rc = cuda_status(e);
   };
-  alloc((void **)&s->X0, R * kInPad * 2);
-  alloc((void **)&s->X0T, (size_t)kInPad * R * 2);
-  for (int i = 0; i < 4; ++i) {
-    alloc((void **)&s->Z[i], R * kWidth * 2);
-    alloc((void **)&s->XT[i], R * kWidth * 2);
-    alloc((void **)&s->dH[i], R * kWidth * 2);
-    alloc((void **)&s->dHT[i], R * kWidth * 2);
-  }
-  for (int i = 0; i < 3; ++i) alloc((void **)&s->X[i], R * kWidth * 2);
-  alloc((void **)&s->yhat, R * 4);
-  alloc((void **)&s->y, R * 4);
-  alloc((void **)&s->dy, R * 4);
-  alloc((void **)&s->partial, (size_t)s->splits * kWidth * kWidth * 4);
   alloc((void **)&s->grad, (size_t)kParams * 4);
-  alloc((void **)&s->loss_part, (R / kThreads + 1) * 4);
   alloc((void **)&s->ident, R * 4);
   s->qrows = std::max(s->rows, 65536);
   const size_t Rq = (size_t)s->qrows;
@@ -457,37 +618,35 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
   alloc((void **)&s->Q[0], Rq * kWidth * 2);
   alloc((void **)&s->Q[1], Rq * kWidth * 2);
   alloc((void **)&s->qy, Rq * 4);
-  alloc((void **)&s->qident, Rq * 4);
   alloc((void **)&s->error, 4);
-  s->mem.resize(o.members);
-  for (auto &m : s->mem) {
+  const size_t E = (size_t)o.members;
+  alloc((void **)&s->W1, E * kWidth * kInPad * 2);
+  for (int i = 0; i < 3; ++i) {
+    alloc((void **)&s->W[i], E * kWidth * kWidth * 2);
+    alloc((void **)&s->WT[i], E * kWidth * kWidth * 2);
+  }
+  s->mem.resize(E);
+  for (size_t e = 0; e < E; ++e) {
+    Member &m = s->mem[e];
     alloc((void **)&m.P, (size_t)kParams * 4);
     alloc((void **)&m.M1, (size_t)kParams * 4);
     alloc((void **)&m.M2, (size_t)kParams * 4);
-    alloc((void **)&m.W1, (size_t)kWidth * kInPad * 2);
+    m.W1 = s->W1 + e * kWidth * kInPad;
     for (int i = 0; i < 3; ++i) {
-      alloc((void **)&m.W[i], (size_t)kWidth * kWidth * 2);
-      alloc((void **)&m.WT[i], (size_t)kWidth * kWidth * 2);
+      m.W[i] = s->W[i] + e * kWidth * kWidth;
+      m.WT[i] = s->WT[i] + e * kWidth * kWidth;
     }
   }
   if (rc != GELIO_OK) return fail(rc);
-  bool ok = make_map(&s->mX0, s->X0, kInPad, R, kTileM) && make_map(&s->mX0T, s->X0T, R, kInPad, kInPad);
-  for (int i = 0; i < 3; ++i) {
-    ok = ok && make_map(&s->mX[i], s->X[i], kWidth, R, kTileM);
-    ok = ok && make_map(&s->mXT[i], s->XT[i], R, kWidth, kWidth);
-  }
-  ok = ok && make_map(&s->mQ0, s->Q0, kInPad, Rq, kTileM) && make_map(&s->mQ[0], s->Q[0], kWidth, Rq, kTileM) &&
-       make_map(&s->mQ[1], s->Q[1], kWidth, Rq, kTileM);
-  for (int i = 0; i < 4; ++i) {
-    ok = ok && make_map(&s->mdH[i], s->dH[i], kWidth, R, kTileM);
-    ok = ok && make_map(&s->mdHT[i], s->dHT[i], R, kWidth, kTileM);
-  }
+  bool ok = make_map(&s->mQ0, s->Q0, kInPad, Rq, kTileM) && make_map(&s->mQ[0], s->Q[0], kWidth, Rq, kTileM) &&
+            make_map(&s->mQ[1], s->Q[1], kWidth, Rq, kTileM);
+  ok = ok && make_map3(&s->tW1, s->W1, kInPad, kWidth, E, kWidth);
+  for (int i = 0; i < 3; ++i)
+    ok = ok && make_map3(&s->tW[i], s->W[i], kWidth, kWidth, E, kWidth) &&
+         make_map3(&s->tWT[i], s->WT[i], kWidth, kWidth, E, kWidth);
   for (auto &m : s->mem) {
     ok = ok && make_map(&m.mW1, m.W1, kInPad, kWidth, kWidth);
-    for (int i = 0; i < 3; ++i) {
-      ok = ok && make_map(&m.mW[i], m.W[i], kWidth, kWidth, kWidth);
-      ok = ok && make_map(&m.mWT[i], m.WT[i], kWidth, kWidth, kWidth);
-    }
+    for (int i = 0; i < 3; ++i) ok = ok && make_map(&m.mW[i], m.W[i], kWidth, kWidth, kWidth);
   }
   if (!ok) return fail(GELIO_ERR_CUDA);
   // initial weights: uniform(+-sqrt(3 / fan_in)), zero biases
@@ -512,10 +671,6 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
     std::vector<int> id(R);
     for (size_t i = 0; i < R; ++i) id[i] = (int)i;
     if (cudaMemcpy(s->ident, id.data(), R * 4, cudaMemcpyHostToDevice) != cudaSuccess) return fail(GELIO_ERR_CUDA);
-    std::vector<int> idq(Rq);
-    for (size_t i = 0; i < Rq; ++i) idq[i] = (int)i;
-    if (cudaMemcpy(s->qident, idq.data(), Rq * 4, cudaMemcpyHostToDevice) != cudaSuccess)
-      return fail(GELIO_ERR_CUDA);
   }
   if (cudaStreamSynchronize(s->stream) != cudaSuccess) return fail(GELIO_ERR_CUDA);
   *out = s;
@@ -590,59 +745,44 @@ int32_t gelio_surrogate_train(gelio_surrogate *s, int32_t epochs, float *last_lo
   }
   const int R = s->rows;
   const int steps = (int)std::max<size_t>(1, nrow / (size_t)R);
-  if (steps > s->step_loss_cap) {
+  const int E = (int)s->mem.size(), G = group_size(s);
+  int rc = ensure_train(s, G);
+  if (rc != GELIO_OK) return rc;
+  if ((size_t)G * steps > s->step_loss_cap) {
     if (s->step_loss) cudaFree(s->step_loss);
     s->step_loss = nullptr;
-    SUR_TRY(gelio::dev_malloc(&s->step_loss, sizeof(float) * steps));
-    s->step_loss_cap = steps;
+    s->step_loss_cap = 0;
+    SUR_TRY(gelio::dev_malloc(&s->step_loss, sizeof(float) * G * steps));
+    s->step_loss_cap = (size_t)G * steps;
   }
-  if (nrow > s->order_cap) {
+  if (G * nrow > s->order_cap) {
     if (s->order) cudaFree(s->order);
     s->order = nullptr;
-    SUR_TRY(gelio::dev_malloc(&s->order, nrow * sizeof(int)));
-    s->order_cap = nrow;
+    s->order_cap = 0;
+    SUR_TRY(gelio::dev_malloc(&s->order, G * nrow * sizeof(int)));
+    s->order_cap = G * nrow;
+  }
+  if (2 * G * nrow > s->h_order_cap) {
+    if (s->h_order) cudaFreeHost(s->h_order);
+    s->h_order = nullptr;
+    s->h_order_cap = 0;
+    SUR_TRY(gelio::pinned_malloc(&s->h_order, 2 * G * nrow * sizeof(int)));
+    s->h_order_cap = 2 * G * nrow;
   }
   const long long total = (long long)epochs * steps;
-  std::vector<int> order(nrow);
-  std::vector<float> sl(steps);
-  for (size_t e = 0; e < s->mem.size(); ++e) {
-    Member &m = s->mem[e];
-    std::mt19937_64 rng(s->o.seed * 1000003ull + e);
-    for (size_t i = 0; i < nrow; ++i) order[i] = (int)i;
-    double loss = 0.0;
-    for (int ep = 0; ep < epochs; ++ep) {
-      std::shuffle(order.begin(), order.end(), rng);
-      // the host order is reshuffled next epoch: the copy completes first
-      SUR_TRY(cudaMemcpyAsync(s->order, order.data(), nrow * sizeof(int), cudaMemcpyHostToDevice, s->stream));
-      SUR_TRY(cudaStreamSynchronize(s->stream));
-      for (int st = 0; st < steps; ++st) {
-        const long long off = (long long)st * R;
-        const int nv = (int)std::min<long long>(R, (long long)nrow - off);
-        k_gather<<<(R + 127) / 128, 128, 0, s->stream>>>(s->d_feats, s->d_targ, s->order, (long long)nrow, off, R,
-                                                         s->X0, s->X0T, s->y);
-        int rc = forward_backward(s, m, nv, s->step_loss + st);
-        if (rc != GELIO_OK) return rc;
-        const long long t = (long long)ep * steps + st;
-        const double frac = total > 1 ? (double)t / (double)(total - 1) : 1.0;
-        const float lr = (float)(s->o.lr_final + 0.5 * (s->o.lr - s->o.lr_final) * (1.0 + std::cos(M_PI * frac)));
-        ++m.adam_t;
-        const float c1 = 1.0f - std::pow(0.9f, (float)m.adam_t), c2 = 1.0f - std::pow(0.999f, (float)m.adam_t);
-        k_adam<<<(kParams + 255) / 256, 256, 0, s->stream>>>(m.P, s->grad, m.M1, m.M2, kParams, lr, 0.9f, 0.999f,
-                                                             1e-8f, c1, c2);
-        if ((rc = pack(s, m)) != GELIO_OK) return rc;
-      }
-      if (ep == epochs - 1) {
-        SUR_TRY(cudaMemcpyAsync(sl.data(), s->step_loss, sizeof(float) * steps, cudaMemcpyDeviceToHost, s->stream));
-        SUR_TRY(cudaStreamSynchronize(s->stream));
-        loss = 0.0;
-        for (int st = 0; st < steps; ++st) loss += sl[st];
+  std::vector<float> sl((size_t)G * steps);
+  for (int m0 = 0; m0 < E; m0 += G) {
+    const int g = std::min(G, E - m0);
+    if ((rc = train_group(s, m0, g, epochs, steps, total, nrow, sl.data())) != GELIO_OK) return rc;
+    for (int k = 0; k < g; ++k) {
+      double loss = 0.0;
+      if (epochs > 0) {
+        for (int st = 0; st < steps; ++st) loss += sl[(size_t)k * steps + st];
         loss /= (double)std::min<size_t>(nrow, (size_t)steps * R);
       }
+      if (last_loss) last_loss[m0 + k] = (float)loss;
+      s->mem[m0 + k].trained = true;
     }
-    int rc = check_error(s);
-    if (rc != GELIO_OK) return rc;
-    if (last_loss) last_loss[e] = (float)loss;
-    m.trained = true;
   }
   return GELIO_OK;
 }
@@ -781,8 +921,16 @@ int32_t gelio_surrogate_gradient(gelio_surrogate *s, int32_t member, const float
                              cudaSuccess ||
                          cudaMemcpyAsync(d_t, t, (size_t)n * 4, cudaMemcpyHostToDevice, s->stream) != cudaSuccess))
     rc = GELIO_ERR_CUDA;
-  if (rc == GELIO_OK) rc = stage_rows(s, d_x, d_t, n);
-  if (rc == GELIO_OK) rc = forward_backward(s, s->mem[member], n, d_loss);
+  if (rc == GELIO_OK) rc = ensure_train(s, 1);
+  if (rc == GELIO_OK) {
+    k_gather<<<(s->rows + 127) / 128, 128, 0, s->stream>>>(d_x, d_t, s->ident, n, 0, s->rows, s->tb.X0, s->tb.y,
+                                                           s->tb.yhat);
+    UpdateArgs u{};
+    u.P[0] = s->mem[member].P;
+    u.grad = s->grad;
+    u.loss = d_loss;
+    rc = train_step(s, member, 1, n, u);
+  }
   float l = 0.f;
   if (rc == GELIO_OK &&
       (cudaMemcpyAsync(grad, s->grad, (size_t)kParams * 4, cudaMemcpyDeviceToHost, s->stream) != cudaSuccess ||

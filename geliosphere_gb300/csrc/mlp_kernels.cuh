@@ -1,17 +1,10 @@
-// Kernels of the spectrum surrogate: a 7 -> 256 -> 256 -> 256 -> 256 -> 1
-// MLP with SiLU, BF16 weights and activations, FP32 accumulation.
+// Inference kernels of the spectrum surrogate and what training shares with
+// them: a 7 -> 256 -> 256 -> 256 -> 256 -> 1 MLP with SiLU, BF16 weights and
+// activations, FP32 accumulation.
 //
-// Every layer product is one tcgen05 GEMM of the form C[M x N] = A[M x K] *
-// B[N x K]^T with both operands K-major in HBM (row-major, K contiguous):
-//   forward   Z_l   = X_{l-1} W_l^T          A = X_{l-1} [rows x in], B = W_l   [256 x in]
-//   input grad dX   = dH_l W_l               A = dH_l    [rows x 256], B = W_l^T [in x 256]
-//   weight grad dW_l = dH_l^T X_{l-1}        A = dH_l^T  [256 x rows], B = X_{l-1}^T [in x rows]
-// so every layer writes its activations / gradients twice, row-major and
-// transposed, from the GEMM epilogue that produces them.  The epilogues are
-// fused: bias + SiLU (+ the 256 -> 1 head on the last hidden layer) going
-// forward, SiLU' of the stored pre-activation going back; weight gradients
-// are split over the batch (split-K) into FP32 partials reduced in a fixed
-// order, so a gradient is deterministic.
+// Every layer product is one tcgen05 GEMM, X_l = SiLU(X_{l-1} W_l^T + b_l), of
+// the form C[M x N] = A[M x K] * B[N x K]^T with both operands K-major in HBM
+// (row-major, K contiguous).  Training is in mlp_train.cuh.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -46,26 +39,16 @@ constexpr int kOffW5 = kOffB4 + kWidth;                     // [256]
 constexpr int kOffB5 = kOffW5 + kWidth;                     // [1]
 constexpr int kParams = kOffB5 + 1;                         // 199,681
 
-enum Mode { FWD = 0, FWD_LAST = 1, INFER = 2, INFER_LAST = 3, DX = 4, DW = 5 };
+enum Mode { INFER = 0, INFER_LAST = 1 };
 
 struct GemmArgs {
-  int M;                  // GEMM rows: batch rows (FWD*, INFER*, DX) or 256 output features (DW)
-  int N;                  // GEMM columns: 256, or 64 for the first layer's DW
-  int K;                  // reduction length: layer fan-in, or batch rows (DW)
-  int k_per_split;        // DW: batch rows per split (multiple of 64); else K
-  int splits;             // DW: number of splits; else 1
-  int ldt;                // row count of the transposed outputs (batch rows)
-  const float *bias;      // FWD*, INFER*: [256]
-  const float *w5;        // *_LAST: head weights [256]
-  const float *b5;        // *_LAST: head bias [1]
-  __nv_bfloat16 *z_out;   // FWD*: pre-activations [M][256]
-  __nv_bfloat16 *x_out;   // FWD, INFER: activations [M][256]
-  __nv_bfloat16 *xt_out;  // FWD*: activations transposed [256][ldt]
-  float *y_out;           // *_LAST: head outputs [M], zeroed before the launch
-  const __nv_bfloat16 *z_prev;   // DX: pre-activations of the layer below [M][256]
-  __nv_bfloat16 *dh_out;  // DX: [M][256]
-  __nv_bfloat16 *dht_out; // DX: [256][ldt]
-  float *partial;         // DW: [splits][N][256]
+  int M;                  // query rows
+  int K;                  // layer fan-in (64 or 256)
+  const float *bias;      // [256]
+  const float *w5;        // INFER_LAST: head weights [256]
+  const float *b5;        // INFER_LAST: head bias [1]
+  __nv_bfloat16 *x_out;   // INFER: activations [M][256]
+  float *y_out;           // INFER_LAST: head outputs [M], zeroed before the launch
   unsigned *error;        // set nonzero when a wait times out
   unsigned long long timeout_ns;
 };
@@ -103,8 +86,8 @@ __device__ __forceinline__ float silu_grad_f(float z) {
 // staging writes on distinct banks.
 constexpr int kStagePitch = 80;
 
-__device__ __forceinline__ void store_rows(const uint4 (&v)[4], __nv_bfloat16 *dst, int row0, int M, int n0,
-                                           unsigned char *stage, int lane) {
+__device__ __forceinline__ void store_rows(const uint4 (&v)[4], __nv_bfloat16 *dst, size_t row0, int n0,
+                                           unsigned char *stage, int lane, size_t M = ~(size_t)0) {
   uint4 *mine = reinterpret_cast<uint4 *>(stage + lane * kStagePitch);
 #pragma unroll
   for (int q = 0; q < 4; ++q) mine[q] = v[q];
@@ -113,77 +96,29 @@ __device__ __forceinline__ void store_rows(const uint4 (&v)[4], __nv_bfloat16 *d
   for (int i = 0; i < 4; ++i) {
     const int r = i * 8 + (lane >> 2), piece = lane & 3;
     const uint4 val = *reinterpret_cast<const uint4 *>(stage + r * kStagePitch + piece * 16);
-    if (row0 + r < M) *reinterpret_cast<uint4 *>(dst + (size_t)(row0 + r) * kWidth + n0 + piece * 8) = val;
+    if (row0 + r < M) *reinterpret_cast<uint4 *>(dst + (row0 + r) * kWidth + n0 + piece * 8) = val;
   }
   __syncwarp();
 }
 
 // Columns [32 c_begin, 32 c_end) of one accumulator row (row = row0 + lane);
-// returns this thread's part of the 256 -> 1 head's dot product (*_LAST
-// modes).  Warp-wide: every lane of the warp calls it.
+// returns this thread's part of the 256 -> 1 head's dot product (INFER_LAST).
+// Warp-wide: every lane of the warp calls it.  sbias: the halved biases.
 template <int MODE>
-__device__ __forceinline__ float gemm_epilogue(const GemmArgs &a, int row, uint32_t trow, int split, int c_begin,
-                                               int c_end, unsigned char *stage, int lane, const float *sbias,
-                                               const float *sw5) {
-  const bool valid = row < a.M;
-  const int row0 = row - lane;
+__device__ __forceinline__ float gemm_epilogue(const GemmArgs &a, int row, uint32_t trow, int c_begin, int c_end,
+                                               unsigned char *stage, int lane, const float *sbias, const float *sw5) {
   float ysum = 0.0f;
   for (int c = c_begin; c < c_end; ++c) {
     float v[32];
     tc::tmem_ld32(trow + (uint32_t)(c * 32), v);     // warp-wide: every lane executes it
     const int n0 = c * 32;
-    if constexpr (MODE == DW) {
-      float *p = a.partial + ((size_t)split * a.N + n0) * kWidth + row;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) p[(size_t)j * kWidth] = v[j];
-      continue;
-    }
     __align__(16) __nv_bfloat16 out[32];
-    if constexpr (MODE == DX) {
-      __align__(16) __nv_bfloat16 zp[32];
-      if (valid) {
-        const uint4 *src = reinterpret_cast<const uint4 *>(a.z_prev + (size_t)row * kWidth + n0);
+    silu_infer32(v, sbias + n0, out);
+    if constexpr (MODE == INFER_LAST) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) reinterpret_cast<uint4 *>(zp)[q] = src[q];
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) reinterpret_cast<uint4 *>(zp)[q] = make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int j = 0; j < 32; ++j) out[j] = __float2bfloat16_rn(v[j] * silu_grad_f(__bfloat162float(zp[j])));
-      store_rows(reinterpret_cast<const uint4(&)[4]>(out), a.dh_out, row0, a.M, n0, stage, lane);
-      if (valid) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) a.dht_out[(size_t)(n0 + j) * a.ldt + row] = out[j];
-      }
-    } else if constexpr (MODE == INFER || MODE == INFER_LAST) {
-      // sbias holds the halved biases in the inference modes
-      silu_infer32(v, sbias + n0, out);
-      if constexpr (MODE == INFER_LAST) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) ysum += __bfloat162float(out[j]) * sw5[n0 + j];
-      } else {
-        store_rows(reinterpret_cast<const uint4(&)[4]>(out), a.x_out, row0, a.M, n0, stage, lane);
-      }
+      for (int j = 0; j < 32; ++j) ysum += __bfloat162float(out[j]) * sw5[n0 + j];
     } else {
-      // training forward
-      __align__(16) __nv_bfloat16 zb[32];
-#pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const float z = v[j] + sbias[n0 + j];
-        zb[j] = __float2bfloat16_rn(z);
-        out[j] = __float2bfloat16_rn(silu_f(z));
-        if (MODE == FWD_LAST) ysum += __bfloat162float(out[j]) * sw5[n0 + j];
-      }
-      if constexpr (MODE == FWD || MODE == FWD_LAST) {
-        store_rows(reinterpret_cast<const uint4(&)[4]>(zb), a.z_out, row0, a.M, n0, stage, lane);
-        if (valid) {
-#pragma unroll
-          for (int j = 0; j < 32; ++j) a.xt_out[(size_t)(n0 + j) * a.ldt + row] = out[j];
-        }
-      }
-      if constexpr (MODE == FWD)
-        store_rows(reinterpret_cast<const uint4(&)[4]>(out), a.x_out, row0, a.M, n0, stage, lane);
+      store_rows(reinterpret_cast<const uint4(&)[4]>(out), a.x_out, (size_t)(row - lane), n0, stage, lane, (size_t)a.M);
     }
   }
   return ysum;
@@ -193,8 +128,7 @@ __device__ __forceinline__ float gemm_epilogue(const GemmArgs &a, int row, uint3
 // round-robin:
 //   warp 0  (one lane)  TMA producer: the weight operand once (resident in
 //           shared memory for the whole launch), then the row tiles of A
-//           through a 4-stage ring; for weight gradients (DW) both operands
-//           stream through the ring;
+//           through a 4-stage ring;
 //   warp 1  (one lane)  MMA issuer: tcgen05.mma into one of two TMEM
 //           accumulators (2 x 256 columns), tcgen05.commit frees a ring
 //           stage and hands a finished accumulator to the epilogue;
@@ -203,8 +137,8 @@ __device__ __forceinline__ float gemm_epilogue(const GemmArgs &a, int row, uint3
 //           taking half of the columns (two warps per scheduler hide the
 //           epilogue's latency), fused epilogue, then hand the accumulator
 //           back; it overlaps the MMAs of the next tile.
-// Shared memory: region 1 (128 KiB) holds the resident weights (or the B
-// stages of DW), region 2 (64 KiB) the A stages.
+// Shared memory: region 1 (128 KiB) holds the resident weights, region 2
+// (64 KiB) the A stages.
 constexpr int kEpiWarps = 8;
 constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 constexpr uint32_t kRegion1 = 4 * kStageB;         // 128 KiB
@@ -213,7 +147,6 @@ constexpr uint32_t kRegion2 = kStages * kStageA;   // 64 KiB
 template <int MODE>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     k_mlp_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs a) {
-  constexpr bool kResidentB = (MODE != DW);
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(16) unsigned char s_stage[kEpiWarps][32 * kStagePitch];   // epilogue store staging
   __shared__ float s_bias[kWidth], s_w5[kWidth];     // epilogue operands, read by every row
@@ -229,8 +162,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   uint32_t *tslot = reinterpret_cast<uint32_t *>(acce + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t bytesB = (uint32_t)a.N * kChunk * 2;
-  const uint32_t idesc = tc::idesc_bf16_f32(kTileM, a.N);
+  const uint32_t idesc = tc::idesc_bf16_f32(kTileM, kWidth);
+  const int nk = a.K / kChunk;
 
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -246,11 +179,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     tc::tma_prefetch(&tmA);
     tc::tma_prefetch(&tmB);
   }
-  if (MODE != DW && MODE != DX) {
-    for (int i = tid; i < kWidth; i += blockDim.x) {
-      s_bias[i] = (MODE == INFER || MODE == INFER_LAST) ? 0.5f * a.bias[i] : a.bias[i];
-      if (MODE == FWD_LAST || MODE == INFER_LAST) s_w5[i] = a.w5[i];
-    }
+  for (int i = tid; i < kWidth; i += blockDim.x) {
+    s_bias[i] = 0.5f * a.bias[i];
+    if (MODE == INFER_LAST) s_w5[i] = a.w5[i];
   }
   if (warp == 1) {
     tc::tmem_alloc(tslot, 2 * kTmemCols);
@@ -261,31 +192,23 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   tc::tc_fence_after();
   const uint32_t tmem = *tslot;
   const unsigned long long deadline = tc::now_ns() + a.timeout_ns;
-  const int m_tiles = (a.M + kTileM - 1) / kTileM;
-  const int tiles = m_tiles * a.splits;
+  const int tiles = (a.M + kTileM - 1) / kTileM;
 
   if (warp == 0) {
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      if (kResidentB) {
-        const int nkb = a.K / kChunk;
-        tc::mbar_expect_tx(bfull, (uint32_t)nkb * bytesB);
-        for (int c = 0; c < nkb; ++c) tc::tma_load_2d(r1 + c * kStageB, &tmB, c * kChunk, 0, bfull);
-      }
+      tc::mbar_expect_tx(bfull, (uint32_t)nk * kStageB);
+      for (int c = 0; c < nk; ++c) tc::tma_load_2d(r1 + c * kStageB, &tmB, c * kChunk, 0, bfull);
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        const int tm = t % m_tiles, split = t / m_tiles;
-        const int k0 = split * a.k_per_split;
-        const int nk = (min(a.k_per_split, a.K - k0) + kChunk - 1) / kChunk;
         for (int kc = 0; kc < nk; ++kc) {
           const uint32_t st = it % kStages;
           if (it >= (uint32_t)kStages && !tc::mbar_wait(&empty[st], ((it / kStages) - 1) & 1, deadline)) {
             ok = false;
             break;
           }
-          tc::mbar_expect_tx(&full[st], kStageA + (kResidentB ? 0u : bytesB));
-          tc::tma_load_2d(r2 + st * kStageA, &tmA, k0 + kc * kChunk, tm * kTileM, &full[st]);
-          if (!kResidentB) tc::tma_load_2d(r1 + st * kStageB, &tmB, k0 + kc * kChunk, 0, &full[st]);
+          tc::mbar_expect_tx(&full[st], kStageA);
+          tc::tma_load_2d(r2 + st * kStageA, &tmA, kc * kChunk, t * kTileM, &full[st]);
           ++it;
         }
       }
@@ -295,18 +218,14 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const unsigned long long d2 = tc::now_ns() + 1000000000ull;
         for (uint32_t j = (it > (uint32_t)kStages ? it - kStages : 0u); j < it; ++j)
           tc::mbar_wait(&full[j % kStages], (j / kStages) & 1, d2);
-        if (kResidentB) tc::mbar_wait(bfull, 0, d2);
+        tc::mbar_wait(bfull, 0, d2);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       uint32_t it = 0, local = 0;
-      bool ok = !kResidentB || tc::mbar_wait(bfull, 0, deadline);
+      bool ok = tc::mbar_wait(bfull, 0, deadline);
       for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        const int split = t / m_tiles;
-        const int k0 = split * a.k_per_split;
-        const int nk = (min(a.k_per_split, a.K - k0) + kChunk - 1) / kChunk;
-        if (nk <= 0) continue;
         const uint32_t buf = local & 1u;
         if (local >= 2 && !tc::mbar_wait(&acce[buf], ((local >> 1) - 1) & 1, deadline)) {
           ok = false;
@@ -322,7 +241,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           }
           tc::tc_fence_after();
           const uint32_t aa = tc::smem_u32(r2 + st * kStageA);
-          const uint32_t bb = tc::smem_u32(r1 + (kResidentB ? (uint32_t)kc : st) * kStageB);
+          const uint32_t bb = tc::smem_u32(r1 + kc * kStageB);
 #pragma unroll
           for (int k = 0; k < kChunk / 16; ++k)
             tc::mma_bf16(d, tc::sdesc_sw128(aa + k * 32), tc::sdesc_sw128(bb + k * 32), idesc,
@@ -344,13 +263,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   } else {
     const int q = warp & 3;                       // TMEM lane quarter of this warp
     const int h = (warp - 2) / 4;                 // column half of this warp
-    const int per = (a.N / 32) / 2;
+    constexpr int per = (kWidth / 32) / 2;
     uint32_t local = 0;
     for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-      const int tm = t % m_tiles, split = t / m_tiles;
-      const int k0 = split * a.k_per_split;
-      const int nk = (min(a.k_per_split, a.K - k0) + kChunk - 1) / kChunk;
-      if (nk <= 0) continue;
       const uint32_t buf = local & 1u;
       const bool got = tc::mbar_wait(&accf[buf], (local >> 1) & 1, deadline);
       if (!__all_sync(0xffffffffu, got)) {
@@ -358,13 +273,13 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         break;
       }
       tc::tc_fence_after();
-      const int row = tm * kTileM + q * 32 + lane;
-      const float ys = gemm_epilogue<MODE>(a, row, tmem + ((uint32_t)(q * 32) << 16) + buf * kTmemCols, split,
-                                           h * per, (h + 1) * per, s_stage[warp - 2], lane, s_bias, s_w5);
+      const int row = t * kTileM + q * 32 + lane;
+      const float ys = gemm_epilogue<MODE>(a, row, tmem + ((uint32_t)(q * 32) << 16) + buf * kTmemCols, h * per,
+                                           (h + 1) * per, s_stage[warp - 2], lane, s_bias, s_w5);
       tc::tc_fence_before();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&acce[buf]);
-      if constexpr (MODE == FWD_LAST || MODE == INFER_LAST) {
+      if constexpr (MODE == INFER_LAST) {
         // y_out is zeroed before the launch; the two halves' sums meet by
         // atomic addition, (0 + x) + y == (0 + y) + x, so the order does not
         // change the result
@@ -658,109 +573,15 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 // CUDA-core kernels around the GEMMs
 // ----------------------------------------------------------------------------
 
-// Batch rows order[offset .. offset + rows) of the training set (past
-// n_order: padding rows of zeros).  Writes X0 [rows][64] (features in
-// columns 0..6; the padding columns stay zero from allocation), X0^T
-// [64][rows] (rows 0..6; skipped when x0t is null, for inference) and the
-// targets.
-__global__ void k_gather(const float *__restrict__ feats, const float *__restrict__ targ,
-                         const int *__restrict__ order, long long n_order, long long offset, int rows,
-                         __nv_bfloat16 *__restrict__ x0, __nv_bfloat16 *__restrict__ x0t, float *__restrict__ y) {
+// Query rows x [n][7] into the BF16 first-layer operand x0 [rows][64]
+// (features in columns 0..6; the padding columns stay zero from allocation);
+// rows past n are zero.
+__global__ void k_query_rows(const float *__restrict__ x, int n, int rows, __nv_bfloat16 *__restrict__ x0) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= rows) return;
-  const long long k = offset + m;
-  const int src = (k < n_order) ? order[k] : -1;
 #pragma unroll
-  for (int f = 0; f < kFeatures; ++f) {
-    const __nv_bfloat16 v = __float2bfloat16_rn(src >= 0 ? feats[(size_t)src * kFeatures + f] : 0.0f);
-    x0[(size_t)m * kInPad + f] = v;
-    if (x0t) x0t[(size_t)f * rows + m] = v;
-  }
-  if (y) y[m] = (src >= 0 && targ) ? targ[src] : 0.0f;
-}
-
-// Loss and the head's backward pass: dy = 2 (yhat - y) / n for the first n
-// rows (0 for padding), dH4 = dy * w5 * SiLU'(Z4) in both layouts, and one
-// squared-error partial per block.
-__global__ void k_head_backward(const float *__restrict__ yhat, const float *__restrict__ y, int n_valid, int rows,
-                                const float *__restrict__ w5, const __nv_bfloat16 *__restrict__ z4,
-                                __nv_bfloat16 *__restrict__ dh4, __nv_bfloat16 *__restrict__ dh4t,
-                                float *__restrict__ dy, float *__restrict__ loss_part) {
-  __shared__ float red[kThreads];
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  float se = 0.0f;
-  if (m < rows) {
-    const float e = (m < n_valid) ? (yhat[m] - y[m]) : 0.0f;
-    se = e * e;
-    const float d = 2.0f * e / (float)n_valid;
-    dy[m] = d;
-    for (int n = 0; n < kWidth; ++n) {
-      const float g = d * __ldg(w5 + n) * silu_grad_f(__bfloat162float(z4[(size_t)m * kWidth + n]));
-      const __nv_bfloat16 b = __float2bfloat16_rn(g);
-      dh4[(size_t)m * kWidth + n] = b;
-      dh4t[(size_t)n * rows + m] = b;
-    }
-  }
-  red[threadIdx.x] = se;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) loss_part[blockIdx.x] = red[0];
-}
-
-// out[r] = sum_c src[r][c] * (w ? w[c] : 1), one block per row, fixed order.
-__global__ void k_rowsum_bf16(const __nv_bfloat16 *__restrict__ src, int cols, const float *__restrict__ w,
-                              float *__restrict__ out) {
-  __shared__ float red[256];
-  const __nv_bfloat16 *row = src + (size_t)blockIdx.x * cols;
-  float s = 0.0f;
-  for (int c = threadIdx.x; c < cols; c += blockDim.x) s += __bfloat162float(row[c]) * (w ? w[c] : 1.0f);
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-    if (threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[blockIdx.x] = red[0];
-}
-
-__global__ void k_sum_f32(const float *__restrict__ src, int n, float *__restrict__ out) {
-  __shared__ float red[256];
-  float s = 0.0f;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) s += src[i];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int k = blockDim.x / 2; k > 0; k >>= 1) {
-    if (threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *out = red[0];
-}
-
-// dW[o][i] (i < fan_in) = sum over splits of partial[s][i][o].
-__global__ void k_reduce_dw(const float *__restrict__ partial, int splits, int n_cols, int fan_in,
-                            float *__restrict__ dw) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= kWidth * fan_in) return;
-  const int o = idx / fan_in, i = idx % fan_in;
-  float s = 0.0f;
-  for (int k = 0; k < splits; ++k) s += partial[((size_t)k * n_cols + i) * kWidth + o];
-  dw[idx] = s;
-}
-
-// Adam (bias-corrected) on the FP32 master parameters.
-__global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m1,
-                       float *__restrict__ m2, int n, float lr, float b1, float b2, float eps, float c1, float c2) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float a = b1 * m1[i] + (1.0f - b1) * gi;
-  const float b = b2 * m2[i] + (1.0f - b2) * gi * gi;
-  m1[i] = a;
-  m2[i] = b;
-  p[i] -= lr * (a / c1) / (sqrtf(b / c2) + eps);
+  for (int f = 0; f < kFeatures; ++f)
+    x0[(size_t)m * kInPad + f] = __float2bfloat16_rn(m < n ? x[(size_t)m * kFeatures + f] : 0.0f);
 }
 
 // BF16 operand copies of the master weights: W1 padded to [256][64], W2..W4

@@ -75,6 +75,15 @@ __device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *tm, in
       : "memory");
 }
 
+// 3D tile load; c2 is the outermost coordinate (a member of the ensemble).
+__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *tm, int c0, int c1, int c2, uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+          smem_u32(dst)),
+      "l"(reinterpret_cast<uint64_t>(tm)), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
+      : "memory");
+}
+
 // ----------------------------------------------------------------- tcgen05
 // Allocation and release are warp-wide (.sync.aligned).
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols) {
@@ -97,12 +106,23 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
+// Both operands MN-major instead (transpose bits 15 and 16).
+constexpr uint32_t kIdescMnMajorAB = (1u << 15) | (1u << 16);
+
 // Shared-memory matrix descriptor, K-major, 128-byte swizzle: start address
 // >> 4 in [0,14), leading byte offset (unused by this layout, 16 B) in
 // [16,30), stride byte offset 1024 B (8-row atom) in [32,46), descriptor
 // version 1 at bit 46, layout type 2 (SWIZZLE_128B) in [61,64).
 __device__ __forceinline__ uint64_t sdesc_sw128(uint32_t saddr) {
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
+         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+
+// The same for an MN-major operand: boxes of 64 MN elements (128 B) x K rows
+// as TMA writes them, 8 K rows at a 1 KiB stride (stride byte offset), the next
+// 64 MN elements `mn_stride` bytes further (leading byte offset).
+__device__ __forceinline__ uint64_t sdesc_sw128_mn(uint32_t saddr, uint32_t mn_stride) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(mn_stride >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
