@@ -213,55 +213,162 @@ __global__ void k_reduce(const double *__restrict__ part, int n_slices, long lon
   out[i] = s + c;
 }
 
-// Evaluate log.dat rows (gelio_evaluate): one thread per row into slices.
-__global__ void k_evaluate(const double *__restrict__ rows, long long n_rows, int n_cols,
-                           int model, int n_slices, double *part) {
+// Evaluate log.dat rows (gelio_evaluate), one thread per row, into slices.
+// Bound by the FP64 pipe (two FMA lanes an SM): 500,000 2D rows took 635 us on
+// the device at ~700 FP64 operations a row; now ~210 operations, the pipe 77%
+// busy on the fullest SM (evaluate call 852 -> 362 us).  One record count a
+// warp: every row would add to the same addresses.
+__device__ __forceinline__ void count_records(double *slice) {
+  const unsigned rows_here = __activemask();
+  if ((threadIdx.x & 31) == __ffs(rows_here) - 1) atomicAdd(&slice[kOffNRecords], (double)__popc(rows_here));
+}
+
+// 2D rows: what depends on the injection energy alone (its rounding, the Weber
+// flux, the bins; a third of the work) is formed once per distinct energy of
+// the block's rows.  Simulations inject on a grid (30 to some hundred
+// energies), so one or two warps of the block do it; rows of all-distinct
+// energies cost what they cost alone and a table insertion.  The block's rows
+// are then ordered by energy and each energy's weights summed in shared memory:
+// added to the slices row by row, 4.5 M global FP64 atomics took as long as the
+// arithmetic.
+constexpr int kEvalBlock = 256;
+constexpr int kEvalSlots = 2 * kEvalBlock;
+__global__ void __launch_bounds__(kEvalBlock) k_evaluate_2d(const double *__restrict__ rows, long long n_rows, int n_cols,
+                                                            int n_slices, double *part) {
+  __shared__ unsigned long long s_key[kEvalSlots];
+  __shared__ double s_weber[kEvalBlock], s_p2[kEvalBlock];      // by distinct energy
+  __shared__ unsigned s_bins[kEvalBlock];
+  __shared__ unsigned short s_index[kEvalSlots], s_slot[kEvalBlock];
+  __shared__ double s_w[3][kEvalBlock];                         // weights of the rows, by energy
+  __shared__ int s_rows[kEvalBlock], s_first[kEvalBlock + 1], s_warp[kEvalBlock / 32];
+  __shared__ int s_count;
+  constexpr unsigned long long kEmpty = ~0ull;
+  for (int j = threadIdx.x; j < kEvalSlots; j += kEvalBlock) s_key[j] = kEmpty;
+  s_rows[threadIdx.x] = 0;
+  if (threadIdx.x == 0) s_count = 0;
+  __syncthreads();
+  const long long i = (long long)blockIdx.x * kEvalBlock + threadIdx.x;
+  const bool valid = i < n_rows;
+  const double *row = rows + (size_t)i * n_cols;
+  int slot = 0;
+  double te = 1.0;
+  if (valid) {
+    te = row[1];
+    unsigned long long key = (unsigned long long)__double_as_longlong(row[0]);
+    if (key == kEmpty) key = 0x7ff8000000000000ull;          // one NaN for another
+    const unsigned h = (unsigned)(key >> 32) * 0x9E3779B1u + (unsigned)key * 0x85EBCA77u;
+    slot = (int)((h >> 16) ^ h) & (kEvalSlots - 1);
+    for (;;) {                                               // the table is twice the block: a free slot is there
+      const unsigned long long old = atomicCAS(&s_key[slot], kEmpty, key);
+      if (old == kEmpty) {
+        const int u = atomicAdd(&s_count, 1);
+        s_index[slot] = (unsigned short)u;
+        s_slot[u] = (unsigned short)slot;
+      }
+      if (old == kEmpty || old == key) break;
+      slot = (slot + 1) & (kEvalSlots - 1);
+    }
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < s_count) {
+    const double ti = round6(__longlong_as_double((long long)s_key[s_slot[threadIdx.x]]));
+    const double p2 = ti * (ti + kTwoT0);
+    s_p2[threadIdx.x] = p2;
+    s_weber[threadIdx.x] = lis_weber(log(ti)) * p2;
+    s_bins[threadIdx.x] = (unsigned)bin_sp(ti, c_tables) | (unsigned)bin_uly(ti, c_tables) << 8 |
+                          (unsigned)bin_ams(ti, c_tables) << 16;
+  }
+  __syncthreads();
+  const int u = valid ? s_index[slot] : 0;
+  const int rank = valid ? atomicAdd(&s_rows[u], 1) : 0;
+  __syncthreads();
+  {                                                            // s_first: exclusive sums of s_rows
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int v = s_rows[threadIdx.x];
+    int inc = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int x = __shfl_up_sync(kFull, inc, d);
+      if (lane >= d) inc += x;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    __syncthreads();
+    int before = 0;
+    for (int w = 0; w < warp; ++w) before += s_warp[w];
+    s_first[threadIdx.x] = before + inc - v;
+    if (threadIdx.x == kEvalBlock - 1) s_first[kEvalBlock] = before + inc;
+  }
+  __syncthreads();
+  if (valid && s_bins[u] != 0u) {
+    te = round6(te);
+    const double inv = 1.0 / (te * (te + kTwoT0)), ratio = s_p2[u] * inv;
+    const int pos = s_first[u] + rank;
+    s_w[0][pos] = s_weber[u] * inv;
+    s_w[1][pos] = lis_usoskin(te, log(te)) * ratio;
+    s_w[2][pos] = lis_burger(te) * ratio;
+  }
+  __syncthreads();
+  double *slice = part + (size_t)(blockIdx.x % n_slices) * kSpecDoubles;
+  for (int j = threadIdx.x; j < 3 * s_count; j += kEvalBlock) {
+    const int e = j / 3, f = j - 3 * e;
+    const unsigned bins = s_bins[e];
+    const int b_sp = bins & 0xff, b_uly = (bins >> 8) & 0xff, b_ams = bins >> 16;
+    if (!(b_sp || (f == 2 && bins != 0u))) continue;
+    double w = 0.0, w2 = 0.0;
+    for (int k = s_first[e]; k < s_first[e + 1]; ++k) {
+      const double x = s_w[f][k];
+      w += x;
+      w2 = fma(x, x, w2);
+    }
+    const double cnt = (double)s_rows[e];
+    if (b_sp) {
+      static_assert(kOffSpJgr - kOffSpWeber == kOffSpBurger - kOffSpJgr &&
+                    kOffSpJgr2 - kOffSpWeber2 == kOffSpBurger2 - kOffSpJgr2, "the three weights' sections are evenly spaced");
+      atomicAdd(&slice[kOffSpWeber + f * (kOffSpJgr - kOffSpWeber) + b_sp], w);
+      atomicAdd(&slice[kOffSpWeber2 + f * (kOffSpJgr2 - kOffSpWeber2) + b_sp], w2);
+      if (f == 0) atomicAdd(&slice[kOffSpN + b_sp], cnt);
+    }
+    if (f == 2 && b_uly) {
+      atomicAdd(&slice[kOffUlyW + b_uly], w);
+      atomicAdd(&slice[kOffUlyW2 + b_uly], w2);
+      atomicAdd(&slice[kOffUlyN + b_uly], cnt);
+    }
+    if (f == 2 && b_ams) {
+      atomicAdd(&slice[kOffAmsW + b_ams], w);
+      atomicAdd(&slice[kOffAmsW2 + b_ams], w2);
+      atomicAdd(&slice[kOffAmsN + b_ams], cnt);
+    }
+  }
+  if (threadIdx.x == 0) {
+    const long long left = n_rows - (long long)blockIdx.x * kEvalBlock;
+    atomicAdd(&slice[kOffNRecords], (double)(left < kEvalBlock ? left : kEvalBlock));
+  }
+}
+
+__global__ void __launch_bounds__(256) k_evaluate_1d(const double *__restrict__ rows, long long n_rows, int n_cols,
+                                                     int model, int n_slices, double *part) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n_rows) return;
   const double *row = rows + (size_t)i * n_cols;
   double *slice = part + (size_t)(blockIdx.x % n_slices) * kSpecDoubles;
   Contribution C;
   const double one = 1.0;
-  if (model >= kModelSolarProp) {
-    eval_2d(round6(row[0]), round6(row[1]), c_tables, C);
-    const double w[3] = {C.w[0], C.w[1], C.w[2]};
-    if (C.b_sp) {
-      atomicAdd(&slice[kOffSpWeber + C.b_sp], w[0]);
-      atomicAdd(&slice[kOffSpJgr + C.b_sp], w[1]);
-      atomicAdd(&slice[kOffSpBurger + C.b_sp], w[2]);
-      atomicAdd(&slice[kOffSpWeber2 + C.b_sp], w[0] * w[0]);
-      atomicAdd(&slice[kOffSpJgr2 + C.b_sp], w[1] * w[1]);
-      atomicAdd(&slice[kOffSpBurger2 + C.b_sp], w[2] * w[2]);
-      atomicAdd(&slice[kOffSpN + C.b_sp], one);
-    }
-    if (C.b_uly) {
-      atomicAdd(&slice[kOffUlyW + C.b_uly], w[2]);
-      atomicAdd(&slice[kOffUlyW2 + C.b_uly], w[2] * w[2]);
-      atomicAdd(&slice[kOffUlyN + C.b_uly], one);
-    }
-    if (C.b_ams) {
-      atomicAdd(&slice[kOffAmsW + C.b_ams], w[2]);
-      atomicAdd(&slice[kOffAmsW2 + C.b_ams], w[2] * w[2]);
-      atomicAdd(&slice[kOffAmsN + C.b_ams], one);
-    }
+  if (model == kModelBp) {
+    eval_bp(round6(row[1]), round6(row[0]), c_tables, C);
   } else {
-    if (model == kModelBp) {
-      eval_bp(round6(row[1]), round6(row[0]), c_tables, C);
-    } else {
-      double T1;
-      eval_fp(round6(row[0]), round6(row[1]), round6(row[2]), round6(row[4]), c_tables, C, T1);
-    }
-    const double w = C.w[0];
-    if (C.b_log >= 0) {
-      atomicAdd(&slice[kOffLogW + C.b_log], w);
-      atomicAdd(&slice[kOffLogW2 + C.b_log], w * w);
-      atomicAdd(&slice[kOffLogN + C.b_log], one);
-    }
-    if (C.b_e2) { atomicAdd(&slice[kOffE2W + C.b_e2 - 1], w); atomicAdd(&slice[kOffE2W2 + C.b_e2 - 1], w * w); atomicAdd(&slice[kOffE2N + C.b_e2 - 1], one); }
-    if (C.b_e3) { atomicAdd(&slice[kOffE3W + C.b_e3 - 1], w); atomicAdd(&slice[kOffE3W2 + C.b_e3 - 1], w * w); atomicAdd(&slice[kOffE3N + C.b_e3 - 1], one); }
-    if (C.b_e4) { atomicAdd(&slice[kOffE4W + C.b_e4 - 1], w); atomicAdd(&slice[kOffE4W2 + C.b_e4 - 1], w * w); atomicAdd(&slice[kOffE4N + C.b_e4 - 1], one); }
+    double T1;
+    eval_fp(round6(row[0]), round6(row[1]), round6(row[2]), round6(row[4]), c_tables, C, T1);
   }
-  atomicAdd(&slice[kOffNRecords], one);
+  const double w = C.w[0];
+  if (C.b_log >= 0) {
+    atomicAdd(&slice[kOffLogW + C.b_log], w);
+    atomicAdd(&slice[kOffLogW2 + C.b_log], w * w);
+    atomicAdd(&slice[kOffLogN + C.b_log], one);
+  }
+  if (C.b_e2) { atomicAdd(&slice[kOffE2W + C.b_e2 - 1], w); atomicAdd(&slice[kOffE2W2 + C.b_e2 - 1], w * w); atomicAdd(&slice[kOffE2N + C.b_e2 - 1], one); }
+  if (C.b_e3) { atomicAdd(&slice[kOffE3W + C.b_e3 - 1], w); atomicAdd(&slice[kOffE3W2 + C.b_e3 - 1], w * w); atomicAdd(&slice[kOffE3N + C.b_e3 - 1], one); }
+  if (C.b_e4) { atomicAdd(&slice[kOffE4W + C.b_e4 - 1], w); atomicAdd(&slice[kOffE4W2 + C.b_e4 - 1], w * w); atomicAdd(&slice[kOffE4N + C.b_e4 - 1], one); }
+  count_records(slice);
 }
 
 // Throughput probes for the roofline denominators.
@@ -360,6 +467,8 @@ struct gelio_ctx {
   int max_smem_optin = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr;
+  cudaStream_t copy_stream = nullptr, eval_stream = nullptr;   // gelio_evaluate: rows on their way up, every other piece
+  cudaEvent_t ev_copy = nullptr;
   std::mutex mu;
   // device buffers
   int cap_sims = 0;
@@ -460,6 +569,9 @@ static void release(gelio_ctx *c) {
   if (c->ev_k0) cudaEventDestroy(c->ev_k0);
   if (c->ev_k1) cudaEventDestroy(c->ev_k1);
   if (c->stream) cudaStreamDestroy(c->stream);
+  if (c->ev_copy) cudaEventDestroy(c->ev_copy);
+  if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
+  if (c->eval_stream) cudaStreamDestroy(c->eval_stream);
 }
 
 // Per-simulation buffers for n simulations: all five new buffers are
@@ -614,6 +726,9 @@ int32_t gelio_create(gelio_ctx **out, int32_t device) {
     c->sm_count = prop.multiProcessorCount;
     c->max_smem_optin = (int)prop.sharedMemPerBlockOptin;
     if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess) { rc = map_cuda(e); break; }
+    if ((e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking)) != cudaSuccess) { rc = map_cuda(e); break; }
+    if ((e = cudaStreamCreateWithFlags(&c->eval_stream, cudaStreamNonBlocking)) != cudaSuccess) { rc = map_cuda(e); break; }
+    if ((e = cudaEventCreateWithFlags(&c->ev_copy, cudaEventDisableTiming)) != cudaSuccess) { rc = map_cuda(e); break; }
     if ((e = cudaEventCreate(&c->ev_k0)) != cudaSuccess) { rc = map_cuda(e); break; }
     if ((e = cudaEventCreate(&c->ev_k1)) != cudaSuccess) { rc = map_cuda(e); break; }
     if ((e = dev_malloc(&c->d_ctl, sizeof(Control))) != cudaSuccess) { rc = map_cuda(e); break; }
@@ -942,20 +1057,60 @@ int32_t gelio_evaluate(gelio_ctx *c, int32_t model, const double *rows, int64_t 
   GELIO_TRY(cudaSetDevice(c->device));
   memset(out, 0, sizeof(*out));
   if (n_rows == 0) return GELIO_OK;
-  const int n_slices = 16;
+  // few rows add straight into the result (a reduction and the clearing of 1 MB
+  // of slices cost more than their contention does)
+  const int n_slices = n_rows <= 32768 ? 1 : 16;
   GELIO_TRY(grow(c->d_part, c->part_bytes, (size_t)n_slices * kSpecDoubles * 8));
   GELIO_TRY(grow(c->d_out, c->out_bytes, sizeof(gelio_spectra)));
   cudaStream_t st = c->stream;
   const size_t bytes = (size_t)n_rows * n_cols * sizeof(double);
   GELIO_TRY(grow(c->d_rows, c->rows_bytes, bytes));
-  GELIO_TRY(cudaMemcpyAsync(c->d_rows, rows, bytes, cudaMemcpyHostToDevice, st));
-  GELIO_TRY(cudaMemsetAsync(c->d_part, 0, (size_t)n_slices * kSpecDoubles * 8, st));
-  const unsigned grid = (unsigned)((n_rows + 255) / 256);
+  double *part = n_slices > 1 ? c->d_part : c->d_out;
+  GELIO_TRY(cudaMemsetAsync(part, 0, (size_t)n_slices * kSpecDoubles * 8, st));
   (void)cudaGetLastError();
-  k_evaluate<<<grid, 256, 0, st>>>(c->d_rows, n_rows, n_cols, model, n_slices, c->d_part);
-  GELIO_TRY(cudaGetLastError());
-  k_reduce<<<(kSpecDoubles + 255) / 256, 256, 0, st>>>(c->d_part, n_slices, kSpecDoubles, c->d_out);
-  GELIO_TRY(cudaGetLastError());
+  // The rows go up in pieces on a stream of their own, each evaluated while
+  // the next is copied (24 MB of 500,000 2D rows take 150 us to copy), the
+  // pieces' kernels on two streams in turn, so that one's last blocks run
+  // beside the next's first.  Pieces of at least kPieceRows: a kernel lasts
+  // 12 us however few its rows, the latency of its FP64 chain.
+  constexpr int64_t kPieceRows = 65536;
+  const int64_t pieces = n_rows < 2 * kPieceRows ? 1 : (n_rows / kPieceRows > 8 ? 8 : n_rows / kPieceRows);
+  const int64_t piece = (n_rows + pieces - 1) / pieces;
+  cudaError_t e = cudaSuccess;
+  if (pieces > 1) {
+    e = cudaEventRecord(c->ev_copy, st);                  // the slices are cleared
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(c->eval_stream, c->ev_copy, 0);
+  }
+  int64_t p = 0;
+  for (int64_t r0 = 0; r0 < n_rows && e == cudaSuccess; r0 += piece, ++p) {
+    const int64_t nr = n_rows - r0 < piece ? n_rows - r0 : piece;
+    double *d = c->d_rows + r0 * n_cols;
+    const cudaStream_t up = pieces > 1 ? c->copy_stream : st, run = (p & 1) ? c->eval_stream : st;
+    e = cudaMemcpyAsync(d, rows + r0 * n_cols, (size_t)nr * n_cols * sizeof(double), cudaMemcpyHostToDevice, up);
+    if (e == cudaSuccess && pieces > 1) e = cudaEventRecord(c->ev_copy, up);
+    if (e == cudaSuccess && pieces > 1) e = cudaStreamWaitEvent(run, c->ev_copy, 0);
+    if (e == cudaSuccess) {
+      if (model >= kModelSolarProp)
+        k_evaluate_2d<<<(unsigned)((nr + kEvalBlock - 1) / kEvalBlock), kEvalBlock, 0, run>>>(d, nr, n_cols, n_slices, part);
+      else
+        k_evaluate_1d<<<(unsigned)((nr + 255) / 256), 256, 0, run>>>(d, nr, n_cols, model, n_slices, part);
+      e = cudaGetLastError();
+    }
+  }
+  if (e == cudaSuccess && pieces > 1) {
+    e = cudaEventRecord(c->ev_copy, c->eval_stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, c->ev_copy, 0);
+  }
+  if (e != cudaSuccess) {           // no copy from the caller's rows outlives the call
+    cudaStreamSynchronize(c->copy_stream);
+    cudaStreamSynchronize(c->eval_stream);
+    cudaStreamSynchronize(st);
+    return map_cuda(e);
+  }
+  if (n_slices > 1) {
+    k_reduce<<<(kSpecDoubles + 255) / 256, 256, 0, st>>>(c->d_part, n_slices, kSpecDoubles, c->d_out);
+    GELIO_TRY(cudaGetLastError());
+  }
   GELIO_TRY(cudaMemcpyAsync(out, c->d_out, sizeof(gelio_spectra), cudaMemcpyDeviceToHost, st));
   GELIO_TRY(cudaStreamSynchronize(st));
   return GELIO_OK;

@@ -87,15 +87,24 @@ struct BinTables {
 __device__ __forceinline__ double pow10_hi(int k) { return kPow10Hi[k + 40]; }
 __device__ __forceinline__ double pow10_lo(int k) { return kPow10Lo[k + 40]; }
 
+//
+// GB300 has two FP64 FMA lanes an SM (a warp instruction holds the SM's pipe
+// for 16 cycles), so this and the weights below are written for few FP64
+// operations: the decimal exponent comes from the binary one by integer
+// arithmetic, and a value that is a six-digit decimal already (a log.dat's
+// are) is recognised from its scaled remainder, without a division.
 static __device__ __noinline__ double round6(double xin) {
   if (!(xin != 0.0) || !(fabs(xin) < 1e300)) return xin;   // 0, NaN, huge: unchanged
   const double sign = (xin < 0.0) ? -1.0 : 1.0;
   const double x = fabs(xin);
-  int e = (int)floor(log10(x));
-  if (e < -34 || e > 34) return xin;
+  // 2^b <= x < 2^(b+1): floor(b log10(2)) is the decimal exponent or one off
+  const int b = ((__double2hiint(x) >> 20) & 0x7ff) - 1023;
+  int e = (b * 1262611) >> 22;
+  if (e < -35 || e > 34) return xin;
   // exact decimal exponent: 10^e <= x < 10^(e+1)
   if (x < pow10_hi(e)) --e;
   else if (x >= pow10_hi(e + 1)) ++e;
+  if (e < -34 || e > 34) return xin;
   const int k = 5 - e;                        // x * 10^k in [1e5, 1e6)
   // m = rint(x * 10^k) with the product carried in double-double
   const double ph = pow10_hi(k), pl = pow10_lo(k);
@@ -103,6 +112,8 @@ static __device__ __noinline__ double round6(double xin) {
   const double perr = fma(x, ph, -p) + x * pl;
   double m = rint(p);
   const double frac = (p - m) + perr;          // exact remainder relative to m
+  // 10^k exact: |x 10^k - m| below half a unit of x means x = m 10^-k, rounded
+  if (k >= 0 && k <= 22 && fabs(frac) < 0.49 * ph * __hiloint2double((b - 52 + 1023) << 20, 0)) return xin;
   if (frac > 0.5) m += 1.0;
   else if (frac < -0.5) m -= 1.0;
   else if (frac == 0.5 || frac == -0.5) {
@@ -112,11 +123,9 @@ static __device__ __noinline__ double round6(double xin) {
   }
   // value m * 10^-k, correctly rounded
   if (k <= 0) return sign * (m * pow10_hi(-k));   // 10^-k exact for -k <= 22
-  const double dh = pow10_hi(k), dl = pow10_lo(k);
-  double y = m / dh;
-  // one correction with the double-double divisor: y = m / (dh + dl)
-  const double res = fma(-y, dh, m) - y * dl;
-  y = y + res / dh;
+  double y = m / ph;
+  // beyond 10^22 one correction with the double-double divisor: y = m / (ph + pl)
+  if (k > 22) y = y + (fma(-y, ph, m) - y * pl) / ph;
   return sign * y;
 }
 
@@ -128,28 +137,21 @@ __device__ __forceinline__ double p_si(double T) {
   return __ddiv_rn(__dmul_rn(rig, kQ), kC);
 }
 
-// LIS fluxes of TwoDimensionBpResults.cpp:50-76.
-__device__ __forceinline__ double lis_weber(double T) {
-  const double l = log(T);
-  const double tem5 = 21.1 * exp(-2.8 * l);
-  const double tem6 = 1.0 + (5.85 * exp(-1.22 * l)) + (1.18 * exp(-2.54 * l));
-  return tem5 / tem6;
+// LIS fluxes of TwoDimensionBpResults.cpp:50-76 at T, with l = log(T): the same
+// products of powers with their logarithms and exponentials shared.
+__device__ __forceinline__ double lis_weber(double l) {
+  return 21.1 * exp(-2.8 * l) / (1.0 + (5.85 * exp(-1.22 * l)) + (1.18 * exp(-2.54 * l)));
 }
-__device__ __forceinline__ double lis_usoskin(double T) {
+// 2.7e3 T^1.12 ((T + 0.67) / 1.67)^-3.93 / beta^2, beta^2 = T (T + 2 Tr) / (T + Tr)^2
+__device__ __forceinline__ double lis_usoskin(double T, double l) {
   const double tt = T + kTr;
-  const double t2 = tt + kTr;
-  const double beta = sqrt(T * t2) / tt;
-  double tem = (T + 0.67) / 1.67;
-  tem = exp(-3.93 * log(tem));
-  double j = 2.7e3 * exp(1.12 * log(T)) * tem;
-  return j / (beta * beta);
+  constexpr double kLog167 = 0.51282362642866375;      // log(1.67)
+  return 2.7e3 * exp(fma(1.12, l, -3.93 * (log(T + 0.67) - kLog167))) * (tt * tt) / (T * (tt + kTr));
 }
+// 1.9e4 P^-2.78 / (1 + 0.4866 P^-2.51), P^2 = T (T + 2 0.938)
 __device__ __forceinline__ double lis_burger(double T) {
-  double tem = sqrt((T * T) + (2.0 * T * 0.938));
-  double j = 1.9 * 1.0e4 * exp(-2.78 * log(tem));
-  tem = sqrt((T * T) + (2.0 * T * 0.938));
-  tem = 0.4866 * exp(-2.51 * log(tem));
-  return j / (1 + tem);
+  const double l2 = log(T * (T + 2.0 * 0.938));
+  return 1.9e4 * exp(-1.39 * l2) / (1.0 + 0.4866 * exp(-1.255 * l2));
 }
 
 // Yamada et al. 1998 weight of OneDimensionBpResults.cpp:58-60 (no 1e45
@@ -158,6 +160,10 @@ __device__ __forceinline__ double yamada(double p) {
   const double w = (kM0 * kM0 * kC * kC * kC * kC) + (p * p * kC * kC);
   return exp(-1.85 * log(w)) / p;
 }
+
+// (p(T1) / p(T2))^2 of two kinetic energies: p^2 c^2 = T (T + 2 T0).
+constexpr double kTwoT0 = 2.0 * kT0w / (kQ * 1e9);      // GeV
+__device__ __forceinline__ double p2_ratio(double T1, double T2) { return T1 * (T1 + kTwoT0) / (T2 * (T2 + kTwoT0)); }
 
 // Kinetic energy [GeV] from an SI momentum, as OneDimensionFpResults.cpp:51-54.
 __device__ __forceinline__ double fp_tkin_from_p(double p1AU) {
@@ -177,10 +183,11 @@ __device__ __forceinline__ int grid_log_bin(double T, double lo_log, double inv_
 }
 
 // SolarProp window bin (1..29) of TwoDimensionBpResults.cpp:80-89, 0 if none.
+// The windows lie around 0.01 1.5^(ii-1), 50% apart and 1% wide: an FP32
+// logarithm finds the one in question.
 __device__ __forceinline__ int bin_sp(double Ti, const BinTables &t) {
-  for (int ii = 1; ii < 30; ii++)
-    if ((Ti > t.sp[ii] * 0.99) && (Ti < t.sp[ii] * 1.01)) return ii;
-  return 0;
+  const int ii = (int)rintf(__log2f(fmaxf((float)Ti, 1e-6f) * 100.0f) * 1.7095113f) + 1;   // 1 / log2(1.5)
+  return (ii >= 1 && ii < 30 && (Ti > t.sp[ii] * 0.99) && (Ti < t.sp[ii] * 1.01)) ? ii : 0;
 }
 __device__ __forceinline__ int bin_uly(double Ti, const BinTables &t) {
   for (int ii = 1; ii < 3; ii++)
@@ -235,16 +242,16 @@ struct Contribution {
 // 2D record: injection energy Ti (1 AU) and exit energy Te (100 AU), both
 // already passed through round6 (the log.dat columns Tkininj and Tkin).
 __device__ inline void eval_2d(double Ti, double Te, const BinTables &t, Contribution &o) {
-  const double p = p_si(Te);
-  const double p1AU = p_si(Ti);
-  const double ratio = (p1AU * p1AU) / (p * p);
+  const double ratio = p2_ratio(Ti, Te);
+  const double l = log(Te);
+  const double usoskin = lis_usoskin(Te, l) * ratio, burger = lis_burger(Te) * ratio;
   // TwoDimensionBpResults.cpp:50-54: the Weber LIS is evaluated at Tkininj.
-  o.w[0] = lis_weber(Ti) / (p * p) * p1AU * p1AU;
-  o.w[1] = lis_usoskin(Te) / (p * p) * p1AU * p1AU;
-  o.w[2] = lis_burger(Te) / (p * p) * p1AU * p1AU;
-  o.gw[0] = lis_weber(Te) * ratio;
-  o.gw[1] = lis_usoskin(Te) * ratio;
-  o.gw[2] = lis_burger(Te) * ratio;
+  o.w[0] = lis_weber(log(Ti)) * ratio;
+  o.w[1] = usoskin;
+  o.w[2] = burger;
+  o.gw[0] = lis_weber(l) * ratio;
+  o.gw[1] = usoskin;
+  o.gw[2] = burger;
   o.b_sp = bin_sp(Ti, t);
   o.b_uly = bin_uly(Ti, t);
   o.b_ams = bin_ams(Ti, t);
@@ -258,10 +265,10 @@ __device__ inline void eval_bp(double Ti, double Te, const BinTables &t, Contrib
   const double p1AU = p_si(Ti);
   double w = yamada(p);
   w = w * p1AU * p1AU;
-  const double ratio = (p1AU * p1AU) / (p * p);
+  const double ratio = p2_ratio(Ti, Te);
   o.w[0] = w; o.w[1] = 0.0; o.w[2] = 0.0;
   o.gw[0] = w;
-  o.gw[1] = lis_weber(Te) * ratio;
+  o.gw[1] = lis_weber(log(Te)) * ratio;
   o.gw[2] = lis_burger(Te) * ratio;
   o.b_log = bin_bp_log(Ti, t);
   o.b_e2 = bin_e2(Ti);
