@@ -140,6 +140,7 @@ struct gelio_surrogate {
   // BF16 operand copies of every member's weights, [members][256][fan-in]
   bf16 *W1 = nullptr, *W[3] = {}, *WT[3] = {};
   CUtensorMap tW1, tW[3], tWT[3];
+  float *epi = nullptr;      // FP32 epilogue operands of inference, [members][5][256]
   TrainBuffers tb;
   float *grad = nullptr;     // gelio_surrogate_gradient's result
   float *step_loss = nullptr;
@@ -155,10 +156,11 @@ struct gelio_surrogate {
   std::vector<float> feats, targ;
   float *d_feats = nullptr, *d_targ = nullptr;
   size_t d_rows_cap = 0, d_rows_used = 0;
-  float *d_query = nullptr, *d_yq = nullptr;   // inference inputs / outputs
+  float *d_query = nullptr, *d_yq = nullptr;   // forward: inputs / outputs
   size_t query_cap = 0;
   // predict: simulations and their row offsets on the device, member outputs
-  // [E][stride], ensemble mean / std [2][rows], pinned staging of both ends
+  // [E][stride], ensemble mean / std [2][rows] and the error flag, pinned
+  // staging of both ends
   unsigned char *d_pup = nullptr;     // [n] gelio_sim_params, then [n + 1] row offsets
   size_t pup_cap = 0;
   float *d_py = nullptr;
@@ -166,13 +168,10 @@ struct gelio_surrogate {
   size_t prows_cap = 0;
   unsigned char *h_pstage = nullptr;
   size_t pstage_cap = 0;
-  // inference batches: larger than training batches, so every SM gets
-  // several tiles per launch and the resident weights are loaded once per tile
-  // group rather than once per tile
+  // first-layer operand of an inference batch; the padding columns stay zero
   int qrows = 0;
-  bf16 *Q0 = nullptr, *Q[2] = {};
-  float *qy = nullptr;
-  CUtensorMap mQ0, mQ[2];
+  bf16 *Q0 = nullptr;
+  CUtensorMap mQ0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;    // device time of the last inference
   double last_ms = 0.0, last_flop = 0.0;
   bool dirty = true;
@@ -194,16 +193,6 @@ int cuda_status_at(cudaError_t e, int line) {
     if (e_ != cudaSuccess) return cuda_status(e_); \
   } while (0)
 
-template <int MODE>
-int launch_gemm(gelio_surrogate *s, const CUtensorMap &A, const CUtensorMap &B, GemmArgs a) {
-  a.error = s->error;
-  a.timeout_ns = 2000000000ull;
-  const int tiles = (a.M + kTileM - 1) / kTileM;
-  const int grid = std::max(1, std::min(tiles, s->sm_count));
-  k_mlp_gemm<MODE><<<grid, kGemmThreads, kGemmSmem, s->stream>>>(A, B, a);
-  return cuda_status(cudaGetLastError());
-}
-
 int set_smem_attrs() {
   static int rc = -1;
   static std::once_flag once;
@@ -213,8 +202,6 @@ int set_smem_attrs() {
       if (e == cudaSuccess)
         e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
     };
-    set((const void *)k_mlp_gemm<INFER>);
-    set((const void *)k_mlp_gemm<INFER_LAST>);
     set((const void *)k_train_gemm<FWD>);
     set((const void *)k_train_gemm<FWD_LAST>);
     set((const void *)k_train_gemm<DX>);
@@ -243,7 +230,7 @@ void free_all(gelio_surrogate *s) {
   free_train(s->tb);
   f(s->grad); f(s->step_loss);
   f(s->ident); f(s->order); f(s->error); f(s->d_feats); f(s->d_targ); f(s->d_query); f(s->d_yq);
-  f(s->Q0); f(s->Q[0]); f(s->Q[1]); f(s->qy);
+  f(s->Q0); f(s->epi);
   f(s->d_pup); f(s->d_py); f(s->d_pstat);
   if (s->h_pstage) cudaFreeHost(s->h_pstage);
   if (s->h_order) cudaFreeHost(s->h_order);
@@ -255,7 +242,8 @@ void free_all(gelio_surrogate *s) {
 
 int pack(gelio_surrogate *s, Member &m) {
   const int n = kWidth * kWidth;
-  k_pack<<<(n + 255) / 256, 256, 0, s->stream>>>(m.P, m.W1, m.W[0], m.W[1], m.W[2], m.WT[0], m.WT[1], m.WT[2]);
+  k_pack<<<(n + 255) / 256, 256, 0, s->stream>>>(m.P, m.W1, m.W[0], m.W[1], m.W[2], m.WT[0], m.WT[1], m.WT[2],
+                                                 s->epi + (&m - s->mem.data()) * kEpiFloats);
   return cuda_status(cudaGetLastError());
 }
 
@@ -379,6 +367,8 @@ int train_step(gelio_surrogate *s, int m0, int G, int n_valid, UpdateArgs &u) {
     u.w = (li == 0) ? s->W1 : s->W[li - 1];
     u.wt = (li == 0) ? nullptr : s->WT[li - 1];
     u.w_ld = (li == 0) ? kInPad : kWidth;
+    u.epi = s->epi;
+    u.epi_layer = li;
     const int blocks = 8 * ((u.fan_in + 31) / 32) + 8 + (li == 3 ? 9 : 0);
     k_update<<<dim3(blocks, G), 256, 0, s->stream>>>(u);
     SUR_TRY(cudaGetLastError());
@@ -386,41 +376,80 @@ int train_step(gelio_surrogate *s, int m0, int G, int n_valid, UpdateArgs &u) {
   return GELIO_OK;
 }
 
-// Inference of member m on the first `M` rows of the inference batch
-// (M a multiple of 128); outputs in s->qy.
-int forward_infer_q(gelio_surrogate *s, Member &m, int M) {
-  int rc;
-  GemmArgs a{};
-  a.M = M;
-  a.K = kInPad; a.bias = m.P + kOffB1; a.x_out = s->Q[0];
-  if ((rc = launch_gemm<INFER>(s, s->mQ0, m.mW1, a)) != GELIO_OK) return rc;
-  a.K = kWidth; a.bias = m.P + kOffB2; a.x_out = s->Q[1];
-  if ((rc = launch_gemm<INFER>(s, s->mQ[0], m.mW[0], a)) != GELIO_OK) return rc;
-  a.bias = m.P + kOffB3; a.x_out = s->Q[0];
-  if ((rc = launch_gemm<INFER>(s, s->mQ[1], m.mW[1], a)) != GELIO_OK) return rc;
-  a.bias = m.P + kOffB4; a.x_out = nullptr; a.w5 = m.P + kOffW5; a.b5 = m.P + kOffB5; a.y_out = s->qy;
-  SUR_TRY(cudaMemsetAsync(s->qy, 0, (size_t)M * 4, s->stream));
-  return launch_gemm<INFER_LAST>(s, s->mQ[0], m.mW[2], a);
+// First-layer operand for an inference batch of `rows` rows (at most
+// kQueryBatch), whole pairs of tiles.
+constexpr size_t kQueryBatch = 262144;
+int ensure_query(gelio_surrogate *s, size_t rows) {
+  size_t cap = 1024;
+  while (cap < std::min(rows, kQueryBatch)) cap *= 2;
+  if ((size_t)s->qrows >= cap) return GELIO_OK;
+  bf16 *fresh = nullptr;
+  SUR_TRY(gelio::dev_malloc(&fresh, cap * kInPad * 2));
+  CUtensorMap map;
+  const cudaError_t e = cudaMemsetAsync(fresh, 0, cap * kInPad * 2, s->stream);
+  if (e != cudaSuccess || !make_map(&map, fresh, kInPad, cap, kTileM)) {
+    cudaFree(fresh);
+    return e != cudaSuccess ? cuda_status(e) : GELIO_ERR_CUDA;
+  }
+  if (s->Q0) cudaFree(s->Q0);
+  s->Q0 = fresh;
+  s->mQ0 = map;
+  s->qrows = (int)cap;
+  return GELIO_OK;
+}
+
+// Members [m0, m1) on the first c rows of the inference batch (s->Q0, zero
+// past c up to a whole tile) in one launch of the fused network kernel; member
+// m0 + e's outputs are added to y[e * stride + row].
+int infer_fused(gelio_surrogate *s, int m0, int m1, int c, float *y, long long stride) {
+  const int E = m1 - m0;
+  if (E > kFusedMaxMembers) return GELIO_ERR_UNSUPPORTED;
+  FusedMaps maps;
+  maps.q0 = s->mQ0;
+  FusedArgs a{};
+  for (int e = 0; e < E; ++e) {
+    maps.w[e][0] = s->mem[m0 + e].mW1;
+    for (int l = 0; l < 3; ++l) maps.w[e][l + 1] = s->mem[m0 + e].mW[l];
+    a.P[e] = s->mem[m0 + e].P;
+  }
+  a.M = c;
+  a.n_pairs = (c + 2 * kTileM - 1) / (2 * kTileM);
+  a.E = E;
+  a.stride = stride;
+  a.epi = s->epi + (size_t)m0 * kEpiFloats;
+  a.y = y;
+  a.error = s->error;
+  a.timeout_ns = 2000000000ull;
+  const int grid = std::max(1, std::min(E * a.n_pairs, s->sm_count));
+  k_mlp_infer_fused<<<grid, kFusedThreads, kFusedSmem, s->stream>>>(maps, a);
+  return cuda_status(cudaGetLastError());
+}
+
+// FLOP of the products over the rows actually multiplied (whole tiles of 128
+// rows; first layer K padded to 64).
+double gemm_flop(size_t padded, size_t members) {
+  return 2.0 * (double)padded * (double)members * ((double)kInPad * kWidth + 3.0 * kWidth * kWidth + (double)kWidth);
 }
 
 bool valid_member(gelio_surrogate *s, int m) { return s && m >= 0 && m < (int)s->mem.size(); }
 
-// Inference of members [m0, m1) on n rows x [n][7]: one upload, one gather
-// per batch of rows shared by the members, outputs y[(m - m0) * n + row].
-int infer_rows(gelio_surrogate *s, int m0, int m1, const float *x, size_t n, float *y) {
+// Inference of one member on n rows x [n][7].
+int infer_rows(gelio_surrogate *s, int m, const float *x, size_t n, float *y) {
   if (n == 0) return GELIO_OK;
-  const size_t E = (size_t)(m1 - m0);
+  int rc = ensure_query(s, n);
+  if (rc != GELIO_OK) return rc;
   if (n > s->query_cap) {
     if (s->d_query) cudaFree(s->d_query);
     if (s->d_yq) cudaFree(s->d_yq);
     s->d_query = s->d_yq = nullptr;
     s->query_cap = 0;
     SUR_TRY(gelio::dev_malloc(&s->d_query, n * kFeatures * 4));
-    SUR_TRY(gelio::dev_malloc(&s->d_yq, n * 16 * 4));
+    SUR_TRY(gelio::dev_malloc(&s->d_yq, n * 4));
     s->query_cap = n;
   }
   SUR_TRY(cudaMemcpyAsync(s->d_query, x, n * kFeatures * 4, cudaMemcpyHostToDevice, s->stream));
   SUR_TRY(cudaEventRecord(s->ev0, s->stream));
+  SUR_TRY(cudaMemsetAsync(s->d_yq, 0, n * 4, s->stream));
   size_t padded = 0;
   for (size_t off = 0; off < n; off += (size_t)s->qrows) {
     const int c = (int)std::min<size_t>((size_t)s->qrows, n - off);
@@ -428,22 +457,15 @@ int infer_rows(gelio_surrogate *s, int m0, int m1, const float *x, size_t n, flo
     padded += (size_t)M;
     k_query_rows<<<(M + 127) / 128, 128, 0, s->stream>>>(s->d_query + off * kFeatures, c, M, s->Q0);
     SUR_TRY(cudaGetLastError());
-    for (size_t e = 0; e < E; ++e) {
-      const int rc = forward_infer_q(s, s->mem[m0 + e], M);
-      if (rc != GELIO_OK) return rc;
-      SUR_TRY(cudaMemcpyAsync(s->d_yq + e * n + off, s->qy, (size_t)c * 4, cudaMemcpyDeviceToDevice, s->stream));
-    }
+    if ((rc = infer_fused(s, m, m + 1, c, s->d_yq + off, (long long)n)) != GELIO_OK) return rc;
   }
   SUR_TRY(cudaEventRecord(s->ev1, s->stream));
-  SUR_TRY(cudaMemcpyAsync(y, s->d_yq, E * n * 4, cudaMemcpyDeviceToHost, s->stream));
-  const int rc = check_error(s);
+  SUR_TRY(cudaMemcpyAsync(y, s->d_yq, n * 4, cudaMemcpyDeviceToHost, s->stream));
+  rc = check_error(s);
   float ms = 0.f;
   if (rc == GELIO_OK && cudaEventElapsedTime(&ms, s->ev0, s->ev1) == cudaSuccess) {
     s->last_ms = ms;
-    // FLOP of the GEMMs over the rows actually multiplied (each inference
-    // batch padded to a multiple of 128 rows; first layer K padded to 64)
-    s->last_flop = 2.0 * (double)padded * (double)E *
-                   ((double)kInPad * kWidth + 3.0 * kWidth * kWidth + (double)kWidth);
+    s->last_flop = gemm_flop(padded, 1);
   }
   return rc;
 }
@@ -612,14 +634,9 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
   };
   alloc((void **)&s->grad, (size_t)kParams * 4);
   alloc((void **)&s->ident, R * 4);
-  s->qrows = std::max(s->rows, 65536);
-  const size_t Rq = (size_t)s->qrows;
-  alloc((void **)&s->Q0, Rq * kInPad * 2);
-  alloc((void **)&s->Q[0], Rq * kWidth * 2);
-  alloc((void **)&s->Q[1], Rq * kWidth * 2);
-  alloc((void **)&s->qy, Rq * 4);
   alloc((void **)&s->error, 4);
   const size_t E = (size_t)o.members;
+  alloc((void **)&s->epi, E * kEpiFloats * 4);
   alloc((void **)&s->W1, E * kWidth * kInPad * 2);
   for (int i = 0; i < 3; ++i) {
     alloc((void **)&s->W[i], E * kWidth * kWidth * 2);
@@ -638,9 +655,7 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
     }
   }
   if (rc != GELIO_OK) return fail(rc);
-  bool ok = make_map(&s->mQ0, s->Q0, kInPad, Rq, kTileM) && make_map(&s->mQ[0], s->Q[0], kWidth, Rq, kTileM) &&
-            make_map(&s->mQ[1], s->Q[1], kWidth, Rq, kTileM);
-  ok = ok && make_map3(&s->tW1, s->W1, kInPad, kWidth, E, kWidth);
+  bool ok = make_map3(&s->tW1, s->W1, kInPad, kWidth, E, kWidth);
   for (int i = 0; i < 3; ++i)
     ok = ok && make_map3(&s->tW[i], s->W[i], kWidth, kWidth, E, kWidth) &&
          make_map3(&s->tWT[i], s->WT[i], kWidth, kWidth, E, kWidth);
@@ -787,67 +802,41 @@ int32_t gelio_surrogate_train(gelio_surrogate *s, int32_t epochs, float *last_lo
   return GELIO_OK;
 }
 
-// Every member on the first c rows of the inference batch (s->Q0, zero past
-// c up to a whole tile) in one launch of the fused network kernel; member e's
-// outputs go to y[e * stride + row].
-int infer_fused(gelio_surrogate *s, int c, float *y, long long stride) {
-  const int E = (int)s->mem.size();
-  if (E > kFusedMaxMembers) return GELIO_ERR_UNSUPPORTED;
-  FusedMaps maps;
-  maps.q0 = s->mQ0;
-  FusedArgs a{};
-  for (int e = 0; e < E; ++e) {
-    maps.w[e][0] = s->mem[e].mW1;
-    for (int l = 0; l < 3; ++l) maps.w[e][l + 1] = s->mem[e].mW[l];
-    a.P[e] = s->mem[e].P;
-  }
-  a.M = c;
-  a.n_pairs = (c + 2 * kTileM - 1) / (2 * kTileM);
-  a.E = E;
-  a.stride = stride;
-  a.y = y;
-  a.error = s->error;
-  a.timeout_ns = 2000000000ull;
-  const int items = E * a.n_pairs;
-  const int grid = std::max(1, std::min(items, s->sm_count));
-  k_mlp_infer_fused<<<grid, kFusedThreads, kFusedSmem, s->stream>>>(maps, a);
-  return cuda_status(cudaGetLastError());
-}
-
 // Ensemble inference of every LOG_GRID point of sims[0..n): the simulations
-// and their row offsets go up (one copy from pinned staging), the features
-// are built on the device per inference batch, every member's layers run on
-// the batch, k_ensemble forms mean and std, and the two come back in one copy.
+// and their row offsets go up (one copy from pinned staging), k_query builds the
+// inputs of a batch, every member's layers run on it in one launch and
+// k_ensemble forms mean and std.  Few rows come back through the staging, the
+// error flag with them; many straight into the caller's arrays (through the
+// staging the host's two copies of 3.2 MB took 200 us of an 870 us call).
 int infer_sims(gelio_surrogate *s, const gelio_sim_params *sims, int n, size_t rows, double *ln_ratio,
                double *ln_std) {
-  const size_t E = s->mem.size();
+  const int E = (int)s->mem.size();
   const size_t stride = (rows + kTileM - 1) / kTileM * kTileM;
-  // device layout: [n] gelio_sim_params, [n + 1] row offsets (both uploaded
-  // in one copy), then [n] QuerySim built on the device
-  const size_t up = (size_t)n * sizeof(gelio_sim_params) + (size_t)(n + 1) * sizeof(long long);
-  const size_t qoff = (up + 63) / 64 * 64;
-  const size_t down = 2 * rows * sizeof(double);
   // the simulations and their row offsets travel in one copy, so they share
   // one allocation (n * 96 bytes keeps the offsets 8-byte aligned)
-  const size_t dev_bytes = qoff + (size_t)n * sizeof(QuerySim);
-  if (dev_bytes > s->pup_cap) {
+  const size_t up = (size_t)n * sizeof(gelio_sim_params) + (size_t)(n + 1) * sizeof(long long);
+  constexpr size_t kStagedRows = 8192;
+  const bool staged = rows <= kStagedRows;
+  const size_t down = (staged ? 2 * rows * sizeof(double) : 0) + sizeof(double);   // ... and the error flag
+  int rc = ensure_query(s, rows);
+  if (rc != GELIO_OK) return rc;
+  if (up > s->pup_cap) {
     unsigned char *fresh = nullptr;
-    SUR_TRY(gelio::dev_malloc(&fresh, dev_bytes));
+    SUR_TRY(gelio::dev_malloc(&fresh, up));
     if (s->d_pup) cudaFree(s->d_pup);
     s->d_pup = fresh;
-    s->pup_cap = dev_bytes;
+    s->pup_cap = up;
   }
   const gelio_sim_params *d_psims = reinterpret_cast<const gelio_sim_params *>(s->d_pup);
   const long long *d_pfirst = reinterpret_cast<const long long *>(s->d_pup + (size_t)n * sizeof(gelio_sim_params));
-  QuerySim *d_pq = reinterpret_cast<QuerySim *>(s->d_pup + qoff);
   if (stride > s->prows_cap) {
     if (s->d_py) cudaFree(s->d_py);
     if (s->d_pstat) cudaFree(s->d_pstat);
     s->d_py = nullptr;
     s->d_pstat = nullptr;
     s->prows_cap = 0;
-    SUR_TRY(gelio::dev_malloc(&s->d_py, 16 * stride * sizeof(float)));
-    SUR_TRY(gelio::dev_malloc(&s->d_pstat, 2 * stride * sizeof(double)));
+    SUR_TRY(gelio::dev_malloc(&s->d_py, E * stride * sizeof(float)));
+    SUR_TRY(gelio::dev_malloc(&s->d_pstat, (2 * stride + 1) * sizeof(double)));
     s->prows_cap = stride;
   }
   if (std::max(up, down) > s->pstage_cap) {
@@ -863,36 +852,41 @@ int infer_sims(gelio_surrogate *s, const gelio_sim_params *sims, int n, size_t r
   for (int i = 0; i < n; ++i) first[i + 1] = first[i] + sims[i].inj_points;
   SUR_TRY(cudaEventRecord(s->ev0, s->stream));
   SUR_TRY(cudaMemcpyAsync(s->d_pup, s->h_pstage, up, cudaMemcpyHostToDevice, s->stream));
-  k_query_sims<<<(n + 127) / 128, 128, 0, s->stream>>>(d_psims, n, d_pq);
-  SUR_TRY(cudaGetLastError());
-  // the fused kernel adds the two column halves of each head output into y
-  SUR_TRY(cudaMemsetAsync(s->d_py, 0, E * stride * sizeof(float), s->stream));
   size_t padded = 0;
   for (size_t off = 0; off < rows; off += (size_t)s->qrows) {
     const int c = (int)std::min<size_t>((size_t)s->qrows, rows - off);
     const int M = (c + kTileM - 1) / kTileM * kTileM;
-    padded += (size_t)(c + 2 * kTileM - 1) / (2 * kTileM) * (2 * kTileM);   // rows the fused kernel multiplies
-    k_query_features<<<(M + 127) / 128, 128, 0, s->stream>>>(d_pq, d_pfirst, n, (long long)off, c, M, s->Q0);
+    padded += (size_t)M;
+    k_query<<<(M + kQueryBlock - 1) / kQueryBlock, kQueryBlock, 0, s->stream>>>(
+        d_psims, d_pfirst, n, (long long)off, c, M, E, (long long)stride, s->Q0, s->d_py);
     SUR_TRY(cudaGetLastError());
-    const int rc = infer_fused(s, c, s->d_py + off, (long long)stride);
-    if (rc != GELIO_OK) return rc;
+    if ((rc = infer_fused(s, 0, E, c, s->d_py + off, (long long)stride)) != GELIO_OK) return rc;
   }
-  k_ensemble<<<(unsigned)((rows + 255) / 256), 256, 0, s->stream>>>(s->d_py, (int)E, (long long)rows,
-                                                                    (long long)stride, s->d_pstat,
-                                                                    s->d_pstat + rows);
+  k_ensemble<<<(unsigned)((rows + 127) / 128), 128, 0, s->stream>>>(
+      s->d_py, E, (long long)rows, (long long)stride, s->d_pstat, s->d_pstat + rows, s->error,
+      reinterpret_cast<unsigned *>(s->d_pstat + 2 * rows));
   SUR_TRY(cudaGetLastError());
   SUR_TRY(cudaEventRecord(s->ev1, s->stream));
-  SUR_TRY(cudaMemcpyAsync(s->h_pstage, s->d_pstat, down, cudaMemcpyDeviceToHost, s->stream));
-  const int rc = check_error(s);
-  if (rc != GELIO_OK) return rc;
-  const double *st = reinterpret_cast<const double *>(s->h_pstage);
-  std::memcpy(ln_ratio, st, rows * sizeof(double));
-  if (ln_std) std::memcpy(ln_std, st + rows, rows * sizeof(double));
+  const size_t bytes = rows * sizeof(double);
+  if (staged) {
+    SUR_TRY(cudaMemcpyAsync(s->h_pstage, s->d_pstat, down, cudaMemcpyDeviceToHost, s->stream));
+  } else {
+    SUR_TRY(cudaMemcpyAsync(s->h_pstage, s->d_pstat + 2 * rows, down, cudaMemcpyDeviceToHost, s->stream));
+    SUR_TRY(cudaMemcpyAsync(ln_ratio, s->d_pstat, bytes, cudaMemcpyDeviceToHost, s->stream));
+    if (ln_std) SUR_TRY(cudaMemcpyAsync(ln_std, s->d_pstat + rows, bytes, cudaMemcpyDeviceToHost, s->stream));
+  }
+  SUR_TRY(cudaStreamSynchronize(s->stream));
+  unsigned error = 0;
+  std::memcpy(&error, s->h_pstage + down - sizeof(double), sizeof(error));
+  if (error) return check_error(s);
+  if (staged) {
+    std::memcpy(ln_ratio, s->h_pstage, bytes);
+    if (ln_std) std::memcpy(ln_std, s->h_pstage + bytes, bytes);
+  }
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, s->ev0, s->ev1) == cudaSuccess) {
     s->last_ms = ms;
-    s->last_flop = 2.0 * (double)padded * (double)E *
-                   ((double)kInPad * kWidth + 3.0 * kWidth * kWidth + (double)kWidth);
+    s->last_flop = gemm_flop(padded, (size_t)E);
   }
   return GELIO_OK;
 }
@@ -902,7 +896,7 @@ int32_t gelio_surrogate_forward(gelio_surrogate *s, int32_t member, const float 
   std::lock_guard<std::mutex> lock(s->mu);
   SUR_TRY(cudaSetDevice(s->device));
   (void)cudaGetLastError();   // a launch check below must see only this call's errors
-  return infer_rows(s, member, member + 1, x, (size_t)n, y);
+  return infer_rows(s, member, x, (size_t)n, y);
 }
 
 int32_t gelio_surrogate_gradient(gelio_surrogate *s, int32_t member, const float *x, const float *t, int32_t n,

@@ -1,9 +1,9 @@
-// Inference kernels of the spectrum surrogate and what training shares with
-// them: a 7 -> 256 -> 256 -> 256 -> 256 -> 1 MLP with SiLU, BF16 weights and
+// Inference kernel of the spectrum surrogate and what training shares with it:
+// a 7 -> 256 -> 256 -> 256 -> 256 -> 1 MLP with SiLU, BF16 weights and
 // activations, FP32 accumulation.
 //
-// Every layer product is one tcgen05 GEMM, X_l = SiLU(X_{l-1} W_l^T + b_l), of
-// the form C[M x N] = A[M x K] * B[N x K]^T with both operands K-major in HBM
+// Every layer product is a tcgen05 GEMM, X_l = SiLU(X_{l-1} W_l^T + b_l), of
+// the form C[M x N] = A[M x K] * B[N x K]^T with both operands K-major
 // (row-major, K contiguous).  Training is in mlp_train.cuh.
 #pragma once
 #include <cuda_bf16.h>
@@ -39,20 +39,6 @@ constexpr int kOffW5 = kOffB4 + kWidth;                     // [256]
 constexpr int kOffB5 = kOffW5 + kWidth;                     // [1]
 constexpr int kParams = kOffB5 + 1;                         // 199,681
 
-enum Mode { INFER = 0, INFER_LAST = 1 };
-
-struct GemmArgs {
-  int M;                  // query rows
-  int K;                  // layer fan-in (64 or 256)
-  const float *bias;      // [256]
-  const float *w5;        // INFER_LAST: head weights [256]
-  const float *b5;        // INFER_LAST: head bias [1]
-  __nv_bfloat16 *x_out;   // INFER: activations [M][256]
-  float *y_out;           // INFER_LAST: head outputs [M], zeroed before the launch
-  unsigned *error;        // set nonzero when a wait times out
-  unsigned long long timeout_ns;
-};
-
 __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + __expf(-z)); }
 
 // Inference SiLU of 32 accumulator columns v with pre-halved biases hb:
@@ -60,7 +46,7 @@ __device__ __forceinline__ float silu_f(float z) { return z / (1.0f + __expf(-z)
 // halving), one tanh.approx.f32 per element (2^-11 relative) instead of an
 // exponential and a reciprocal, the FP32 arithmetic in pairs (f32x2) and the
 // BF16 rounding two at a time.  Training keeps silu_f, whose derivative the
-// backward pass uses; both layer-by-layer and fused inference use this.
+// backward pass uses.
 __device__ __forceinline__ float tanh_approx(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -68,10 +54,15 @@ __device__ __forceinline__ float tanh_approx(float x) {
 }
 __device__ __forceinline__ void silu_infer32(const float (&v)[32], const float *hb, __nv_bfloat16 (&out)[32]) {
 #pragma unroll
-  for (int j = 0; j < 32; j += 2) {
-    const float2 h = __ffma2_rn(make_float2(v[j], v[j + 1]), make_float2(0.5f, 0.5f), make_float2(hb[j], hb[j + 1]));
-    const float2 t = make_float2(tanh_approx(h.x), tanh_approx(h.y));
-    *reinterpret_cast<__nv_bfloat162 *>(&out[j]) = __float22bfloat162_rn(__ffma2_rn(h, t, h));
+  for (int j = 0; j < 32; j += 4) {
+    const float4 b = __ldg(reinterpret_cast<const float4 *>(hb + j));
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const float2 h = __ffma2_rn(make_float2(v[j + 2 * i], v[j + 2 * i + 1]), make_float2(0.5f, 0.5f),
+                                  i == 0 ? make_float2(b.x, b.y) : make_float2(b.z, b.w));
+      const float2 t = make_float2(tanh_approx(h.x), tanh_approx(h.y));
+      *reinterpret_cast<__nv_bfloat162 *>(&out[j + 2 * i]) = __float22bfloat162_rn(__ffma2_rn(h, t, h));
+    }
   }
 }
 __device__ __forceinline__ float silu_grad_f(float z) {
@@ -87,7 +78,7 @@ __device__ __forceinline__ float silu_grad_f(float z) {
 constexpr int kStagePitch = 80;
 
 __device__ __forceinline__ void store_rows(const uint4 (&v)[4], __nv_bfloat16 *dst, size_t row0, int n0,
-                                           unsigned char *stage, int lane, size_t M = ~(size_t)0) {
+                                           unsigned char *stage, int lane) {
   uint4 *mine = reinterpret_cast<uint4 *>(stage + lane * kStagePitch);
 #pragma unroll
   for (int q = 0; q < 4; ++q) mine[q] = v[q];
@@ -96,233 +87,49 @@ __device__ __forceinline__ void store_rows(const uint4 (&v)[4], __nv_bfloat16 *d
   for (int i = 0; i < 4; ++i) {
     const int r = i * 8 + (lane >> 2), piece = lane & 3;
     const uint4 val = *reinterpret_cast<const uint4 *>(stage + r * kStagePitch + piece * 16);
-    if (row0 + r < M) *reinterpret_cast<uint4 *>(dst + (row0 + r) * kWidth + n0 + piece * 8) = val;
+    *reinterpret_cast<uint4 *>(dst + (row0 + r) * kWidth + n0 + piece * 8) = val;
   }
   __syncwarp();
 }
 
-// Columns [32 c_begin, 32 c_end) of one accumulator row (row = row0 + lane);
-// returns this thread's part of the 256 -> 1 head's dot product (INFER_LAST).
-// Warp-wide: every lane of the warp calls it.  sbias: the halved biases.
-template <int MODE>
-__device__ __forceinline__ float gemm_epilogue(const GemmArgs &a, int row, uint32_t trow, int c_begin, int c_end,
-                                               unsigned char *stage, int lane, const float *sbias, const float *sw5) {
-  float ysum = 0.0f;
-  for (int c = c_begin; c < c_end; ++c) {
-    float v[32];
-    tc::tmem_ld32(trow + (uint32_t)(c * 32), v);     // warp-wide: every lane executes it
-    const int n0 = c * 32;
-    __align__(16) __nv_bfloat16 out[32];
-    silu_infer32(v, sbias + n0, out);
-    if constexpr (MODE == INFER_LAST) {
-#pragma unroll
-      for (int j = 0; j < 32; ++j) ysum += __bfloat162float(out[j]) * sw5[n0 + j];
-    } else {
-      store_rows(reinterpret_cast<const uint4(&)[4]>(out), a.x_out, (size_t)(row - lane), n0, stage, lane, (size_t)a.M);
-    }
-  }
-  return ysum;
-}
-
-// One CTA per SM, warp-specialised, tiles of 128 GEMM rows handed out
-// round-robin:
-//   warp 0  (one lane)  TMA producer: the weight operand once (resident in
-//           shared memory for the whole launch), then the row tiles of A
-//           through a 4-stage ring;
-//   warp 1  (one lane)  MMA issuer: tcgen05.mma into one of two TMEM
-//           accumulators (2 x 256 columns), tcgen05.commit frees a ring
-//           stage and hands a finished accumulator to the epilogue;
-//   warps 2-9           epilogue: tcgen05.ld one row per thread (warp w reads
-//           TMEM lanes 32 (w % 4) .. +31), two warps per lane quarter each
-//           taking half of the columns (two warps per scheduler hide the
-//           epilogue's latency), fused epilogue, then hand the accumulator
-//           back; it overlaps the MMAs of the next tile.
-// Shared memory: region 1 (128 KiB) holds the resident weights, region 2
-// (64 KiB) the A stages.
+// Training GEMMs (mlp_train.cuh): shared memory regions and warps.
 constexpr int kEpiWarps = 8;
 constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 constexpr uint32_t kRegion1 = 4 * kStageB;         // 128 KiB
 constexpr uint32_t kRegion2 = kStages * kStageA;   // 64 KiB
 
-template <int MODE>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-    k_mlp_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmArgs a) {
-  extern __shared__ unsigned char smem_raw[];
-  __shared__ __align__(16) unsigned char s_stage[kEpiWarps][32 * kStagePitch];   // epilogue store staging
-  __shared__ float s_bias[kWidth], s_w5[kWidth];     // epilogue operands, read by every row
-  const uint32_t s0 = tc::smem_u32(smem_raw);
-  unsigned char *base = smem_raw + ((1024u - (s0 & 1023u)) & 1023u);
-  unsigned char *r1 = base;
-  unsigned char *r2 = base + kRegion1;
-  uint64_t *full = reinterpret_cast<uint64_t *>(r2 + kRegion2);
-  uint64_t *empty = full + kStages;
-  uint64_t *bfull = empty + kStages;
-  uint64_t *accf = bfull + 1;
-  uint64_t *acce = accf + 2;
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(acce + 2);
-
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t idesc = tc::idesc_bf16_f32(kTileM, kWidth);
-  const int nk = a.K / kChunk;
-
-  if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) {
-      tc::mbar_init(&full[s], 1);
-      tc::mbar_init(&empty[s], 1);
-    }
-    tc::mbar_init(bfull, 1);
-    for (int b = 0; b < 2; ++b) {
-      tc::mbar_init(&accf[b], 1);
-      tc::mbar_init(&acce[b], kEpiWarps);
-    }
-    tc::fence_mbar_init();
-    tc::tma_prefetch(&tmA);
-    tc::tma_prefetch(&tmB);
-  }
-  for (int i = tid; i < kWidth; i += blockDim.x) {
-    s_bias[i] = 0.5f * a.bias[i];
-    if (MODE == INFER_LAST) s_w5[i] = a.w5[i];
-  }
-  if (warp == 1) {
-    tc::tmem_alloc(tslot, 2 * kTmemCols);
-    tc::tmem_relinquish();
-  }
-  tc::tc_fence_before();
-  __syncthreads();
-  tc::tc_fence_after();
-  const uint32_t tmem = *tslot;
-  const unsigned long long deadline = tc::now_ns() + a.timeout_ns;
-  const int tiles = (a.M + kTileM - 1) / kTileM;
-
-  if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      tc::mbar_expect_tx(bfull, (uint32_t)nk * kStageB);
-      for (int c = 0; c < nk; ++c) tc::tma_load_2d(r1 + c * kStageB, &tmB, c * kChunk, 0, bfull);
-      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        for (int kc = 0; kc < nk; ++kc) {
-          const uint32_t st = it % kStages;
-          if (it >= (uint32_t)kStages && !tc::mbar_wait(&empty[st], ((it / kStages) - 1) & 1, deadline)) {
-            ok = false;
-            break;
-          }
-          tc::mbar_expect_tx(&full[st], kStageA);
-          tc::tma_load_2d(r2 + st * kStageA, &tmA, kc * kChunk, t * kTileM, &full[st]);
-          ++it;
-        }
-      }
-      if (!ok) {
-        atomicExch(a.error, 1u);
-        // copies in flight land before the shared memory is given back
-        const unsigned long long d2 = tc::now_ns() + 1000000000ull;
-        for (uint32_t j = (it > (uint32_t)kStages ? it - kStages : 0u); j < it; ++j)
-          tc::mbar_wait(&full[j % kStages], (j / kStages) & 1, d2);
-        tc::mbar_wait(bfull, 0, d2);
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      uint32_t it = 0, local = 0;
-      bool ok = tc::mbar_wait(bfull, 0, deadline);
-      for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
-        const uint32_t buf = local & 1u;
-        if (local >= 2 && !tc::mbar_wait(&acce[buf], ((local >> 1) - 1) & 1, deadline)) {
-          ok = false;
-          break;
-        }
-        tc::tc_fence_after();
-        const uint32_t d = tmem + buf * kTmemCols;
-        for (int kc = 0; kc < nk; ++kc) {
-          const uint32_t st = it % kStages;
-          if (!tc::mbar_wait(&full[st], (it / kStages) & 1, deadline)) {
-            ok = false;
-            break;
-          }
-          tc::tc_fence_after();
-          const uint32_t aa = tc::smem_u32(r2 + st * kStageA);
-          const uint32_t bb = tc::smem_u32(r1 + kc * kStageB);
-#pragma unroll
-          for (int k = 0; k < kChunk / 16; ++k)
-            tc::mma_bf16(d, tc::sdesc_sw128(aa + k * 32), tc::sdesc_sw128(bb + k * 32), idesc,
-                         (kc > 0 || k > 0) ? 1u : 0u);
-          tc::mma_commit(&empty[st]);
-          ++it;
-        }
-        if (!ok) break;
-        tc::mma_commit(&accf[buf]);
-        ++local;
-      }
-      if (!ok) {
-        atomicExch(a.error, 2u);
-        // products in flight finish before TMEM is given back
-        const unsigned long long d2 = tc::now_ns() + 1000000000ull;
-        if (it > 0) tc::mbar_wait(&empty[(it - 1) % kStages], ((it - 1) / kStages) & 1, d2);
-      }
-    }
-  } else {
-    const int q = warp & 3;                       // TMEM lane quarter of this warp
-    const int h = (warp - 2) / 4;                 // column half of this warp
-    constexpr int per = (kWidth / 32) / 2;
-    uint32_t local = 0;
-    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-      const uint32_t buf = local & 1u;
-      const bool got = tc::mbar_wait(&accf[buf], (local >> 1) & 1, deadline);
-      if (!__all_sync(0xffffffffu, got)) {
-        if (lane == 0) atomicExch(a.error, 3u);
-        break;
-      }
-      tc::tc_fence_after();
-      const int row = t * kTileM + q * 32 + lane;
-      const float ys = gemm_epilogue<MODE>(a, row, tmem + ((uint32_t)(q * 32) << 16) + buf * kTmemCols, h * per,
-                                           (h + 1) * per, s_stage[warp - 2], lane, s_bias, s_w5);
-      tc::tc_fence_before();
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive(&acce[buf]);
-      if constexpr (MODE == INFER_LAST) {
-        // y_out is zeroed before the launch; the two halves' sums meet by
-        // atomic addition, (0 + x) + y == (0 + y) + x, so the order does not
-        // change the result
-        if (row < a.M) atomicAdd(&a.y_out[row], h == 0 ? ys + __ldg(a.b5) : ys);
-      }
-      ++local;
-    }
-  }
-  __syncthreads();
-  if (warp == 1) {
-    tc::tc_fence_after();
-    tc::tmem_dealloc(tmem, 2 * kTmemCols);
-  }
-}
-
 // ----------------------------------------------------------------------------
-// Whole-network inference, all ensemble members in one persistent launch.
+// Whole-network inference, several ensemble members in one persistent launch.
 //
-// Work item = (member e, 256 query rows): two 128-row tiles run the four
-// hidden layers in lockstep and share every weight chunk.  The activations
-// never leave the SM: each layer's epilogue writes bias + SiLU as BF16
-// straight into shared memory in the K-major 128-byte-swizzle layout that
-// the next layer's tcgen05.mma reads (the layout TMA would write), and the
-// last layer's epilogue forms the 256 -> 1 head.  Only the first layer's
-// input (the query features, TMA) and the weights (32 KiB K-chunks of
-// [256 N][64 K], TMA from L2, a 2-stage ring) are loaded.
-//   warp 0 (one lane)  TMA: the item's two input tiles, then 13 weight chunks
+// Work item = (member, 256 query rows): two 128-row tiles X, Y (the last item of
+// a member may have X alone) run the four hidden layers and share every weight
+// chunk.  The activations never leave the SM: each layer's epilogue writes
+// bias + SiLU as BF16 straight into shared memory in the K-major
+// 128-byte-swizzle layout that the next layer's tcgen05.mma reads (the layout
+// TMA would write), and the last layer's epilogue forms the 256 -> 1 head.  Only
+// the first layer's input (the query features, TMA) and the weights (32 KiB
+// K-chunks of [256 N][64 K], TMA from L2, a ring of kFusedStages) are loaded.
+//   warp 0 (one lane)  TMA: the first item's input tiles, then 13 weight chunks
+//                      an item
 //   warp 1 (one lane)  MMA: per layer and K-chunk one N = 256 product per tile
-//                      into that tile's TMEM accumulator (2 x 256 columns),
-//                      the tiles staggered by two chunks so that one tile's
-//                      epilogue runs under the other tile's products
+//                      into that tile's TMEM accumulator (2 x 256 columns)
 //   warps 2-17         epilogue: warp w takes TMEM lane quarter w % 4 of
 //                      tile ((w - 2) / 4) % 2, columns 128 ((w - 2) / 8) ..
-//                      + 127 of its 32 rows (two warps per row quarter, so
-//                      each drains half the accumulator: the epilogue is
-//                      bound by the latency of its TMEM loads)
-// Every value equals the layer-by-layer INFER / INFER_LAST path bit for bit:
-// the same operands in the same K order, the same epilogue arithmetic and
-// the head summed as (sum of columns 0-127 + b5) + sum of columns 128-255.
-// Shared memory: A (2 x 64 KiB) + weight ring (2 x 32 KiB) + biases.
+//                      + 127 of its 32 rows; the tile's first warp also loads
+//                      its input for the next item as soon as the last layer's
+//                      products have read the tile's buffer
+//
+// What bounds it: shared memory.  A product reads 48 KiB of operands for 512
+// cycles of tensor core (96 of the 128 bytes a cycle), and the epilogues'
+// stores and the weights' arrival share the same port: a product takes ~930
+// cycles, an epilogue 3,300-5,500 (2,048 of them tanh on the special-function
+// unit), and X's run ahead of Y's only as far as the ring's three stages let
+// it.  The order of the products hardly matters (measured: 556-596 us of device
+// time for 200,000 rows and 5 members in five orders; two stages and one batch
+// per 65,536 rows: 625).  Per SM 0.40 of the tensor core's measured BF16 rate.
 // ----------------------------------------------------------------------------
 constexpr int kFusedMaxMembers = 16;
-constexpr int kFusedStages = 2;
+constexpr int kFusedStages = 3;
 constexpr int kFusedEpiWarps = 16;
 constexpr int kFusedThreads = 64 + 32 * kFusedEpiWarps;
 constexpr uint32_t kFusedA = kTileM * kWidth * 2;                 // 64 KiB: one tile's activations
@@ -333,13 +140,18 @@ struct FusedMaps {
   CUtensorMap w[kFusedMaxMembers][4];              // W1 [256][64], W2-W4 [256][256], box {64, 256}
 };
 
+// FP32 operands of the epilogues, by member: halved biases of the four layers
+// and the head weights.
+constexpr int kEpiFloats = 5 * kWidth;
+
 struct FusedArgs {
   int M;                        // query rows
   int n_pairs;                  // ceil(M / 256)
   int E;                        // members
   long long stride;             // y row stride per member
-  const float *P[kFusedMaxMembers];   // FP32 parameters of each member (biases, head)
-  float *y;                     // [E][stride] head outputs
+  const float *epi;             // [E][5][256]
+  const float *P[kFusedMaxMembers];   // FP32 parameters of each member (head bias)
+  float *y;                     // [E][stride] head outputs, zeroed before the launch
   unsigned *error;
   unsigned long long timeout_ns;
 };
@@ -347,38 +159,40 @@ struct FusedArgs {
 __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-__device__ __forceinline__ void named_sync(int id, int count) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
-}
+
+// Order of a layer's eight products, bit i = tile of the i-th (0 X, 1 Y), each
+// tile's K-chunks in order: X0 X1 Y0 X2 X3 Y1 Y2 Y3.
+constexpr uint32_t kFusedOrder = 0xE4u;
 
 __global__ void __launch_bounds__(kFusedThreads, 1)
     k_mlp_infer_fused(const __grid_constant__ FusedMaps maps, const FusedArgs a) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ float s_b[4][kWidth], s_w5[kWidth];
   const uint32_t s0 = tc::smem_u32(smem_raw);
   unsigned char *base = smem_raw + ((1024u - (s0 & 1023u)) & 1023u);
   unsigned char *ring = base + 2 * kFusedA;          // A of tile t: base + t * kFusedA
   uint64_t *full = reinterpret_cast<uint64_t *>(ring + kFusedStages * kStageB);
   uint64_t *empty = full + kFusedStages;
-  uint64_t *a_full = empty + kFusedStages;      // the item's input tiles landed
-  uint64_t *a_empty = a_full + 1;               // the item's last products read A
-  uint64_t *acc_full = a_empty + 1;             // [tile]: a layer's products are in TMEM
+  uint64_t *a_full = empty + kFusedStages;      // [tile]: the item's input landed
+  uint64_t *acc_full = a_full + 2;              // [tile]: a layer's products are in TMEM
   uint64_t *acc_empty = acc_full + 2;           // [tile]: a layer's epilogue read TMEM and wrote A
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(acc_empty + 2);
+  uint64_t *drain = acc_empty + 2;              // products finished, after a wait ran out
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(drain + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int items = a.E * a.n_pairs;
+  // tiles of item w: Y is there if any of its rows is
+  auto tiles_of = [&](int w) { return ((w % a.n_pairs) * 2 + 1) * kTileM < a.M ? 2 : 1; };
   if (tid == 0) {
     for (int st = 0; st < kFusedStages; ++st) {
       tc::mbar_init(&full[st], 1);
       tc::mbar_init(&empty[st], 1);
     }
-    tc::mbar_init(a_full, 1);
-    tc::mbar_init(a_empty, 1);
     for (int t = 0; t < 2; ++t) {
+      tc::mbar_init(&a_full[t], 1);
       tc::mbar_init(&acc_full[t], 1);
       tc::mbar_init(&acc_empty[t], kFusedEpiWarps / 2);
     }
+    tc::mbar_init(drain, 1);
     tc::fence_mbar_init();
     tc::tma_prefetch(&maps.q0);
   }
@@ -391,19 +205,26 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
   tc::tc_fence_after();
   const uint32_t tmem = *tslot;
   const unsigned long long deadline = tc::now_ns() + a.timeout_ns;
+  // the first item from w on (this CTA's step) that has tile t
+  auto next_with = [&](int w, int t) {
+    while (w < items && t >= tiles_of(w)) w += (int)gridDim.x;
+    return w;
+  };
+  auto load_input = [&](int w, int t) {
+    tc::mbar_expect_tx(&a_full[t], kStageA);
+    tc::tma_load_2d(base + t * kFusedA, &maps.q0, 0, ((w % a.n_pairs) * 2 + t) * kTileM, &a_full[t]);
+  };
 
   if (warp == 0) {
-    if (lane == 0) {
-      uint32_t it = 0, local = 0, a_loads = 0;
+    if (lane == 0 && (int)blockIdx.x < items) {
+      uint32_t it = 0;
       bool ok = true;
-      for (int w = blockIdx.x; w < items && ok; w += gridDim.x, ++local) {
-        const int e = w / a.n_pairs, pair = w % a.n_pairs;
-        // the previous item's last products have read A
-        if (local > 0 && !tc::mbar_wait(a_empty, (local - 1) & 1, deadline)) { ok = false; break; }
-        ++a_loads;
-        tc::mbar_expect_tx(a_full, 2 * kStageA);
-        tc::tma_load_2d(base, &maps.q0, 0, pair * 2 * kTileM, a_full);
-        tc::tma_load_2d(base + kFusedA, &maps.q0, 0, pair * 2 * kTileM + kTileM, a_full);
+      for (int t = 0; t < 2; ++t) {
+        const int n = next_with(blockIdx.x, t);
+        if (n < items) load_input(n, t);
+      }
+      for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        const int e = w / a.n_pairs;
         for (int l = 0; l < 4 && ok; ++l) {
           const int nk = (l == 0) ? 1 : kWidth / kChunk;
           for (int kc = 0; kc < nk; ++kc) {
@@ -425,65 +246,67 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         const unsigned long long d2 = tc::now_ns() + 1000000000ull;
         for (uint32_t j = (it > (uint32_t)kFusedStages ? it - kFusedStages : 0u); j < it; ++j)
           tc::mbar_wait(&full[j % kFusedStages], (j / kFusedStages) & 1, d2);
-        if (a_loads > 0) tc::mbar_wait(a_full, (a_loads - 1) & 1, d2);
+        for (int t = 0; t < 2; ++t)
+          if (next_with(blockIdx.x, t) < items) tc::mbar_wait(&a_full[t], 0, d2);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc = tc::idesc_bf16_f32(kTileM, kWidth);
-      uint32_t it = 0, layer = 0, local = 0;
+      uint32_t it = 0, layers[2] = {0, 0}, inputs[2] = {0, 0};
       bool ok = true;
-      for (int w = blockIdx.x; w < items && ok; w += gridDim.x, ++local) {
-        if (!tc::mbar_wait(a_full, local & 1, deadline)) { ok = false; break; }
-        for (int l = 0; l < 4 && ok; ++l, ++layer) {
-          // Issue order per layer (K chunks c0..c3, tiles X, Y sharing each
-          // chunk's stage): X c0 c1, Y c0 c1, X c2 c3, Y c2 c3.  X's products
-          // are complete two chunks before Y's, so X's epilogue overlaps Y's
-          // last products and Y's epilogue the next layer's first products
-          // of X.  Each tile's previous epilogue must have read its TMEM
-          // accumulator and written its A before the tile's first product.
+      for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        const int nt = tiles_of(w);
+        for (int l = 0; l < 4 && ok; ++l) {
           const int nk = (l == 0) ? 1 : kWidth / kChunk;
-          auto mma_tile = [&](int t, int kc, uint32_t st) {
-            const uint32_t aa = tc::smem_u32(base + t * kFusedA + kc * kStageA);
+          int ready = 0;                            // chunks of this layer known to have landed
+          // one product of the layer: waits for its operands and, with a tile's
+          // first, for the tile's previous epilogue; commits what it completes
+          auto product = [&](int t, int k) -> bool {
+            if (k == 0) {
+              if (l == 0 && !tc::mbar_wait(&a_full[t], inputs[t]++ & 1, deadline)) return false;
+              if (layers[t] > 0 && !tc::mbar_wait(&acc_empty[t], (layers[t] - 1) & 1, deadline)) return false;
+            }
+            const uint32_t st = (it + k) % kFusedStages;
+            if (k >= ready) {
+              if (!tc::mbar_wait(&full[st], ((it + k) / kFusedStages) & 1, deadline)) return false;
+              ready = k + 1;
+            }
+            tc::tc_fence_after();
+            const uint32_t aa = tc::smem_u32(base + t * kFusedA + k * kStageA);
             const uint32_t bb = tc::smem_u32(ring + st * kStageB);
 #pragma unroll
-            for (int k = 0; k < kChunk / 16; ++k)
-              tc::mma_bf16(tmem + (uint32_t)t * kTmemCols, tc::sdesc_sw128(aa + k * 32), tc::sdesc_sw128(bb + k * 32),
-                           idesc, (kc > 0 || k > 0) ? 1u : 0u);
+            for (int j = 0; j < kChunk / 16; ++j)
+              tc::mma_bf16(tmem + (uint32_t)t * kTmemCols, tc::sdesc_sw128(aa + j * 32), tc::sdesc_sw128(bb + j * 32),
+                           idesc, (k > 0 || j > 0) ? 1u : 0u);
+            if (t == nt - 1) tc::mma_commit(&empty[st]);      // Y follows X on every chunk
+            if (k == nk - 1) {
+              tc::mma_commit(&acc_full[t]);
+              ++layers[t];
+            }
+            return true;
           };
-          if (layer > 0 && !tc::mbar_wait(&acc_empty[0], (layer - 1) & 1, deadline)) { ok = false; break; }
-          tc::tc_fence_after();
-          for (int g = 0; g < nk && ok; g += 2) {
-            const int cnt = min(2, nk - g);
-            for (int j = 0; j < cnt; ++j) {
-              const uint32_t st = (it + j) % kFusedStages;
-              if (!tc::mbar_wait(&full[st], ((it + j) / kFusedStages) & 1, deadline)) { ok = false; break; }
-              tc::tc_fence_after();
-              mma_tile(0, g + j, st);
+          if (l == 0) {
+            ok = product(0, 0) && (nt == 1 || product(1, 0));
+          } else if (nt == 1) {
+            ok = product(0, 0) && product(0, 1) && product(0, 2) && product(0, 3);
+          } else {
+            int next[2] = {0, 0};
+#pragma unroll                                      // (every index below is a constant)
+            for (int i = 0; i < 8; ++i) {
+              const int t = (kFusedOrder >> i) & 1u;
+              ok = ok && product(t, next[t]);
+              ++next[t];
             }
-            if (!ok) break;
-            if (g + cnt == nk) tc::mma_commit(&acc_full[0]);
-            if (g == 0) {
-              if (layer > 0 && !tc::mbar_wait(&acc_empty[1], (layer - 1) & 1, deadline)) { ok = false; break; }
-              tc::tc_fence_after();
-            }
-            for (int j = 0; j < cnt; ++j) {
-              const uint32_t st = (it + j) % kFusedStages;
-              mma_tile(1, g + j, st);
-              tc::mma_commit(&empty[st]);
-            }
-            it += cnt;
           }
-          if (!ok) break;
-          tc::mma_commit(&acc_full[1]);
-          if (l == 3) tc::mma_commit(a_empty);
+          it += nk;
         }
       }
       if (!ok) {
         atomicExch(a.error, 12u);
         // products in flight finish before TMEM is given back
-        const unsigned long long d2 = tc::now_ns() + 1000000000ull;
-        if (it > 0) tc::mbar_wait(&empty[(it - 1) % kFusedStages], ((it - 1) / kFusedStages) & 1, d2);
+        tc::mma_commit(drain);
+        tc::mbar_wait(drain, 0, tc::now_ns() + 1000000000ull);
       }
     }
   } else {
@@ -493,28 +316,25 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
     const int r = q * 32 + lane;                   // row in the tile
     const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)t * kTmemCols + (uint32_t)(half * 128);
     unsigned char *arow = base + t * kFusedA + r * 128;
-    uint32_t layer = 0;
+    const bool loader = warp == 2 + 4 * t && lane == 0;
+    uint32_t layer = 0, loads = 1;                  // layers of this tile; inputs of this tile loaded
     bool ok = true;
-    // A warp whose wait ran out keeps walking the items without waiting or
-    // working, so every epilogue warp reaches the same named barriers.
-    for (int w = blockIdx.x; w < items; w += gridDim.x) {
+    for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+      if (t >= tiles_of(w)) continue;
       const int e = w / a.n_pairs, pair = w % a.n_pairs;
-      // this member's biases and head (every epilogue warp is past the
-      // previous item before they are replaced)
-      named_sync(1, 32 * kFusedEpiWarps);
-      const float *P = a.P[e];
-      for (int i = tid - 64; i < kWidth; i += 32 * kFusedEpiWarps) {
-        s_b[0][i] = 0.5f * P[kOffB1 + i];          // halved: silu_infer32
-        s_b[1][i] = 0.5f * P[kOffB2 + i];
-        s_b[2][i] = 0.5f * P[kOffB3 + i];
-        s_b[3][i] = 0.5f * P[kOffB4 + i];
-        s_w5[i] = P[kOffW5 + i];
-      }
-      named_sync(1, 32 * kFusedEpiWarps);
+      const float *epi = a.epi + (size_t)e * kEpiFloats;
       for (int l = 0; l < 4; ++l, ++layer) {
-        if (ok) ok = __all_sync(0xffffffffu, tc::mbar_wait(&acc_full[t], layer & 1, deadline));
-        if (!ok) continue;
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&acc_full[t], layer & 1, deadline));
+        if (!ok) break;
         tc::tc_fence_after();
+        if (l == 3) {                              // every product has read the tile's buffer
+          const int n = next_with(w + (int)gridDim.x, t);
+          if (n < items) {
+            if (loader) load_input(n, t);
+            ++loads;
+          }
+          __syncwarp();                            // the loads of TMEM below are warp-wide
+        }
         float hs = 0.0f;                       // head: this warp's half of the columns
         // 32-column chunks of the accumulator, the next chunk's TMEM load in
         // flight while this one is evaluated
@@ -530,10 +350,11 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(buf[c & 1][j]);
           __align__(16) __nv_bfloat16 out[32];
-          silu_infer32(v, &s_b[l][cc * 32], out);
+          silu_infer32(v, epi + l * kWidth + cc * 32, out);
           if (l == 3) {
+            const float *w5 = epi + 4 * kWidth + cc * 32;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) hs += __bfloat162float(out[j]) * s_w5[cc * 32 + j];
+            for (int j = 0; j < 32; ++j) hs = fmaf(__bfloat162float(out[j]), __ldg(w5 + j), hs);
           }
           if (l < 3) {
             // columns 32cc .. 32cc+31 = K-chunk cc / 2, 16-byte pieces 4 (cc % 2) .. +3
@@ -553,14 +374,17 @@ __global__ void __launch_bounds__(kFusedThreads, 1)
         if (lane == 0) tc::mbar_arrive(&acc_empty[t]);
         if (l == 3) {
           // y is zeroed before the launch: (columns 0-127 + b5) and columns
-          // 128-255 meet by atomic addition, (0 + x) + y == (0 + y) + x, the
-          // sum of the layer-by-layer path bit for bit
+          // 128-255 meet by atomic addition, (0 + x) + y == (0 + y) + x
           const int row = pair * 2 * kTileM + t * kTileM + r;
-          if (row < a.M) atomicAdd(&a.y[(size_t)e * a.stride + row], half == 0 ? hs + P[kOffB5] : hs);
+          if (row < a.M) atomicAdd(&a.y[(size_t)e * a.stride + row], half == 0 ? hs + __ldg(a.P[e] + kOffB5) : hs);
         }
       }
     }
-    if (!ok && lane == 0) atomicExch(a.error, 13u);
+    if (!ok && lane == 0) {
+      atomicExch(a.error, 13u);
+      // an input in flight lands before the shared memory is given back
+      if (loader && loads > 1) tc::mbar_wait(&a_full[t], (loads - 1) & 1, tc::now_ns() + 1000000000ull);
+    }
   }
   __syncthreads();
   if (warp == 1) {
@@ -584,12 +408,19 @@ __global__ void k_query_rows(const float *__restrict__ x, int n, int rows, __nv_
     x0[(size_t)m * kInPad + f] = __float2bfloat16_rn(m < n ? x[(size_t)m * kFeatures + f] : 0.0f);
 }
 
-// BF16 operand copies of the master weights: W1 padded to [256][64], W2..W4
-// and their transposes.
+// Operand copies of one member's master parameters: BF16 W1 padded to [256][64],
+// W2..W4 and their transposes; FP32 epilogue operands.
 __global__ void k_pack(const float *__restrict__ p, __nv_bfloat16 *__restrict__ w1, __nv_bfloat16 *__restrict__ w2,
                        __nv_bfloat16 *__restrict__ w3, __nv_bfloat16 *__restrict__ w4, __nv_bfloat16 *__restrict__ w2t,
-                       __nv_bfloat16 *__restrict__ w3t, __nv_bfloat16 *__restrict__ w4t) {
+                       __nv_bfloat16 *__restrict__ w3t, __nv_bfloat16 *__restrict__ w4t, float *__restrict__ epi) {
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx < kWidth) {
+    epi[idx] = 0.5f * p[kOffB1 + idx];
+    epi[kWidth + idx] = 0.5f * p[kOffB2 + idx];
+    epi[2 * kWidth + idx] = 0.5f * p[kOffB3 + idx];
+    epi[3 * kWidth + idx] = 0.5f * p[kOffB4 + idx];
+    epi[4 * kWidth + idx] = p[kOffW5 + idx];
+  }
   if (idx < kWidth * kInPad) {
     const int o = idx / kInPad, i = idx % kInPad;
     w1[idx] = __float2bfloat16_rn(i < kFeatures ? p[kOffW1 + o * kFeatures + i] : 0.0f);
@@ -612,72 +443,77 @@ __global__ void k_pack(const float *__restrict__ p, __nv_bfloat16 *__restrict__ 
 // Inference queries built on the device (gelio_surrogate_predict).
 // ---------------------------------------------------------------------------
 
-// One simulation of a predict query, prepared once per simulation by
-// k_query_sims: its six network inputs that do not depend on the energy and
-// its LOG_GRID range.
-struct QuerySim {
-  float f[6];
-  int points;
-  float pad;
-  double lmin, lmax;       // log of the grid's lowest and highest energy
-};
-static_assert(sizeof(QuerySim) == 48, "QuerySim is staged as 48-byte records");
-
-// The normalisation of gelio_surrogate_features, evaluated in FP64 and
-// rounded to FP32 as the host function does, one thread per simulation.
-__global__ void k_query_sims(const gelio_sim_params *__restrict__ sims, int n, QuerySim *__restrict__ out) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const gelio_sim_params s = sims[i];
-  const double rad = 180.0 / 3.14159265358979323846;
-  QuerySim q;
-  q.f[0] = (float)((log10((double)s.K0 / 4.4683705e-27) - 22.5) * 2.0);
-  q.f[1] = (float)(((double)s.V / 6.68458712e-9 - 550.0) / 200.0);
-  q.f[2] = (float)(((double)s.tilt * rad - 40.0) / 35.0);
-  q.f[3] = (float)s.polarity;
-  q.f[4] = (float)(((double)s.r_injection - 40.5) / 39.5);
-  q.f[5] = (float)(((double)s.theta_injection * rad - 90.0) / 80.0);
-  q.points = s.inj_points;
-  q.pad = 0.f;
-  q.lmin = log((double)s.inj_min);
-  q.lmax = log((double)s.inj_max);
-  out[i] = q;
-}
-
 // Rows [off, off + c) of the query (row = first[i] + j: grid point j of
 // simulation i) into the BF16 first-layer operand x0 [M][kInPad]; rows c..M-1
-// of the tile padding are zero.  Per row only the energy input is computed:
-// the LOG_GRID energy as the SDE kernels build it (FP64 exp, rounded to FP32)
-// and log10 of it / 2, as gelio_surrogate_features.
-__global__ void k_query_features(const QuerySim *__restrict__ sims, const long long *__restrict__ first,
-                                 int n_sims, long long off, int c, int M, __nv_bfloat16 *__restrict__ x0) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= M) return;
-  float f[kFeatures] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  if (m < c) {
-    const long long row = off + m;
-    int lo = 0, hi = n_sims - 1;          // last simulation with first[i] <= row
+// of the tile padding are zero.  Zeroes the members' outputs of these rows.
+//
+// The inputs are those of gelio_surrogate_features, evaluated in FP64 and
+// rounded to FP32 as the host function does: six depend on the simulation and
+// are formed once per simulation of the block's rows (a thread each), the
+// seventh is the LOG_GRID energy as the SDE kernels build it (FP64 exp, rounded
+// to FP32) and log10 of it / 2.  Bound by the FP64 pipe.
+constexpr int kQueryBlock = 128;
+__global__ void __launch_bounds__(kQueryBlock) k_query(const gelio_sim_params *__restrict__ sims,
+                                                       const long long *__restrict__ first, int n_sims, long long off,
+                                                       int c, int M, int E, long long stride,
+                                                       __nv_bfloat16 *__restrict__ x0, float *__restrict__ y) {
+  __shared__ float s_f[kQueryBlock][6];
+  __shared__ double s_lmin[kQueryBlock], s_range[kQueryBlock];
+  __shared__ int s_points[kQueryBlock];
+  const int m0 = blockIdx.x * kQueryBlock, m = m0 + threadIdx.x;
+  // last simulation with first[i] <= row
+  auto find = [&](long long row) {
+    int lo = 0, hi = n_sims - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
       if (first[mid] <= row) lo = mid; else hi = mid - 1;
     }
-    const QuerySim q = sims[lo];
-    const int j = (int)(row - first[lo]);
-    const double fr = (q.points > 1) ? (double)j / (double)(q.points - 1) : 0.0;
-    const float T = (float)exp(q.lmin + fr * (q.lmax - q.lmin));
-#pragma unroll
-    for (int k = 0; k < 6; ++k) f[k] = q.f[k];
-    f[6] = (float)(log10((double)T) / 2.0);
+    return lo;
+  };
+  // simulations have one grid point or more: the block's rows belong to at
+  // most kQueryBlock of them
+  const int i0 = find(off + min(m0, c - 1)), i1 = find(off + min(m0 + kQueryBlock, c) - 1);
+  if (i0 + (int)threadIdx.x <= i1) {
+    const gelio_sim_params s = sims[i0 + threadIdx.x];
+    const double rad = 180.0 / 3.14159265358979323846;
+    float *f = s_f[threadIdx.x];
+    f[0] = (float)((log10((double)s.K0 / 4.4683705e-27) - 22.5) * 2.0);
+    f[1] = (float)(((double)s.V / 6.68458712e-9 - 550.0) / 200.0);
+    f[2] = (float)(((double)s.tilt * rad - 40.0) / 35.0);
+    f[3] = (float)s.polarity;
+    f[4] = (float)(((double)s.r_injection - 40.5) / 39.5);
+    f[5] = (float)(((double)s.theta_injection * rad - 90.0) / 80.0);
+    s_points[threadIdx.x] = s.inj_points;
+    const double lmin = log((double)s.inj_min);
+    s_lmin[threadIdx.x] = lmin;
+    s_range[threadIdx.x] = log((double)s.inj_max) - lmin;
   }
+  __syncthreads();
+  if (m >= M) return;
+  __align__(16) __nv_bfloat16 v[8];
 #pragma unroll
-  for (int k = 0; k < kFeatures; ++k) x0[(size_t)m * kInPad + k] = __float2bfloat16_rn(f[k]);
+  for (int k = 0; k < 8; ++k) v[k] = __float2bfloat16_rn(0.0f);
+  if (m < c) {
+    const long long row = off + m;
+    const int i = find(row), q = i - i0, j = (int)(row - first[i]), points = s_points[q];
+    const double fr = (points > 1) ? (double)j / (double)(points - 1) : 0.0;
+    const float T = (float)exp(s_lmin[q] + fr * s_range[q]);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) v[k] = __float2bfloat16_rn(s_f[q][k]);
+    v[6] = __float2bfloat16_rn((float)(log10((double)T) / 2.0));
+    for (int e = 0; e < E; ++e) y[(size_t)e * stride + row] = 0.0f;
+  }
+  *reinterpret_cast<uint4 *>(x0 + (size_t)m * kInPad) = *reinterpret_cast<const uint4 *>(v);
 }
 
 // Ensemble mean and sample standard deviation (FP64) of E member outputs
-// y[e * stride + row].
+// y[e * stride + row]; the error flag follows the results, so that one copy
+// brings both.
 __global__ void k_ensemble(const float *__restrict__ y, int E, long long rows, long long stride,
-                           double *__restrict__ mean, double *__restrict__ sd) {
+                           double *__restrict__ mean, double *__restrict__ sd, const unsigned *__restrict__ error,
+                           unsigned *__restrict__ error_out) {
   const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (r == 0) *error_out = *error;
   if (r >= rows) return;
   double mu = 0.0;
   for (int e = 0; e < E; ++e) mu += (double)y[(size_t)e * stride + r];

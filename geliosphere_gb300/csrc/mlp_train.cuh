@@ -399,6 +399,8 @@ struct UpdateArgs {
   __nv_bfloat16 *w;         // BF16 operand copies of the layer, by member: [E][256][w_ld]
   __nv_bfloat16 *wt;        // transposed [E][256][256], null for the first layer
   int w_ld;
+  float *epi;               // FP32 epilogue operands of inference [E][5][256]
+  int epi_layer;            // this layer's row of it
 };
 
 // Adam (bias-corrected) on one FP32 master parameter; returns its new value.
@@ -483,8 +485,14 @@ __global__ void __launch_bounds__(256) k_update(const UpdateArgs u) {
     __syncthreads();
     class_tree(red, tid);
     if (tid < 32) {
-      if (u.grad) u.grad[off + f0 + lane] = red[0][lane];
-      else adam(u, slot, off + f0 + lane, red[0][lane]);
+      if (u.grad) {
+        u.grad[off + f0 + lane] = red[0][lane];
+      } else {
+        const float v = adam(u, slot, off + f0 + lane, red[0][lane]);
+        float *epi = u.epi + (size_t)(u.m0 + slot) * kEpiFloats + f0 + lane;
+        if (b < 8) epi[u.epi_layer * kWidth] = 0.5f * v;
+        else epi[4 * kWidth] = v;
+      }
     }
     return;
   }
