@@ -336,16 +336,20 @@ struct QEnt {
   unsigned slot_gbin;        // group slot (low 16 bits), grid bin + 1 (high 16 bits)
 };
 constexpr int kQueue = 64;   // entries per warp (<= 31 left + 32 pushed)
-// 1D: at most this many running trajectories in a warp whose tickets are
+// At most this many running trajectories in a warp whose tickets are
 // exhausted switch to normals drawn by the whole warp (>= 4 groups ahead each)
 constexpr int kCoopLanes = 8;
+// normals of a group of four steps
+__host__ __device__ constexpr int group_normals(int model) {
+  return model == kModelGeliosphere ? 12 : (model == kModelSolarProp ? 8 : 4);
+}
 
 // Dynamic shared memory of a persistent CTA: histograms of `slots`
 // simulations (rounded up to 16 bytes), then per warp its exit queue, its
-// cooperative normals (1D: 32 groups of four) and its queue length.
+// cooperative normals (32 groups of four steps) and its queue length.
 __host__ __device__ constexpr size_t hist_doubles(size_t slots, size_t window) { return (slots * window + 1) & ~(size_t)1; }
 __host__ __device__ constexpr size_t coop_bytes(int model, size_t real_bytes) {
-  return (model == kModelFp || model == kModelBp) ? 32 * 4 * real_bytes : 0;
+  return 32 * group_normals(model) * real_bytes;
 }
 __host__ __device__ constexpr size_t warp_bytes(int model, size_t real_bytes) {
   return kQueue * sizeof(QEnt) + coop_bytes(model, real_bytes) + sizeof(int);
@@ -433,8 +437,8 @@ static __device__ __noinline__ void emit_fp(Control *ctl, const SimDev *sims, ge
   }
 }
 
-// Advance one lane by one step of MODEL; normals are drawn per step group.
-// Returns the step result; `z` carries the per-call normals.
+// Advance one lane by one step of MODEL on the normals of one Philox call
+// (the plain kernel); j: the step within the call.  Returns the step result.
 template <int MODEL, class R>
 __device__ __forceinline__ int model_step(Lane<R> &L, const Consts<R> &K, const R *z, int j) {
   if constexpr (MODEL == kModelGeliosphere) return step_geliosphere(L, K, z[0], z[1], z[2]);
@@ -450,10 +454,9 @@ template <int MODEL> struct StepsPerCall {
 // 2D Geliosphere draws three normals per step (the reference's other two
 // multiply B13 = B23 = 0).  Each group of four steps takes its twelve normals
 // from three Philox calls, counters 3 g, 3 g + 1, 3 g + 2 for group
-// g = step / 4: step 4 g + p uses normals 3 p .. 3 p + 2 of the group, and
-// the ones a call draws ahead are carried in the lane.  Particles start only
-// at refill boundaries (multiples of four steps), so the lanes of a warp
-// share the phase p and the fourth step's skipped draw is warp-uniform.
+// g = step / 4: step 4 g + p uses normals 3 p .. 3 p + 2 of the group.  The
+// persistent kernel draws a group at once; here (the plain kernel) the ones a
+// call draws ahead are carried in the lane.
 template <class R>
 __device__ __forceinline__ void draw_geliosphere(Lane<R> &L, R *z) {
   const uint32_t p = L.steps & 3u;
@@ -594,8 +597,8 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   // (asked for, the longest went to the CTAs that started first: 60,000 2D
   // particles 28.3 ms, dealt 25.0).  The counter hands out those after.
   //
-  // exhausted (1D models, warp-uniform): every ticket is handed out, so no lane
-  // of this warp will be refilled again and the window grows to cut the votes
+  // exhausted (warp-uniform): every ticket is handed out, so no lane of this
+  // warp will be refilled again
   {
     const Spread spread = spread_lanes<R>(gpre[ne], gridDim.x, (unsigned)a.ctas_per_sm, warps);
     drained = (unsigned)lane >= spread.lanes || warp >= spread.warps;
@@ -650,7 +653,7 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
         }
         base = __shfl_sync(kFull, base, leader);
       }
-      if (Prefetch<MODEL>::value && base + (unsigned long long)__popc(need) >= total) exhausted = true;
+      if (base + (unsigned long long)__popc(need) >= total) exhausted = true;
       if (!active && !drained) {
         const unsigned long long t = base + __popc(need & lanemask_lt());
         if (t < total) {
@@ -682,8 +685,6 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
       break;
     }
     // 3) integrate `refill` steps (1D: at least 64 once the tickets are exhausted)
-    constexpr int spc = StepsPerCall<MODEL>::value;
-    const int win = (Prefetch<MODEL>::value && exhausted && a.refill < 64) ? 64 : a.refill;
     const uint32_t cap32 = (a.max_steps > 0xffffffffull) ? 0xffffffffu : (uint32_t)a.max_steps;
     // the end of a lane's trajectory (2D, B-p) with the result of its last step
     auto end_lane = [&](int res) {
@@ -744,20 +745,25 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
         }
       }
     };
-    if constexpr (Prefetch<MODEL>::value) {
-      // The tail of a 1D run: this warp's tickets are exhausted and at most
-      // kCoopLanes of its trajectories still run (F-p: often one chain of
-      // ~10^6 steps).  A trajectory's normals depend only on (key, particle,
-      // group of four steps), so every lane of the warp draws one group for
-      // one of the running trajectories -- 32 / n groups ahead for each of n
-      // -- into shared memory, and the running lanes then integrate those
-      // groups without drawing: a lone chain pays one warp-wide draw per 128
-      // steps instead of one per 4 steps on its own instruction stream.  The
-      // normals are those of the per-lane draws (a lane at a window start is
-      // at a group boundary), so the results are identical.
+    // The tail of a run: this warp's tickets are exhausted and at most
+    // kCoopLanes of its trajectories still run (F-p: often one chain of ~10^6
+    // steps; 2D: 10^4 to 6 10^4).  A trajectory's normals depend only on (key,
+    // particle, group of four steps), so every lane of the warp draws one group
+    // for one of the running trajectories -- 32 / n groups ahead for each of n
+    // -- into shared memory, and the running lanes then integrate those groups
+    // without drawing: a lone chain pays one warp-wide draw per 128 steps
+    // instead of one per 4 steps (2D: 3 or 2) on its own instruction stream.
+    // The normals are those of the per-lane draws (a lane at a window start is
+    // at a group boundary), so the results are identical.  4,096 2D Geliosphere
+    // trajectories 12.3 -> 9.7 ms, 4 x 12,000 26.1 -> 23.7, SolarProp-like 20,000
+    // 23.1 -> 22.3.
+    constexpr int NG = group_normals(MODEL);
+    const R *mine = nullptr;                           // this lane's normals, in order of its steps
+    int win = (Prefetch<MODEL>::value && exhausted && a.refill < 64) ? 64 : a.refill;
+    if (exhausted) {
       const unsigned act = __ballot_sync(kFull, active);
       const int na = __popc(act);
-      if (exhausted && na <= kCoopLanes) {
+      if (na <= kCoopLanes) {
         const int G = 32 / na;
         const int jt = lane % na, gi = lane / na;     // this lane draws group gi of the jt-th running lane
         unsigned m = act;
@@ -767,18 +773,27 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
         const uint32_t k1 = __shfl_sync(kFull, L.key1, src);
         const uint32_t st = __shfl_sync(kFull, L.steps, src);
         const unsigned long long pid = __shfl_sync(kFull, L.pid, src);
-        R zz[4];
-        normals4<R>(k0, k1, st / 4u + (uint32_t)gi, kStreamSde, pid, zz);
         if (gi < G) {
+#pragma unroll 1
+          for (int c = 0; c < NG / 4; ++c) {
+            R zz[4];
+            normals4<R>(k0, k1, (st / 4u + (uint32_t)gi) * (NG / 4) + c, kStreamSde, pid, zz);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) coop[(jt * G + gi) * 4 + j] = zz[j];
+            for (int j = 0; j < 4; ++j) coop[(jt * G + gi) * NG + 4 * c + j] = zz[j];
+          }
         }
         __syncwarp();
+        mine = coop + __popc(act & lanemask_lt()) * G * NG;
+        win = 4 * G;
+      }
+    }
+    if constexpr (Prefetch<MODEL>::value) {
+      if (mine != nullptr) {
         if (active) {
-          const R *mine = coop + __popc(act & lanemask_lt()) * G * 4;
           R z[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) z[j] = mine[j];
+          const int G = win / 4;
           for (int g = 1; g <= G && active; ++g) {
             R zn[4];                                   // the next group's, loaded under this one's steps
             const int gn = g < G ? g : 0;
@@ -793,28 +808,69 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
         continue;
       }
     }
-    for (int k = 0; k < win; k += (Prefetch<MODEL>::value ? 4 : spc)) {
-      if (active) {
-        R z[4];
-        if constexpr (Prefetch<MODEL>::value) {
+    if constexpr (Prefetch<MODEL>::value) {
+      for (int k = 0; k < win; k += 4) {
+        if (active) {
+          R z[4];
 #pragma unroll
           for (int j = 0; j < 4; ++j) z[j] = zq[j];
           normals_of<R>(philox_draw(rng, L.steps / 4u + 1u), zq);
           group_1d(z);
-        } else {
-          draw<MODEL, R>(L, z);
+        }
+      }
+    } else {
+      // one test per step covers the rare events: an exit, a stop, the step cap
+      // (an exit on the capped step counts as an exit)
+      auto step_2d = [&](R n0, R n1, R n2) {
+        const int res = (MODEL == kModelGeliosphere) ? step_geliosphere(L, K, n0, n1, n2) : step_solarprop(L, K, n0, n1);
+        ++L.steps;
+        if (res != kContinue || L.steps >= cap32) end_lane(res);
+      };
+      if constexpr (MODEL == kModelSolarProp) {
+        // two steps a Philox call, from registers or from the warp's draws
+        for (int k = 0; k < win; k += 2) {
+          if (active) {
+            R z[4];
+            if (mine != nullptr) {
 #pragma unroll
-          for (int j = 0; j < spc; ++j) {
-            if (active) {
-              const int res = model_step<MODEL, R>(L, K, z, j);
-              ++L.steps;
-              // one test per step covers the rare events: an exit, a stop,
-              // the step cap (an exit on the capped step counts as an exit)
-              if (res != kContinue || L.steps >= cap32) end_lane(res);
+              for (int j = 0; j < 4; ++j) z[j] = mine[k * 2 + j];
+            } else {
+              normals4<R>(L.key0, L.key1, L.steps >> 1, kStreamSde, L.pid, z);
             }
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+              if (active) step_2d(z[2 * j], z[2 * j + 1], R(0));
+          }
+        }
+      } else if (mine != nullptr) {
+        for (int k = 0; k < win && active; ++k, mine += 3) step_2d(mine[0], mine[1], mine[2]);
+      } else {
+        // A lane draws the normals of its next four steps into shared memory
+        // (the i-th at 32 i + lane) and then takes the steps: the three calls of
+        // a group share their round keys and what the particle index makes of
+        // the first two rounds, and no step asks for its place in the group.
+        // The steps stay a loop: laid out twice or four times they no longer
+        // fit the schedulers' instruction caches (4 x 2.5 M 499 -> 510 and
+        // 578 ms).
+        R *own = coop + lane;
+        for (int k = 0; k < win; k += 4) {
+          if (active) {
+            const uint32_t call = (L.steps >> 2) * 3u;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              R zz[4];
+              normals4<R>(L.key0, L.key1, call + c, kStreamSde, L.pid, zz);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) own[(4 * c + j) * 32] = zz[j];
+            }
+            const R *zp = own;
+#pragma unroll 1
+            for (int j = 0; j < 4; ++j, zp += 3 * 32)
+              if (active) step_2d(zp[0], zp[32], zp[64]);
           }
         }
       }
+      __syncwarp();                                    // the buffer is drawn again next window
     }
   }
   __syncthreads();

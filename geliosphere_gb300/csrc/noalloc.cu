@@ -48,7 +48,7 @@ constexpr size_t kOffGpre = align256(kOffGsim + sizeof(int) * 4 * kMaxN);
 constexpr size_t kOffPart = align256(kOffGpre + sizeof(unsigned long long) * 4 * (kMaxN + 1));
 constexpr size_t kScratchBytes = align256(kOffPart + sizeof(double) * (size_t)kSlices * kMaxN * kSpecDoubles);
 static_assert(kScratchBytes == GELIO_NOALLOC_SCRATCH_BYTES, "gelio.h states the scratch size");
-static_assert((256 / 32) * warp_bytes(kModelFp, sizeof(double)) <= 48 * 1024, "queues fit the default shared memory");
+static_assert((256 / 32) * warp_bytes(kModelGeliosphere, sizeof(double)) <= 48 * 1024, "queues fit the default shared memory");
 
 }  // namespace
 
@@ -89,7 +89,7 @@ cudaError_t launch(int m, int variant, unsigned grid, unsigned block, size_t sme
 }
 
 constexpr unsigned kBlock = 256;
-constexpr size_t kQueueBytes = (kBlock / 32) * warp_bytes(kModelFp, sizeof(double));   // the most of any kernel
+constexpr size_t kQueueBytes = (kBlock / 32) * warp_bytes(kModelGeliosphere, sizeof(double));   // the most of any kernel
 
 // Once per device, with that device current: resolve the scratch array's
 // device address, fill the bin tables and record the occupancy.  Runs on the
