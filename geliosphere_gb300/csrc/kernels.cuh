@@ -86,7 +86,6 @@ struct KArgs {
   unsigned long long time_limit_ns; // 0 = no watchdog
   int smem_slots;                 // >0: histograms of the group's first smem_slots sims in shared memory
   int refill;                     // steps between refills (multiple of 4)
-  int ctas_per_sm;                // of this launch (placement of small runs)
   // plain / replay kernel
   int plain_sim;                  // simulation index of a plain launch
   unsigned long long plain_first, plain_count;
@@ -337,8 +336,9 @@ struct QEnt {
 };
 constexpr int kQueue = 64;   // entries per warp (<= 31 left + 32 pushed)
 // At most this many running trajectories in a warp whose tickets are
-// exhausted switch to normals drawn by the whole warp (>= 4 groups ahead each)
-constexpr int kCoopLanes = 8;
+// exhausted switch to normals drawn by the whole warp (>= 4 groups ahead each;
+// FP64 16, >= 2 groups: a draw there is ~130 operations of the FP64 pipe).
+template <class R> constexpr int kCoopLanes = (sizeof(R) == 8) ? 16 : 8;
 // normals of a group of four steps
 __host__ __device__ constexpr int group_normals(int model) {
   return model == kModelGeliosphere ? 12 : (model == kModelSolarProp ? 8 : 4);
@@ -532,30 +532,18 @@ __device__ __forceinline__ int find_group_index(const unsigned long long *prefix
   return lo;
 }
 
-// Placement of a run of fewer trajectories than the launch has lanes.  Such a
-// run ends with its longest chains, and a chain is slowed by the warps it
-// shares its SM with and by the other lanes of its warp (their branches are
-// its own).  Handed out 32 to the warp that asks first, 4,096 trajectories sat
-// in 128 warps on 16 of the 152 SMs.  Instead each CTA opens only as many
-// warps as put kSpreadWarps on an SM (two a scheduler hide each other's
-// latency; FP64: one a scheduler, the SM's FP64 pipe takes 16 cycles an
-// instruction) and each warp as many lanes as the run needs.  A run that needs
-// more opens every warp, then every lane.  4,096 2D Geliosphere trajectories
-// 19.7 -> 16.3 ms; 4,001 1D B-p trajectories in FP64 steps 1,205 -> 849 ms.
-struct Spread {
-  unsigned warps, lanes;          // per CTA, per warp
-};
-template <class R>
-__device__ __forceinline__ Spread spread_lanes(unsigned long long total, unsigned ctas, unsigned ctas_per_sm,
-                                               unsigned warps_per_cta) {
-  constexpr unsigned kSpreadWarps = (sizeof(R) == 8) ? 4u : 8u;
-  Spread s;
-  s.warps = min(warps_per_cta, max(1u, kSpreadWarps / max(1u, ctas_per_sm)));
-  s.lanes = 32u;
-  if (total > (unsigned long long)ctas * s.warps * 32u) s.warps = warps_per_cta;
-  const unsigned long long w = (unsigned long long)ctas * s.warps;
-  if (total < w * 32u) s.lanes = (unsigned)((total + w - 1) / w);
-  return s;
+// Lanes that each warp of the launch opens.  A run of fewer trajectories than
+// the launch has lanes ends with its longest chains, and a chain is slowed by
+// the warps it shares its SM with and by the other lanes of its warp (their
+// branches are its own).  Handed out 32 to the warp that asks first, 4,096
+// trajectories sat in 128 warps on 16 of the 152 SMs.  Such a run is spread over
+// all warps, as many lanes in each as it needs: few enough, often, that the warp
+// draws their normals (kCoopLanes).  4,096 2D Geliosphere trajectories 19.7 ->
+// 16.3 ms, 4,001 1D B-p trajectories in FP64 steps 1,205 -> 849 ms; on half of
+// the warps 5,000 B-p trajectories took 10% longer.
+__device__ __forceinline__ unsigned spread_lanes(unsigned long long total, unsigned ctas, unsigned warps_per_cta) {
+  const unsigned long long w = (unsigned long long)ctas * warps_per_cta;
+  return total < w * 32u ? (unsigned)((total + w - 1) / w) : 32u;
 }
 
 // ---------------------------------------------------------------------------
@@ -600,9 +588,9 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   // exhausted (warp-uniform): every ticket is handed out, so no lane of this
   // warp will be refilled again
   {
-    const Spread spread = spread_lanes<R>(gpre[ne], gridDim.x, (unsigned)a.ctas_per_sm, warps);
-    drained = (unsigned)lane >= spread.lanes || warp >= spread.warps;
-    exhausted = gpre[ne] <= (unsigned long long)gridDim.x * spread.warps * spread.lanes;
+    const unsigned lanes = spread_lanes(gpre[ne], gridDim.x, warps);
+    drained = (unsigned)lane >= lanes;
+    exhausted = gpre[ne] <= (unsigned long long)gridDim.x * warps * lanes;
   }
   int slot = 0;
   unsigned window = 0;
@@ -644,11 +632,11 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
     if (need) {
       const int leader = __ffs(need) - 1;
       const unsigned long long total = gpre[ne];
-      const Spread spread = spread_lanes<R>(total, gridDim.x, (unsigned)a.ctas_per_sm, warps);
-      unsigned long long base = ((unsigned long long)warp * gridDim.x + blockIdx.x) * spread.lanes;
+      const unsigned lanes = spread_lanes(total, gridDim.x, warps);
+      unsigned long long base = ((unsigned long long)warp * gridDim.x + blockIdx.x) * lanes;
       if (window > 1u) {
         if (lane == leader) {
-          const unsigned long long dealt = (unsigned long long)gridDim.x * spread.warps * spread.lanes;
+          const unsigned long long dealt = (unsigned long long)gridDim.x * warps * lanes;
           base = dealt + atomicAdd(&a.ctl->ticket[MODEL], (unsigned long long)__popc(need));
         }
         base = __shfl_sync(kFull, base, leader);
@@ -763,7 +751,7 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
     if (exhausted) {
       const unsigned act = __ballot_sync(kFull, active);
       const int na = __popc(act);
-      if (na <= kCoopLanes) {
+      if (na <= kCoopLanes<R>) {
         const int G = 32 / na;
         const int jt = lane % na, gi = lane / na;     // this lane draws group gi of the jt-th running lane
         unsigned m = act;

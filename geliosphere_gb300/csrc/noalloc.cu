@@ -194,7 +194,6 @@ extern "C" int32_t gelio_run_noalloc(const gelio_sim_params *d_sims, int32_t n_s
   a.time_limit_ns = (opts && opts->time_limit_s > 0.0) ? (unsigned long long)(opts->time_limit_s * 1e9) : 0ull;
   a.smem_slots = 0;                        // histograms go to the scratch slices
   const unsigned grid = (unsigned)(s->sm_count * s->occ[variant]);
-  a.ctas_per_sm = s->occ[variant];
   for (int m = 0; m < 4; ++m) {
     a.refill = (opts && opts->refill_interval > 0) ? opts->refill_interval : (m == kModelFp ? 4 : 16);
     if (launch(m, variant, grid, kBlock, kQueueBytes, st, a) != cudaSuccess) return GELIO_ERR_CUDA;

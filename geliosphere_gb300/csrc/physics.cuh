@@ -75,7 +75,7 @@ template <> struct Math<double> {
   static constexpr bool kCompensate = false;
   __device__ static __forceinline__ double sqrt(double x) { return ::sqrt(x); }
   __device__ static __forceinline__ double rsqrt(double x) { return ::rsqrt(x); }
-  __device__ static __forceinline__ double rcp(double x) { return 1.0 / x; }
+  __device__ static __forceinline__ double rcp(double x) { return __drcp_rn(x); }   // = 1.0 / x, both correctly rounded
   __device__ static __forceinline__ double div(double a, double b) { return a / b; }
   __device__ static __forceinline__ void sincos(double x, double *s, double *c) { ::sincos(x, s, c); }
   __device__ static __forceinline__ double sin(double x) { return ::sin(x); }
@@ -83,13 +83,11 @@ template <> struct Math<double> {
   __device__ static __forceinline__ double atan(double x) { return ::atan(x); }
   __device__ static __forceinline__ double abs(double x) { return fabs(x); }
   __device__ static __forceinline__ double copysign(double x, double y) { return ::copysign(x, y); }
-  __device__ static __forceinline__ double min(double x, double y) { return fmin(x, y); }
   __device__ static __forceinline__ double fma(double a, double b, double c) { return ::fma(a, b, c); }
   __device__ static __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
   __device__ static __forceinline__ double mul_add(double a, double b, double c) {
     return __dadd_rn(__dmul_rn(a, b), c);
   }
-  __device__ static __forceinline__ double max(double x, double y) { return fmax(x, y); }
 };
 
 // Kahan-compensated scalar: value v, running compensation c (true ~ v - c).
@@ -661,7 +659,15 @@ __device__ __forceinline__ bool four_quiet_steps(Lane<R> &L, const Consts<R> &k,
   const R T0 = (R)kT0;
   Acc<R> r = L.r, P = L.P, sumac = L.sumac;
   R Pt = L.Pt, q = L.q;
-  R lo = r.v, hi = r.v, beta = Pt * q, beta_low = beta;
+  R beta = Pt * q;
+  // Running bounds of r and beta.  FP64: of their high words, which order
+  // positive numbers, so that the bounds stay off the FP64 pipe.
+  R lo = r.v, hi = r.v, beta_low = beta;
+  int lo_hw = 0, hi_hw = 0, beta_hw = 0;
+  if constexpr (sizeof(R) == 8) {
+    lo_hw = hi_hw = __double2hiint(r.v);
+    beta_hw = __double2hiint(beta);
+  }
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const R inv_r = M::rcp(r.v);
@@ -679,14 +685,26 @@ __device__ __forceinline__ bool four_quiet_steps(Lane<R> &L, const Consts<R> &k,
     Pt = P.v;
     q = M::rsqrt(M::mul_add(Pt, Pt, T0 * T0));
     beta = Pt * q;
-    lo = M::min(lo, r.v);
-    hi = M::max(hi, r.v);
-    if (MODEL == kModelBp || j < 3) beta_low = M::min(beta_low, beta);
+    if constexpr (sizeof(R) == 4) {
+      lo = M::min(lo, r.v);
+      hi = M::max(hi, r.v);
+      if (MODEL == kModelBp || j < 3) beta_low = M::min(beta_low, beta);
+    } else {
+      lo_hw = ::min(lo_hw, __double2hiint(r.v));
+      hi_hw = ::max(hi_hw, __double2hiint(r.v));
+      if (MODEL == kModelBp || j < 3) beta_hw = ::min(beta_hw, __double2hiint(beta));
+    }
   }
   const R r_low = (MODEL == kModelBp) ? (R)0.3f : (R)1.5f;
   // (a NaN passes through the minimum and maximum: in r it stays to the last
   // step, in beta it is no event)
-  const bool quiet = lo >= r_low && hi <= R(100) && r.v <= R(100) && beta_low > (R)0.01f;
+  bool quiet;
+  if constexpr (sizeof(R) == 4) {
+    quiet = lo >= r_low && hi <= R(100) && r.v <= R(100) && beta_low > (R)0.01f;
+  } else {
+    // equal high words: not sure, an event; a NaN's or a negative number's miss a bound
+    quiet = lo_hw > __double2hiint(r_low) && hi_hw < __double2hiint(100.0) && beta_hw > __double2hiint((double)0.01f);
+  }
   if (quiet) {
     L.r = r;
     L.P = P;

@@ -38,8 +38,8 @@ def test_every_particle_once(engine, model, prec, counts):
         same(a, b)
 
 
-# around the placement's lines: the warps opened on two CTAs a SM (152 SMs x 8), all warps, all lanes
-@pytest.mark.parametrize("n", [1215, 1217, 38911, 38913, 77823, 77825])
+# around the placement's lines: one, two, sixteen and all lanes of the launch's 2,432 warps
+@pytest.mark.parametrize("n", [2431, 2433, 38911, 38913, 77823, 77825])
 def test_small_runs_at_the_lines_of_the_placement(engine, n):
     sim = make_sim(abi.GELIO_MODEL_2D_SOLARPROP, n, injection=LOG, inj_min=30.0, inj_max=100.0, inj_points=7, seed=3)
     same(engine.run(sim).spectra[0], engine.run(sim, plain=True).spectra[0])
