@@ -51,6 +51,13 @@ constexpr int kModelGeliosphere = 3;
 // ---------------------------------------------------------------------------
 template <class R> struct Math;
 
+// sinf of the current sheet's angle beyond 10^5 rad (no usual energy reaches
+// it), out of line: inside the 2D steps' loop the reduction of such arguments is
+// only in the way of the schedulers' instruction caches (4 x 2.5 M Geliosphere
+// 496.0 -> 492.4 ms, the 48-row batch 114.3 -> 112.6; the same for theta's
+// sincosf gained nothing).
+static __device__ __noinline__ float far_sin(float x) { return sinf(x); }
+
 template <> struct Math<float> {
   static constexpr bool kCompensate = true;
   __device__ static __forceinline__ float sqrt(float x) { return sqrtf(x); }
@@ -58,7 +65,7 @@ template <> struct Math<float> {
   __device__ static __forceinline__ float rcp(float x) { return __fdividef(1.0f, x); }
   __device__ static __forceinline__ float div(float a, float b) { return __fdividef(a, b); }
   __device__ static __forceinline__ void sincos(float x, float *s, float *c) { sincosf(x, s, c); }
-  __device__ static __forceinline__ float sin(float x) { return sinf(x); }
+  __device__ static __forceinline__ float sin(float x) { return fabsf(x) <= 1.0e5f ? sinf(x) : far_sin(x); }
   __device__ static __forceinline__ float acos(float x) { return acosf(x); }
   __device__ static __forceinline__ float atan(float x) { return atanf(x); }
   __device__ static __forceinline__ float abs(float x) { return fabsf(x); }
