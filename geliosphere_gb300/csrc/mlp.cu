@@ -119,10 +119,10 @@ struct Member {
 struct TrainBuffers {
   int G = 0;
   bf16 *X0 = nullptr, *Z[4] = {}, *X[4] = {}, *dH[4] = {};
-  float *yhat = nullptr, *y = nullptr, *dy = nullptr, *partial = nullptr, *cls = nullptr, *cls5 = nullptr;
+  float *yhat = nullptr, *y = nullptr, *dy = nullptr, *cls = nullptr;
   float *loss_part = nullptr;
   CUtensorMap aX0, aX[3], adH[4];        // row tiles of 128 (K-major operands)
-  CUtensorMap bX0, bX[3], bdH[4];        // boxes of 64 rows (MN-major operands of dW)
+  DwMaps dw;                             // boxes of 64 rows (MN-major operands of dW)
 };
 
 }  // namespace
@@ -137,7 +137,8 @@ struct gelio_surrogate {
   gelio_ctx *ctx = nullptr;
   gelio_surrogate_opts o{};
   int device = 0, sm_count = 0, rows = 0;   // rows = batch rows
-  cudaStream_t stream = nullptr;
+  cudaStream_t stream = nullptr, side = nullptr;   // side: bias and head gradients of a training step
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   std::vector<Member> mem;
   // BF16 operand copies of every member's weights, [members][256][fan-in]
   bf16 *W1 = nullptr, *W[3] = {}, *WT[3] = {};
@@ -202,12 +203,13 @@ int set_smem_attrs() {
     cudaError_t e = cudaSuccess;
     auto set = [&](const void *f) {
       if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem);
+        e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTrainSmem);
     };
     set((const void *)k_train_gemm<FWD>);
     set((const void *)k_train_gemm<FWD_LAST>);
     set((const void *)k_train_gemm<DX>);
-    set((const void *)k_train_gemm<DW>);
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute((const void *)k_train_dw, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDwSmem);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute((const void *)k_mlp_infer_fused, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kFusedSmem);
@@ -220,7 +222,7 @@ void free_train(TrainBuffers &t) {
   auto f = [](void *p) { if (p) cudaFree(p); };
   f(t.X0);
   for (int i = 0; i < 4; ++i) { f(t.Z[i]); f(t.X[i]); f(t.dH[i]); }
-  f(t.yhat); f(t.y); f(t.dy); f(t.partial); f(t.cls); f(t.cls5); f(t.loss_part);
+  f(t.yhat); f(t.y); f(t.dy); f(t.cls); f(t.loss_part);
   t = TrainBuffers();
 }
 
@@ -239,6 +241,9 @@ void free_all(gelio_surrogate *s) {
   for (auto &e : s->ev_copy) if (e) cudaEventDestroy(e);
   if (s->ev0) cudaEventDestroy(s->ev0);
   if (s->ev1) cudaEventDestroy(s->ev1);
+  if (s->ev_fork) cudaEventDestroy(s->ev_fork);
+  if (s->ev_join) cudaEventDestroy(s->ev_join);
+  if (s->side) cudaStreamDestroy(s->side);
   if (s->stream) cudaStreamDestroy(s->stream);
 }
 
@@ -266,7 +271,7 @@ int check_error(gelio_surrogate *s) {
 // always took), within the ensemble.
 int group_size(const gelio_surrogate *s) {
   const size_t R = (size_t)s->rows;
-  const size_t per = R * kInPad * 2 + 12 * R * kWidth * 2 + (R / kSplitRows) * kWidth * kWidth * 4;
+  const size_t per = R * kInPad * 2 + 12 * R * kWidth * 2;
   return (int)std::max<size_t>(1, std::min(s->mem.size(), ((size_t)2 << 30) / per));
 }
 
@@ -289,17 +294,15 @@ int ensure_train(gelio_surrogate *s, int G) {
   alloc(&t.yhat, g * R);
   alloc(&t.y, g * R);
   alloc(&t.dy, g * R);
-  alloc(&t.partial, g * (R / kSplitRows) * kWidth * kWidth);
-  alloc(&t.cls, g * kClasses * kWidth);
-  alloc(&t.cls5, g * kClasses * kWidth);
+  alloc(&t.cls, g * 5 * kClasses * kWidth);
   alloc(&t.loss_part, g * (R / kHeadRows));
   if (e == cudaSuccess) e = cudaMemsetAsync(t.X0, 0, g * R * kInPad * 2, s->stream);   // the padding columns
   bool ok = e == cudaSuccess;
-  ok = ok && make_map3(&t.aX0, t.X0, kInPad, R, g, kTileM) && make_map3(&t.bX0, t.X0, kInPad, R, g, kChunk);
+  ok = ok && make_map3(&t.aX0, t.X0, kInPad, R, g, kTileM) && make_map3(&t.dw.x[0], t.X0, kInPad, R, g, kChunk);
   for (int i = 0; i < 4; ++i) {
     if (i < 3)
-      ok = ok && make_map3(&t.aX[i], t.X[i], kWidth, R, g, kTileM) && make_map3(&t.bX[i], t.X[i], kWidth, R, g, kChunk);
-    ok = ok && make_map3(&t.adH[i], t.dH[i], kWidth, R, g, kTileM) && make_map3(&t.bdH[i], t.dH[i], kWidth, R, g, kChunk);
+      ok = ok && make_map3(&t.aX[i], t.X[i], kWidth, R, g, kTileM) && make_map3(&t.dw.x[i + 1], t.X[i], kWidth, R, g, kChunk);
+    ok = ok && make_map3(&t.adH[i], t.dH[i], kWidth, R, g, kTileM) && make_map3(&t.dw.dh[i], t.dH[i], kWidth, R, g, kChunk);
   }
   if (!ok) {
     free_train(t);
@@ -314,22 +317,22 @@ int ensure_train(gelio_surrogate *s, int G) {
 
 template <int MODE>
 int launch_train(gelio_surrogate *s, const CUtensorMap &A, const CUtensorMap &B, const TrainArgs &a) {
-  int grid;
-  if (MODE == DW) grid = std::min(s->sm_count, a.G * (a.rows / kSplitRows) * 2);
-  else grid = a.G * std::max(1, std::min(s->sm_count / a.G, a.rows / kTileM));   // the same CTAs for each slot
-  k_train_gemm<MODE><<<grid, kGemmThreads, kGemmSmem, s->stream>>>(A, B, a);
+  // the same number of CTAs for each slot
+  const int grid = a.G * std::max(1, std::min(s->sm_count / a.G, a.rows / kTileM));
+  k_train_gemm<MODE><<<grid, kTrainThreads, kTrainSmem, s->stream>>>(A, B, a);
   return cuda_status(cudaGetLastError());
 }
 
 // One step of members [m0, m0 + G) on the gathered batches: forward, backward
-// and, layer by layer from the top, the update that u describes (Adam's step,
-// or the gradient of one member).  A layer's dX runs before its weights change.
+// and the update that u describes (Adam's step, or the gradient of one member).
+// The bias and head gradients run beside the weight gradients, on a stream of
+// their own.
 int train_step(gelio_surrogate *s, int m0, int G, int n_valid, UpdateArgs &u) {
   TrainBuffers &t = s->tb;
   const int R = s->rows;
   int rc;
   TrainArgs a{};
-  a.rows = R; a.G = G; a.m0 = m0; a.N = kWidth;
+  a.rows = R; a.G = G; a.m0 = m0;
   a.error = s->error; a.timeout_ns = 2000000000ull;
   for (int g = 0; g < G; ++g) a.P[g] = s->mem[m0 + g].P;
   // forward
@@ -341,40 +344,42 @@ int train_step(gelio_surrogate *s, int m0, int G, int n_valid, UpdateArgs &u) {
   if ((rc = launch_train<FWD>(s, t.aX[1], s->tW[1], a)) != GELIO_OK) return rc;
   a.off_bias = kOffB4; a.z_out = t.Z[3]; a.x_out = t.X[3]; a.y_out = t.yhat;
   if ((rc = launch_train<FWD_LAST>(s, t.aX[2], s->tW[2], a)) != GELIO_OK) return rc;
-  // head
+  // head, then the hidden layers, top down
   k_head_backward<<<dim3(R / kHeadRows, G), 256, 0, s->stream>>>(t.yhat, t.y, n_valid, R, a, t.Z[3], t.dH[3], t.dy,
                                                                  t.loss_part);
-  k_class_sums<<<dim3(kClasses / 32, kWidth / 64, G), 256, 0, s->stream>>>(t.X[3], t.dy, R, t.cls5);
   SUR_TRY(cudaGetLastError());
-  // hidden layers, top down
-  const int offW[4] = {kOffW1, kOffW2, kOffW3, kOffW4};
-  const int offB[4] = {kOffB1, kOffB2, kOffB3, kOffB4};
-  u.rows = R; u.splits = R / kSplitRows; u.partial = t.partial; u.cls = t.cls; u.m0 = m0;
-  for (int li = 3; li >= 0; --li) {
-    k_class_sums<<<dim3(kClasses / 32, kWidth / 64, G), 256, 0, s->stream>>>(t.dH[li], nullptr, R, t.cls);
-    SUR_TRY(cudaGetLastError());
-    if (li > 0) {
-      a.K = kWidth; a.N = kWidth; a.z_prev = t.Z[li - 1]; a.dh_out = t.dH[li - 1];
-      if ((rc = launch_train<DX>(s, t.adH[li], s->tWT[li - 1], a)) != GELIO_OK) return rc;
-    }
-    a.K = kSplitRows; a.N = (li == 0) ? kInPad : kWidth; a.partial = t.partial;
-    if ((rc = launch_train<DW>(s, t.bdH[li], li == 0 ? t.bX0 : t.bX[li - 1], a)) != GELIO_OK) return rc;
-    u.N = a.N;
-    u.fan_in = (li == 0) ? kFeatures : kWidth;
-    u.off_w = offW[li];
-    u.off_b = offB[li];
-    u.cls5 = (li == 3) ? t.cls5 : nullptr;
-    u.dy = t.dy;
-    u.loss_part = t.loss_part;
-    u.w = (li == 0) ? s->W1 : s->W[li - 1];
-    u.wt = (li == 0) ? nullptr : s->WT[li - 1];
-    u.w_ld = (li == 0) ? kInPad : kWidth;
-    u.epi = s->epi;
-    u.epi_layer = li;
-    const int blocks = 8 * ((u.fan_in + 31) / 32) + 8 + (li == 3 ? 9 : 0);
-    k_update<<<dim3(blocks, G), 256, 0, s->stream>>>(u);
-    SUR_TRY(cudaGetLastError());
+  for (int li = 3; li > 0; --li) {
+    a.K = kWidth; a.z_prev = t.Z[li - 1]; a.dh_out = t.dH[li - 1];
+    if ((rc = launch_train<DX>(s, t.adH[li], s->tWT[li - 1], a)) != GELIO_OK) return rc;
   }
+  u.rows = R; u.G = G; u.m0 = m0;
+  for (int li = 0; li < 4; ++li) {
+    u.w[li] = (li == 0) ? s->W1 : s->W[li - 1];
+    u.wt[li] = (li == 0) ? nullptr : s->WT[li - 1];
+  }
+  u.epi = s->epi;
+  u.cls = t.cls;
+  u.dy = t.dy;
+  u.loss_part = t.loss_part;
+  u.error = s->error;
+  u.timeout_ns = a.timeout_ns;
+  SUR_TRY(cudaEventRecord(s->ev_fork, s->stream));
+  SUR_TRY(cudaStreamWaitEvent(s->side, s->ev_fork, 0));
+  ClassSources c{};
+  for (int li = 0; li < 4; ++li) c.src[li] = t.dH[li];
+  c.src[4] = t.X[3];
+  c.dy = t.dy;
+  // 64 inputs a tile while that is one item an SM or fewer (26 a member: 5
+  // members of 16,384 rows 128 us; at 128 inputs 70 of the SMs work, 190 us)
+  const int n_tile = 26 * G <= s->sm_count ? 64 : 128;
+  const int items = G * 2 * (3 * (kWidth / n_tile) + 1);
+  k_train_dw<<<std::min(items, s->sm_count), kTrainThreads, kDwSmem, s->stream>>>(t.dw, u, n_tile);
+  SUR_TRY(cudaGetLastError());
+  k_class_sums<<<dim3(kClasses / kClassBlock, kWidth / 64, 5 * G), 256, 0, s->side>>>(c, R, t.cls);
+  k_update_biases<<<dim3(41, G), 256, 0, s->side>>>(u);
+  SUR_TRY(cudaGetLastError());
+  SUR_TRY(cudaEventRecord(s->ev_join, s->side));
+  SUR_TRY(cudaStreamWaitEvent(s->stream, s->ev_join, 0));
   return GELIO_OK;
 }
 
@@ -528,6 +533,7 @@ int train_group(gelio_surrogate *s, int m0, int g, int epochs, int steps, long l
   }
   join();
   if (rc != GELIO_OK) {
+    cudaStreamSynchronize(s->side);
     cudaStreamSynchronize(s->stream);
     return rc;
   }
@@ -602,8 +608,9 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
   cudaDeviceGetAttribute(&s->sm_count, cudaDevAttrMultiProcessorCount, s->device);
   if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess) return fail(GELIO_ERR_CUDA);
   if (cudaEventCreate(&s->ev0) != cudaSuccess || cudaEventCreate(&s->ev1) != cudaSuccess) return fail(GELIO_ERR_CUDA);
-  for (auto &e : s->ev_copy)
-    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(GELIO_ERR_CUDA);
+  if (cudaStreamCreateWithFlags(&s->side, cudaStreamNonBlocking) != cudaSuccess) return fail(GELIO_ERR_CUDA);
+  for (cudaEvent_t *e : {&s->ev_copy[0], &s->ev_copy[1], &s->ev_fork, &s->ev_join})
+    if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return fail(GELIO_ERR_CUDA);
   const size_t R = (size_t)s->rows;
   auto alloc = [&](void **p, size_t bytes) {
     if (rc != GELIO_OK) return;
@@ -676,6 +683,7 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
 void gelio_surrogate_destroy(gelio_surrogate *s) {
   if (!s) return;
   cudaSetDevice(s->device);
+  if (s->side) cudaStreamSynchronize(s->side);
   if (s->stream) cudaStreamSynchronize(s->stream);
   free_all(s);
   delete s;
@@ -921,6 +929,7 @@ int32_t gelio_surrogate_gradient(gelio_surrogate *s, int32_t member, const float
        cudaMemcpyAsync(&l, d_loss, 4, cudaMemcpyDeviceToHost, s->stream) != cudaSuccess))
     rc = GELIO_ERR_CUDA;
   if (rc == GELIO_OK) rc = check_error(s);
+  cudaStreamSynchronize(s->side);
   cudaStreamSynchronize(s->stream);
   if (loss) *loss = l / (float)n;
   cudaFree(d_x);

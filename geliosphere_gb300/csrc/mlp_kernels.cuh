@@ -19,12 +19,9 @@ constexpr int kFeatures = 7;      // (K0, V, tilt, polarity, r, theta, log T)
 constexpr int kInPad = 64;        // first-layer K padded to one 128-byte row
 constexpr int kTileM = 128;       // GEMM rows per tile (TMEM lanes)
 constexpr int kChunk = 64;        // K per pipeline stage (128 B of BF16)
-constexpr int kStages = 4;
-constexpr int kThreads = 128;
 constexpr uint32_t kStageA = kTileM * kChunk * 2;   // 16 KiB
 constexpr uint32_t kStageB = kWidth * kChunk * 2;   // 32 KiB (N = 256)
 constexpr uint32_t kTmemCols = 256;
-constexpr size_t kGemmSmem = 1024 + (size_t)kStages * (kStageA + kStageB) + 128;
 
 // Flat parameter layout (FP32 master copy and gradients).
 constexpr int kOffW1 = 0;                                   // [256][7]
@@ -91,12 +88,6 @@ __device__ __forceinline__ void store_rows(const uint4 (&v)[4], __nv_bfloat16 *d
   }
   __syncwarp();
 }
-
-// Training GEMMs (mlp_train.cuh): shared memory regions and warps.
-constexpr int kEpiWarps = 8;
-constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
-constexpr uint32_t kRegion1 = 4 * kStageB;         // 128 KiB
-constexpr uint32_t kRegion2 = kStages * kStageA;   // 64 KiB
 
 // ----------------------------------------------------------------------------
 // Whole-network inference, several ensemble members in one persistent launch.

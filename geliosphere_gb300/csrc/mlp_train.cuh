@@ -5,18 +5,18 @@
 // m0..m0+G-1 of the ensemble), every activation buffer is [G][rows][256].
 // One member alone fills neither the SMs (128 row tiles of a 16,384-row batch)
 // nor hides the launches: 27 launches and 410 us a step and member at 16,384
-// rows, now 21 launches and 125 us a member for a group of five (200,000 rows,
-// 2 epochs: 49.2 -> 15.8 ms).
+// rows, now 12 launches and 85 us a member for a group of five (200,000 rows,
+// 2 epochs: 49.2 -> 10.8 ms).
 //
 // All operands are row-major in HBM, written once:
 //   forward   Z_l  = X_{l-1} W_l^T    A = X_{l-1} [rows x in]   (K-major)  B = W_l   [256 x in]
 //   dX        dH_{l-1} = dH_l W_l * SiLU'(Z_{l-1})  A = dH_l    (K-major)  B = W_l^T [in x 256]
 //   dW        dW_l = dH_l^T X_{l-1}   A = dH_l, B = X_{l-1}, both read MN-major (the
 //             reduction runs over the rows), so no transposed copy is written
-// Weight gradients are split over the batch into FP32 partials of 256 rows,
-// added in their order; bias and head gradients are sums over the rows of one
-// class modulo 256, added by a fixed tree: a gradient is deterministic and
-// does not depend on the group it is computed in.
+// Weight gradients are sums of FP32 partials of 256 batch rows, added in their
+// order; bias and head gradients are sums over the rows of one class modulo 256,
+// added by a fixed tree: a gradient is deterministic and does not depend on the
+// group it is computed in.
 #pragma once
 #include "mlp_kernels.cuh"
 
@@ -28,14 +28,20 @@ constexpr int kClasses = 256;     // row classes of the bias and head gradients
 constexpr int kSplitRows = 256;   // batch rows of one dW partial
 constexpr int kHeadRows = 128;    // rows of one loss partial
 
-enum TrainMode { FWD = 0, FWD_LAST = 1, DX = 2, DW = 3 };
+enum TrainMode { FWD = 0, FWD_LAST = 1, DX = 2 };
+
+constexpr int kTrainStages = 4;
+constexpr int kEpiWarps = 8;
+constexpr int kTrainThreads = 64 + 32 * kEpiWarps;
+constexpr uint32_t kRegion1 = 4 * kStageB;              // 128 KiB: a layer's weights
+constexpr uint32_t kRegion2 = kTrainStages * kStageA;   // 64 KiB: row tiles
+constexpr size_t kTrainSmem = 1024 + (size_t)kRegion1 + kRegion2 + 128;
 
 struct TrainArgs {
   int rows;                 // batch rows (a multiple of 256)
   int G;                    // members in this launch
   int m0;                   // first member (weights, parameters)
-  int N;                    // GEMM columns: 256, or 64 for the first layer's DW
-  int K;                    // layer fan-in (FWD*: 64 or 256, DX: 256); DW: kSplitRows
+  int K;                    // layer fan-in (FWD*: 64 or 256, DX: 256)
   const float *P[kMaxMembers];   // FP32 parameters by slot
   int off_bias;
   __nv_bfloat16 *z_out;     // FWD*: pre-activations
@@ -43,7 +49,6 @@ struct TrainArgs {
   float *y_out;             // FWD_LAST: head outputs [G][rows], zeroed before
   const __nv_bfloat16 *z_prev;   // DX
   __nv_bfloat16 *dh_out;    // DX
-  float *partial;           // DW: [G][rows / 256][N][256]
   unsigned *error;
   unsigned long long timeout_ns;
 };
@@ -51,9 +56,8 @@ struct TrainArgs {
 // Columns [32 c_begin, 32 c_end) of one accumulator row (row = row0 + lane of
 // the slot's batch); returns this thread's part of the head's dot product.
 template <int MODE>
-__device__ __forceinline__ float train_epilogue(const TrainArgs &a, size_t row, uint32_t trow, float *part, int c_begin,
-                                                int c_end, unsigned char *stage, int lane, const float *sbias,
-                                                const float *sw5) {
+__device__ __forceinline__ float train_epilogue(const TrainArgs &a, size_t row, uint32_t trow, int c_begin, int c_end,
+                                                unsigned char *stage, int lane, const float *sbias, const float *sw5) {
   const size_t row0 = row - lane;
   float ysum = 0.0f;
   for (int c = c_begin; c < c_end; ++c) {
@@ -66,12 +70,6 @@ __device__ __forceinline__ float train_epilogue(const TrainArgs &a, size_t row, 
     }
     float v[32];
     tc::tmem_ld32(trow + (uint32_t)(c * 32), v);     // warp-wide: every lane executes it
-    if constexpr (MODE == DW) {
-      float *p = part + (size_t)n0 * kWidth;
-#pragma unroll
-      for (int j = 0; j < 32; ++j) p[(size_t)j * kWidth] = v[j];
-      continue;
-    }
     __align__(16) __nv_bfloat16 out[32];
     if constexpr (MODE == DX) {
 #pragma unroll
@@ -93,23 +91,23 @@ __device__ __forceinline__ float train_epilogue(const TrainArgs &a, size_t row, 
   return ysum;
 }
 
-// One CTA per SM, warp-specialised.  FWD*, DX: CTA c serves member slot
-// c % G, whose weight operand stays in shared memory for the launch, and takes
-// the slot's 128-row tiles round-robin.  DW: a tile is (slot, split of 256
-// rows, 128 output features), both operands through the ring.
+// A layer's products of the forward pass and of dX.  One CTA per SM,
+// warp-specialised: CTA c serves member slot c % G, whose weight operand stays
+// in shared memory for the launch, and takes the slot's 128-row tiles
+// round-robin.  Bound by its HBM traffic (X or dH and Z read, Z and X or dH
+// written: 126 MB for five members of 16,384 rows in 27-32 us; 16 epilogue warps
+// instead of 8 changed nothing).
 //   warp 0  (one lane)  TMA producer
 //   warp 1  (one lane)  MMA issuer: tcgen05.mma into one of two TMEM
 //           accumulators (2 x 256 columns)
 //   warps 2-9           epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31, two
 //           warps a quarter, each half of the columns; it overlaps the MMAs of
 //           the next tile
-// Shared memory: region 1 (128 KiB) the resident weights or the B stages of
-// DW, region 2 (64 KiB) the A stages.
+// Shared memory: region 1 (128 KiB) the resident weights, region 2 (64 KiB) the
+// row tiles.
 template <int MODE>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(kTrainThreads, 1)
     k_train_gemm(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const TrainArgs a) {
-  constexpr bool kResidentB = (MODE != DW);
-  constexpr uint32_t kBox = kChunk * 128;            // DW: a {64 columns, 64 rows} box
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(16) unsigned char s_stage[kEpiWarps][32 * kStagePitch];
   __shared__ float s_bias[kWidth], s_w5[kWidth];
@@ -118,24 +116,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   unsigned char *r1 = base;
   unsigned char *r2 = base + kRegion1;
   uint64_t *full = reinterpret_cast<uint64_t *>(r2 + kRegion2);
-  uint64_t *empty = full + kStages;
-  uint64_t *bfull = empty + kStages;
+  uint64_t *empty = full + kTrainStages;
+  uint64_t *bfull = empty + kTrainStages;
   uint64_t *accf = bfull + 1;
   uint64_t *acce = accf + 2;
   uint32_t *tslot = reinterpret_cast<uint32_t *>(acce + 2);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t bytesB = (uint32_t)a.N * kChunk * 2;
   // this CTA's tiles: first, first + step, ... < tiles
-  const int my_slot = kResidentB ? (int)blockIdx.x % a.G : 0;
-  const int first = kResidentB ? (int)blockIdx.x / a.G : (int)blockIdx.x;
-  const int step = kResidentB ? (int)gridDim.x / a.G : (int)gridDim.x;
-  const int per_slot = kResidentB ? a.rows / kTileM : (a.rows / kSplitRows) * 2;
-  const int tiles = kResidentB ? per_slot : per_slot * a.G;
+  const int slot = (int)blockIdx.x % a.G, first = (int)blockIdx.x / a.G, step = (int)gridDim.x / a.G;
+  const int tiles = a.rows / kTileM;
   const int nk = a.K / kChunk;
 
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < kTrainStages; ++s) {
       tc::mbar_init(&full[s], 1);
       tc::mbar_init(&empty[s], 1);
     }
@@ -149,7 +143,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     tc::tma_prefetch(&tmB);
   }
   if (MODE == FWD || MODE == FWD_LAST) {
-    const float *P = a.P[my_slot];
+    const float *P = a.P[slot];
     for (int i = tid; i < kWidth; i += blockDim.x) {
       s_bias[i] = P[a.off_bias + i];
       if (MODE == FWD_LAST) s_w5[i] = P[kOffW5 + i];
@@ -166,32 +160,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const unsigned long long deadline = tc::now_ns() + a.timeout_ns;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (lane == 0 && first < tiles) {
       uint32_t it = 0;
       bool ok = true;
-      if (kResidentB && first < tiles) {
-        tc::mbar_expect_tx(bfull, (uint32_t)nk * bytesB);
-        for (int c = 0; c < nk; ++c) tc::tma_load_3d(r1 + c * kStageB, &tmB, c * kChunk, 0, a.m0 + my_slot, bfull);
-      }
+      tc::mbar_expect_tx(bfull, (uint32_t)nk * kStageB);
+      for (int c = 0; c < nk; ++c) tc::tma_load_3d(r1 + c * kStageB, &tmB, c * kChunk, 0, a.m0 + slot, bfull);
       for (int t = first; t < tiles && ok; t += step) {
-        const int slot = kResidentB ? my_slot : t / per_slot;
-        const int local = kResidentB ? t : t % per_slot;
         for (int kc = 0; kc < nk; ++kc) {
-          const uint32_t st = it % kStages;
-          if (it >= (uint32_t)kStages && !tc::mbar_wait(&empty[st], ((it / kStages) - 1) & 1, deadline)) {
+          const uint32_t st = it % kTrainStages;
+          if (it >= (uint32_t)kTrainStages && !tc::mbar_wait(&empty[st], ((it / kTrainStages) - 1) & 1, deadline)) {
             ok = false;
             break;
           }
-          tc::mbar_expect_tx(&full[st], kStageA + (kResidentB ? 0u : bytesB));
-          if (kResidentB) {
-            tc::tma_load_3d(r2 + st * kStageA, &tmA, kc * kChunk, local * kTileM, slot, &full[st]);
-          } else {
-            const int row = (local >> 1) * kSplitRows + kc * kChunk, col = (local & 1) * kTileM;
-            for (int b = 0; b < kTileM / 64; ++b)
-              tc::tma_load_3d(r2 + st * kStageA + b * kBox, &tmA, col + b * 64, row, slot, &full[st]);
-            for (int b = 0; b < a.N / 64; ++b)
-              tc::tma_load_3d(r1 + st * kStageB + b * kBox, &tmB, b * 64, row, slot, &full[st]);
-          }
+          tc::mbar_expect_tx(&full[st], kStageA);
+          tc::tma_load_3d(r2 + st * kStageA, &tmA, kc * kChunk, t * kTileM, slot, &full[st]);
           ++it;
         }
       }
@@ -199,16 +181,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         atomicExch(a.error, 1u);
         // copies in flight land before the shared memory is given back
         const unsigned long long d2 = tc::now_ns() + 1000000000ull;
-        for (uint32_t j = (it > (uint32_t)kStages ? it - kStages : 0u); j < it; ++j)
-          tc::mbar_wait(&full[j % kStages], (j / kStages) & 1, d2);
-        if (kResidentB) tc::mbar_wait(bfull, 0, d2);
+        for (uint32_t j = (it > (uint32_t)kTrainStages ? it - kTrainStages : 0u); j < it; ++j)
+          tc::mbar_wait(&full[j % kTrainStages], (j / kTrainStages) & 1, d2);
+        tc::mbar_wait(bfull, 0, d2);
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && first < tiles) {
-      const uint32_t idesc = tc::idesc_bf16_f32(kTileM, a.N) | (kResidentB ? 0u : tc::kIdescMnMajorAB);
+      const uint32_t idesc = tc::idesc_bf16_f32(kTileM, kWidth);
       uint32_t it = 0, local = 0;
-      bool ok = !kResidentB || tc::mbar_wait(bfull, 0, deadline);
+      bool ok = tc::mbar_wait(bfull, 0, deadline);
       for (int t = first; t < tiles && ok; t += step) {
         const uint32_t buf = local & 1u;
         if (local >= 2 && !tc::mbar_wait(&acce[buf], ((local >> 1) - 1) & 1, deadline)) {
@@ -218,23 +200,18 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         tc::tc_fence_after();
         const uint32_t d = tmem + buf * kTmemCols;
         for (int kc = 0; kc < nk; ++kc) {
-          const uint32_t st = it % kStages;
-          if (!tc::mbar_wait(&full[st], (it / kStages) & 1, deadline)) {
+          const uint32_t st = it % kTrainStages;
+          if (!tc::mbar_wait(&full[st], (it / kTrainStages) & 1, deadline)) {
             ok = false;
             break;
           }
           tc::tc_fence_after();
           const uint32_t aa = tc::smem_u32(r2 + st * kStageA);
-          const uint32_t bb = tc::smem_u32(r1 + (kResidentB ? (uint32_t)kc : st) * kStageB);
+          const uint32_t bb = tc::smem_u32(r1 + kc * kStageB);
 #pragma unroll
-          for (int k = 0; k < kChunk / 16; ++k) {
-            const uint32_t acc = (kc > 0 || k > 0) ? 1u : 0u;
-            if (kResidentB)
-              tc::mma_bf16(d, tc::sdesc_sw128(aa + k * 32), tc::sdesc_sw128(bb + k * 32), idesc, acc);
-            else                                     // 16 rows of 128 bytes further
-              tc::mma_bf16(d, tc::sdesc_sw128_mn(aa + k * 2048, kBox), tc::sdesc_sw128_mn(bb + k * 2048, kBox), idesc,
-                           acc);
-          }
+          for (int k = 0; k < kChunk / 16; ++k)
+            tc::mma_bf16(d, tc::sdesc_sw128(aa + k * 32), tc::sdesc_sw128(bb + k * 32), idesc,
+                         (kc > 0 || k > 0) ? 1u : 0u);
           tc::mma_commit(&empty[st]);
           ++it;
         }
@@ -246,17 +223,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         atomicExch(a.error, 2u);
         // products in flight finish before TMEM is given back
         const unsigned long long d2 = tc::now_ns() + 1000000000ull;
-        if (it > 0) tc::mbar_wait(&empty[(it - 1) % kStages], ((it - 1) / kStages) & 1, d2);
+        if (it > 0) tc::mbar_wait(&empty[(it - 1) % kTrainStages], ((it - 1) / kTrainStages) & 1, d2);
       }
     }
   } else {
     const int q = warp & 3;                       // TMEM lane quarter of this warp
     const int h = (warp - 2) / 4;                 // column half of this warp
-    const int per = (a.N / 32) / 2;
+    constexpr int per = (kWidth / 32) / 2;
     uint32_t count = 0;
     for (int t = first; t < tiles; t += step) {
-      const int slot = kResidentB ? my_slot : t / per_slot;
-      const int local = kResidentB ? t : t % per_slot;
       const uint32_t buf = count & 1u;
       const bool got = tc::mbar_wait(&accf[buf], (count >> 1) & 1, deadline);
       if (!__all_sync(0xffffffffu, got)) {
@@ -264,12 +239,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         break;
       }
       tc::tc_fence_after();
-      const int r = q * 32 + lane;
-      const size_t row = (size_t)slot * a.rows + (size_t)local * kTileM + r;
-      float *part = nullptr;
-      if constexpr (MODE == DW)
-        part = a.partial + ((size_t)slot * (per_slot / 2) + (local >> 1)) * a.N * kWidth + (local & 1) * kTileM + r;
-      const float ys = train_epilogue<MODE>(a, row, tmem + ((uint32_t)(q * 32) << 16) + buf * kTmemCols, part, h * per,
+      const size_t row = (size_t)slot * a.rows + (size_t)t * kTileM + q * 32 + lane;
+      const float ys = train_epilogue<MODE>(a, row, tmem + ((uint32_t)(q * 32) << 16) + buf * kTmemCols, h * per,
                                             (h + 1) * per, s_stage[warp - 2], lane, s_bias, s_w5);
       tc::tc_fence_before();
       __syncwarp();
@@ -278,7 +249,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         // y_out is zeroed before the launch; the two halves' sums meet by
         // atomic addition, (0 + x) + y == (0 + y) + x, so the order does not
         // change the result
-        atomicAdd(&a.y_out[row], h == 0 ? ys + __ldg(a.P[my_slot] + kOffB5) : ys);
+        atomicAdd(&a.y_out[row], h == 0 ? ys + __ldg(a.P[slot] + kOffB5) : ys);
       }
       ++count;
     }
@@ -287,6 +258,262 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   if (warp == 1) {
     tc::tc_fence_after();
     tc::tmem_dealloc(tmem, 2 * kTmemCols);
+  }
+}
+
+struct UpdateArgs {
+  float *P[kMaxMembers], *M1[kMaxMembers], *M2[kMaxMembers];
+  float lr[kMaxMembers], c1[kMaxMembers], c2[kMaxMembers];   // Adam: rate and bias corrections by slot
+  float b1, b2, eps;
+  float *grad;              // non-null: write the gradient (slot 0) and leave the parameters
+  int rows, G, m0;
+  __nv_bfloat16 *w[4];      // BF16 operand copies of the layers, by member: [E][256][64 or 256]
+  __nv_bfloat16 *wt[4];     // transposed [E][256][256], null for the first layer
+  float *epi;               // FP32 epilogue operands of inference [E][5][256]
+  const float *cls;         // class sums [G][5][256][256]: dH_1 .. dH_4, X4 dy
+  const float *dy;          // [G][rows]
+  const float *loss_part;   // [G][rows / 128]
+  float *loss;              // loss[slot * loss_stride]
+  long long loss_stride;
+  unsigned *error;
+  unsigned long long timeout_ns;
+};
+
+__device__ __forceinline__ int layer_weights(int li) {
+  return li == 0 ? kOffW1 : li == 1 ? kOffW2 : li == 2 ? kOffW3 : kOffW4;
+}
+__device__ __forceinline__ int layer_bias(int li) {
+  return li == 0 ? kOffB1 : li == 1 ? kOffB2 : li == 2 ? kOffB3 : kOffB4;
+}
+
+// Adam (bias-corrected) on one FP32 master parameter; returns its new value.
+__device__ __forceinline__ float adam(const UpdateArgs &u, int slot, int i, float gi) {
+  float *p = u.P[slot], *m1 = u.M1[slot], *m2 = u.M2[slot];
+  const float a = fmaf(1.0f - u.b1, gi, __fmul_rn(u.b1, m1[i]));
+  const float b = fmaf(__fmul_rn(1.0f - u.b2, gi), gi, __fmul_rn(u.b2, m2[i]));
+  m1[i] = a;
+  m2[i] = b;
+  const float v = p[i] - u.lr[slot] * (a / u.c1[slot]) / (sqrtf(b / u.c2[slot]) + u.eps);
+  p[i] = v;
+  return v;
+}
+
+// ----------------------------------------------------------------------------
+// Weight gradients of all four layers and the optimiser's step, one launch.
+//
+// A work item is a tile of one layer's dW: 128 output features x N inputs (N =
+// 64 or 128; the first layer's 64 padded inputs are one tile), reduced over the
+// whole batch: dH_l^T X_{l-1}, both operands row-major in HBM and read MN-major.
+// The tensor core forms one partial per 256 rows in one of four TMEM
+// accumulators, the epilogue adds each to its FP32 registers, in order, and
+// at the end takes the parameters' step: no partial goes through HBM (they were
+// 335 MB a step for five members, written and read back), and the gradient is
+// stored only where it is asked for.
+//   warp 0  (one lane)  TMA producer: per 64 batch rows the boxes of both operands
+//   warp 1  (one lane)  MMA issuer
+//   warps 2-9           epilogue: warp w TMEM lanes 32 (w % 4) .. +31 (output
+//           features), half (w - 2) / 4 of the tile's columns
+// Bound by the operands' way from L2 (6 MB an item at N = 64, 130 items for five
+// members of 16,384 rows: 128 us, 6 TB/s; through partials in HBM and an update
+// kernel of their own, 250 us).  With many members N = 128 halves the items.
+// ----------------------------------------------------------------------------
+constexpr int kDwStages = 6;
+constexpr uint32_t kDwBox = kChunk * 128;               // 8 KiB: 64 columns of 64 rows
+constexpr uint32_t kDwStage = 4 * kDwBox;               // 128 features, up to 128 inputs
+constexpr int kDwBuffers = 4;
+constexpr int kDwCols = 128;
+constexpr size_t kDwSmem = 1024 + (size_t)kDwStages * kDwStage + 256;
+
+struct DwMaps {
+  CUtensorMap dh[4], x[4];          // boxes of {64 columns, 64 rows, 1 slot}
+};
+
+__global__ void __launch_bounds__(kTrainThreads, 1)
+    k_train_dw(const __grid_constant__ DwMaps maps, const UpdateArgs u, const int n_tile) {
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t s0 = tc::smem_u32(smem_raw);
+  unsigned char *base = smem_raw + ((1024u - (s0 & 1023u)) & 1023u);
+  uint64_t *full = reinterpret_cast<uint64_t *>(base + kDwStages * kDwStage);
+  uint64_t *empty = full + kDwStages;
+  uint64_t *accf = empty + kDwStages;
+  uint64_t *acce = accf + kDwBuffers;
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(acce + kDwBuffers);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n_tiles = kWidth / n_tile;                  // of layers 2 to 4
+  const int big = u.G * 3 * 2 * n_tiles, items = big + u.G * 2;
+  const int chunks = u.rows / kChunk, parts = u.rows / kSplitRows;
+  constexpr int kPart = kSplitRows / kChunk;            // chunks of a partial
+
+  if (tid == 0) {
+    for (int s = 0; s < kDwStages; ++s) {
+      tc::mbar_init(&full[s], 1);
+      tc::mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < kDwBuffers; ++b) {
+      tc::mbar_init(&accf[b], 1);
+      tc::mbar_init(&acce[b], kEpiWarps);
+    }
+    tc::fence_mbar_init();
+  }
+  if (warp == 1) {
+    tc::tmem_alloc(tslot, kDwBuffers * kDwCols);
+    tc::tmem_relinquish();
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = *tslot;
+  const unsigned long long deadline = tc::now_ns() + u.timeout_ns;
+  // item -> layer, slot, features' half, first input, inputs
+  struct Item {
+    int li, slot, m, n0, N;
+  };
+  auto item = [&](int w) {
+    Item t;
+    if (w < big) {
+      const int r = w / n_tiles;
+      t.n0 = (w % n_tiles) * n_tile;
+      t.N = n_tile;
+      t.m = r & 1;
+      t.li = 1 + (r >> 1) % 3;
+      t.slot = (r >> 1) / 3;
+    } else {
+      t.n0 = 0;
+      t.N = kInPad;
+      t.m = (w - big) & 1;
+      t.li = 0;
+      t.slot = (w - big) >> 1;
+    }
+    return t;
+  };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        const Item t = item(w);
+        const uint32_t bytes = 2 * kDwBox + (uint32_t)(t.N / 64) * kDwBox;
+        for (int c = 0; c < chunks; ++c) {
+          const uint32_t st = it % kDwStages;
+          if (it >= (uint32_t)kDwStages && !tc::mbar_wait(&empty[st], ((it / kDwStages) - 1) & 1, deadline)) {
+            ok = false;
+            break;
+          }
+          unsigned char *d = base + st * kDwStage;
+          tc::mbar_expect_tx(&full[st], bytes);
+          for (int b = 0; b < 2; ++b)
+            tc::tma_load_3d(d + b * kDwBox, &maps.dh[t.li], t.m * kTileM + b * 64, c * kChunk, t.slot, &full[st]);
+          for (int b = 0; b < t.N / 64; ++b)
+            tc::tma_load_3d(d + (2 + b) * kDwBox, &maps.x[t.li], t.n0 + b * 64, c * kChunk, t.slot, &full[st]);
+          ++it;
+        }
+      }
+      if (!ok) {
+        atomicExch(u.error, 4u);
+        // copies in flight land before the shared memory is given back
+        const unsigned long long d2 = tc::now_ns() + 1000000000ull;
+        for (uint32_t j = (it > (uint32_t)kDwStages ? it - kDwStages : 0u); j < it; ++j)
+          tc::mbar_wait(&full[j % kDwStages], (j / kDwStages) & 1, d2);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      uint32_t it = 0, count = 0;                       // chunks; partials
+      bool ok = true;
+      for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+        const Item t = item(w);
+        const uint32_t idesc = tc::idesc_bf16_f32(kTileM, t.N) | tc::kIdescMnMajorAB;
+        for (int p = 0; p < parts && ok; ++p, ++count) {
+          const uint32_t buf = count % kDwBuffers;
+          if (count >= (uint32_t)kDwBuffers && !tc::mbar_wait(&acce[buf], ((count / kDwBuffers) - 1) & 1, deadline)) {
+            ok = false;
+            break;
+          }
+          for (int kc = 0; kc < kPart; ++kc) {
+            const uint32_t st = it % kDwStages;
+            if (!tc::mbar_wait(&full[st], (it / kDwStages) & 1, deadline)) {
+              ok = false;
+              break;
+            }
+            tc::tc_fence_after();
+            const uint32_t aa = tc::smem_u32(base + st * kDwStage), bb = aa + 2 * kDwBox;
+#pragma unroll
+            for (int k = 0; k < kChunk / 16; ++k)        // 16 rows of 128 bytes further
+              tc::mma_bf16(tmem + buf * kDwCols, tc::sdesc_sw128_mn(aa + k * 2048, kDwBox),
+                           tc::sdesc_sw128_mn(bb + k * 2048, kDwBox), idesc, (kc > 0 || k > 0) ? 1u : 0u);
+            tc::mma_commit(&empty[st]);
+            ++it;
+          }
+          if (!ok) break;
+          tc::mma_commit(&accf[buf]);
+        }
+      }
+      if (!ok) {
+        atomicExch(u.error, 5u);
+        // products in flight finish before TMEM is given back
+        if (it > 0) tc::mbar_wait(&empty[(it - 1) % kDwStages], ((it - 1) / kDwStages) & 1, tc::now_ns() + 1000000000ull);
+      }
+    }
+  } else {
+    const int q = warp & 3;                       // TMEM lane quarter of this warp
+    const int h = (warp - 2) / 4;                 // column half of this warp
+    uint32_t count = 0;
+    bool ok = true;
+    for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
+      const Item t = item(w);
+      const int mine = t.N / 2;                   // columns of this warp: 64 or 32
+      const uint32_t tcol = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(h * mine);
+      float s[64];
+#pragma unroll
+      for (int j = 0; j < 64; ++j) s[j] = 0.0f;
+      for (int p = 0; p < parts; ++p, ++count) {
+        const uint32_t buf = count % kDwBuffers;
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&accf[buf], (count / kDwBuffers) & 1, deadline));
+        if (!ok) break;
+        tc::tc_fence_after();
+        float v[32];
+        tc::tmem_ld32(tcol + buf * kDwCols, v);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) s[j] += v[j];
+        if (mine == 64) {
+          tc::tmem_ld32(tcol + buf * kDwCols + 32, v);
+#pragma unroll
+          for (int j = 0; j < 32; ++j) s[32 + j] += v[j];
+        }
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&acce[buf]);
+      }
+      if (!ok) {
+        if (lane == 0) atomicExch(u.error, 6u);
+        break;
+      }
+      // output feature o, inputs i0 .. i0 + mine - 1
+      const int o = t.m * kTileM + q * 32 + lane, i0 = t.n0 + h * mine;
+      const int fan_in = t.li == 0 ? kFeatures : kWidth, ld = t.li == 0 ? kInPad : kWidth;
+      const int off = layer_weights(t.li) + o * fan_in;
+      __nv_bfloat16 *wr = u.w[t.li] + ((size_t)(u.m0 + t.slot) * kWidth + o) * ld;
+      __nv_bfloat16 *wc = u.wt[t.li] ? u.wt[t.li] + (size_t)(u.m0 + t.slot) * kWidth * kWidth + o : nullptr;
+#pragma unroll
+      for (int j = 0; j < 64; ++j) {
+        const int i = i0 + j;
+        if (j < mine && i < fan_in) {
+          if (u.grad) {
+            u.grad[off + i] = s[j];
+          } else {
+            const __nv_bfloat16 b = __float2bfloat16_rn(adam(u, t.slot, off + i, s[j]));
+            wr[i] = b;
+            if (wc) wc[(size_t)i * kWidth] = b;
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc(tmem, kDwBuffers * kDwCols);
   }
 }
 
@@ -358,145 +585,63 @@ __global__ void __launch_bounds__(256) k_head_backward(const float *__restrict__
   }
 }
 
-// Class sums of the bias and head gradients: out[slot][t][f] = sum over the
-// rows c = t, t + 256, ... of src[c][f] (* w[c]), in that order.  A block takes
-// 32 classes x 64 columns, a thread 8 columns of a class (16-byte loads, four
-// rows of 128 bytes a warp).  HBM-bound; read from transposed copies by one
-// block a column it took 32 us a layer and member.
-__global__ void __launch_bounds__(256) k_class_sums(const __nv_bfloat16 *__restrict__ src, const float *__restrict__ w,
-                                                    int rows, float *__restrict__ out) {
-  const int f0 = blockIdx.y * 64 + (threadIdx.x & 7) * 8;
-  const int t = blockIdx.x * 32 + (threadIdx.x >> 3);
-  const size_t base = (size_t)blockIdx.z * rows;
-  float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
+// Class sums of the bias and head gradients: source k of slot g, its sums over
+// the rows c = t, t + 256, ..., in that order, to out[g][k][t][f]: k = 0..3 dH_1
+// .. dH_4, k = 4 X4 weighted by dy.  A block takes 16 classes x 64 columns of one
+// source, a thread 4 columns of a class (8-byte loads, two rows of 128 bytes a
+// warp, 16 rows in flight).  HBM-bound; it runs beside the weight gradients.
+// Read from transposed copies by one block a column it took 32 us a source and
+// member.
+constexpr int kClassBlock = 16;
+struct ClassSources {
+  const __nv_bfloat16 *src[5];
+  const float *dy;
+};
+__global__ void __launch_bounds__(256) k_class_sums(const ClassSources a, int rows, float *__restrict__ out) {
+  const int k = blockIdx.z % 5, slot = blockIdx.z / 5;
+  const int f0 = blockIdx.y * 64 + (threadIdx.x & 15) * 4;
+  const int t = blockIdx.x * kClassBlock + (threadIdx.x >> 4);
+  const size_t base = (size_t)slot * rows;
+  const __nv_bfloat16 *src = a.src[k];
+  const float *w = (k == 4) ? a.dy : nullptr;
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 16
   for (int c = t; c < rows; c += kClasses) {
-    const uint4 v = *reinterpret_cast<const uint4 *>(src + (base + c) * kWidth + f0);
+    const uint2 v = *reinterpret_cast<const uint2 *>(src + (base + c) * kWidth + f0);
     const __nv_bfloat16 *x = reinterpret_cast<const __nv_bfloat16 *>(&v);
     const float wc = w ? w[base + c] : 1.0f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s[j] = fmaf(__bfloat162float(x[j]), wc, s[j]);
+    for (int j = 0; j < 4; ++j) s[j] = fmaf(__bfloat162float(x[j]), wc, s[j]);
   }
-  float4 *o = reinterpret_cast<float4 *>(out + ((size_t)blockIdx.z * kClasses + t) * kWidth + f0);
-  o[0] = make_float4(s[0], s[1], s[2], s[3]);
-  o[1] = make_float4(s[4], s[5], s[6], s[7]);
+  *reinterpret_cast<float4 *>(out + ((size_t)blockIdx.z * kClasses + t) * kWidth + f0) =
+      make_float4(s[0], s[1], s[2], s[3]);
 }
 
-struct UpdateArgs {
-  float *P[kMaxMembers], *M1[kMaxMembers], *M2[kMaxMembers];
-  float lr[kMaxMembers], c1[kMaxMembers], c2[kMaxMembers];   // Adam: rate and bias corrections by slot
-  float b1, b2, eps;
-  float *grad;              // non-null: write the gradient (slot 0) and leave the parameters
-  int rows, splits, N, fan_in, off_w, off_b;
-  const float *partial;     // [G][splits][N][256]
-  const float *cls;         // class sums of dH_l [G][256][256]
-  const float *cls5;        // top layer: of X4 dy (head weights), else null
-  const float *dy;          // top layer: [G][rows] (head bias)
-  const float *loss_part;   // top layer: [G][rows / 128]
-  float *loss;              // top layer: loss[slot * loss_stride]
-  long long loss_stride;
-  int m0;
-  __nv_bfloat16 *w;         // BF16 operand copies of the layer, by member: [E][256][w_ld]
-  __nv_bfloat16 *wt;        // transposed [E][256][256], null for the first layer
-  int w_ld;
-  float *epi;               // FP32 epilogue operands of inference [E][5][256]
-  int epi_layer;            // this layer's row of it
-};
-
-// Adam (bias-corrected) on one FP32 master parameter; returns its new value.
-__device__ __forceinline__ float adam(const UpdateArgs &u, int slot, int i, float gi) {
-  float *p = u.P[slot], *m1 = u.M1[slot], *m2 = u.M2[slot];
-  const float a = fmaf(1.0f - u.b1, gi, __fmul_rn(u.b1, m1[i]));
-  const float b = fmaf(__fmul_rn(1.0f - u.b2, gi), gi, __fmul_rn(u.b2, m2[i]));
-  m1[i] = a;
-  m2[i] = b;
-  const float v = p[i] - u.lr[slot] * (a / u.c1[slot]) / (sqrtf(b / u.c2[slot]) + u.eps);
-  p[i] = v;
-  return v;
-}
-
-// red[0..255][0..31] -> red[0][c] by the fixed tree (t += t + s, s = 128 .. 1).
-__device__ __forceinline__ void class_tree(float (*red)[33], int tid) {
-  for (int s = kClasses / 2; s > 0; s >>= 1) {
-    for (int i = tid; i < s * 32; i += 256) red[i >> 5][i & 31] += red[(i >> 5) + s][i & 31];
-    __syncthreads();
-  }
-}
-
-// The gradient of one layer from its partials, the optimiser's step and the
-// BF16 operand copies, in one pass: the gradient is not stored, the
-// parameters are read and written once.  Blocks [0, tiles): 32 x 32 tiles of
-// dW (o the contiguous axis of the partials, i that of the parameters: the
-// tile turns in shared memory); then 8 blocks of 32 biases; for the top layer 8
-// of 32 head weights and one of the head bias and the loss.
-__global__ void __launch_bounds__(256) k_update(const UpdateArgs u) {
+// Biases, head weights, head bias and loss from their class sums, by a fixed
+// tree (t += t + s, s = 128 .. 1), and the optimiser's step: blocks 0..39 take
+// 32 columns of a source, block 40 the head bias and the loss.
+__global__ void __launch_bounds__(256) k_update_biases(const UpdateArgs u) {
   __shared__ float red[kClasses][33];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, slot = blockIdx.y;
-  const int i_tiles = (u.fan_in + 31) / 32;
-  const int tiles = 8 * i_tiles;
-  int b = blockIdx.x;
-  if (b < tiles) {
-    const int o0 = (b / i_tiles) * 32, i0 = (b % i_tiles) * 32;
-    const float *part = u.partial + (size_t)slot * u.splits * u.N * kWidth + o0 + lane;
-    float s[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll 8
-    for (int k = 0; k < u.splits; ++k) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int i = i0 + warp + 8 * j;
-        if (i < u.fan_in) s[j] += part[((size_t)k * u.N + i) * kWidth];
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 4; ++j) red[warp + 8 * j][lane] = s[j];       // [i][o]
-    __syncthreads();
-    const int i = i0 + lane;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int o = warp + 8 * j;
-      if (i < u.fan_in) {
-        const int idx = u.off_w + (o0 + o) * u.fan_in + i;
-        const float gi = red[lane][o];
-        if (u.grad) {
-          u.grad[idx] = gi;
-        } else {
-          const float v = adam(u, slot, idx, gi);
-          u.w[((size_t)(u.m0 + slot) * kWidth + o0 + o) * u.w_ld + i] = __float2bfloat16_rn(v);
-          red[lane][o] = v;
-        }
-      }
-    }
-    if (u.wt && !u.grad) {
-      __syncthreads();
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int ii = warp + 8 * j;
-        u.wt[((size_t)(u.m0 + slot) * kWidth + i0 + ii) * kWidth + o0 + lane] = __float2bfloat16_rn(red[ii][lane]);
-      }
-    }
-    return;
-  }
-  b -= tiles;
-  if (b < 16) {
-    const float *src = (b < 8) ? u.cls : u.cls5;
-    const int f0 = (b & 7) * 32, off = (b < 8) ? u.off_b : kOffW5;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, slot = blockIdx.y, b = blockIdx.x;
+  if (b < 40) {
+    const int k = b >> 3, f0 = (b & 7) * 32, off = (k < 4) ? layer_bias(k) : kOffW5;
     for (int t = warp; t < kClasses; t += 8)
-      red[t][lane] = src[((size_t)slot * kClasses + t) * kWidth + f0 + lane];
+      red[t][lane] = u.cls[(((size_t)slot * 5 + k) * kClasses + t) * kWidth + f0 + lane];
     __syncthreads();
-    class_tree(red, tid);
+    for (int s = kClasses / 2; s > 0; s >>= 1) {
+      for (int i = tid; i < s * 32; i += 256) red[i >> 5][i & 31] += red[(i >> 5) + s][i & 31];
+      __syncthreads();
+    }
     if (tid < 32) {
       if (u.grad) {
         u.grad[off + f0 + lane] = red[0][lane];
       } else {
         const float v = adam(u, slot, off + f0 + lane, red[0][lane]);
-        float *epi = u.epi + (size_t)(u.m0 + slot) * kEpiFloats + f0 + lane;
-        if (b < 8) epi[u.epi_layer * kWidth] = 0.5f * v;
-        else epi[4 * kWidth] = v;
+        u.epi[(size_t)(u.m0 + slot) * kEpiFloats + k * kWidth + f0 + lane] = (k < 4) ? 0.5f * v : v;
       }
     }
     return;
   }
-  // head bias and loss: class sums of dy and of the loss partials, same tree
   float *s0 = &red[0][0], *s1 = s0 + kClasses;
   float a0 = 0.f, a1 = 0.f;
   const float *dy = u.dy + (size_t)slot * u.rows;
