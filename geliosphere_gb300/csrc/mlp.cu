@@ -383,6 +383,23 @@ int train_step(gelio_surrogate *s, int m0, int G, int n_valid, UpdateArgs &u) {
   return GELIO_OK;
 }
 
+// A launch whose CTAs may start while the kernel before it on the stream still
+// runs; the kernel itself waits for it (wait_for_previous_kernel).
+template <class... P, class... A>
+cudaError_t launch_early(gelio_surrogate *s, void (*kernel)(P...), unsigned grid, unsigned block, size_t smem, A... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s->stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Members [m0, m1) on the first c rows of the inference batch (s->Q0, zero
 // past c up to a whole tile) in one launch of the fused network kernel; member
 // m0 + e's outputs are added to y[e * stride + row].
@@ -406,8 +423,7 @@ int infer_fused(gelio_surrogate *s, int m0, int m1, int c, float *y, long long s
   a.error = s->error;
   a.timeout_ns = 2000000000ull;
   const int grid = std::max(1, std::min(E * a.n_pairs, s->sm_count));
-  k_mlp_infer_fused<<<grid, kFusedThreads, kFusedSmem, s->stream>>>(maps, a);
-  return cuda_status(cudaGetLastError());
+  return cuda_status(launch_early(s, k_mlp_infer_fused, grid, kFusedThreads, kFusedSmem, maps, a));
 }
 
 // FLOP of the products over the rows actually multiplied (whole tiles of 128
@@ -856,10 +872,9 @@ int infer_sims(gelio_surrogate *s, const gelio_sim_params *sims, int n, size_t r
     SUR_TRY(cudaGetLastError());
     if ((rc = infer_fused(s, 0, E, c, s->d_py + off, (long long)stride)) != GELIO_OK) return rc;
   }
-  k_ensemble<<<(unsigned)((rows + 127) / 128), 128, 0, s->stream>>>(
-      s->d_py, E, (long long)rows, (long long)stride, s->d_pstat, s->d_pstat + rows, s->error,
-      reinterpret_cast<unsigned *>(s->d_pstat + 2 * rows));
-  SUR_TRY(cudaGetLastError());
+  SUR_TRY(launch_early(s, k_ensemble, (unsigned)((rows + 127) / 128), 128, 0, (const float *)s->d_py, E, (long long)rows,
+                       (long long)stride, s->d_pstat, s->d_pstat + rows, (const unsigned *)s->error,
+                       reinterpret_cast<unsigned *>(s->d_pstat + 2 * rows)));
   SUR_TRY(cudaEventRecord(s->ev1, s->stream));
   const size_t bytes = rows * sizeof(double);
   if (staged) {
