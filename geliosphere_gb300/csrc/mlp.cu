@@ -10,6 +10,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <random>
@@ -151,7 +152,8 @@ struct gelio_surrogate {
   int *ident = nullptr;      // 0, 1, ..., rows - 1
   int *order = nullptr;      // this epoch's shuffled row orders, [group][rows of the set]
   size_t order_cap = 0;
-  int *h_order = nullptr;    // pinned staging of two epochs' orders
+  int *h_order = nullptr;    // staging of two epochs' orders
+  bool h_order_pinned = false;
   size_t h_order_cap = 0;
   cudaEvent_t ev_copy[2] = {nullptr, nullptr};   // an epoch's orders have left the staging
   unsigned *error = nullptr;
@@ -226,6 +228,12 @@ void free_train(TrainBuffers &t) {
   t = TrainBuffers();
 }
 
+void free_orders(gelio_surrogate *s) {
+  if (s->h_order) s->h_order_pinned ? (void)cudaFreeHost(s->h_order) : std::free(s->h_order);
+  s->h_order = nullptr;
+  s->h_order_cap = 0;
+}
+
 void free_all(gelio_surrogate *s) {
   auto f = [](void *p) { if (p) cudaFree(p); };
   for (auto &m : s->mem) { f(m.P); f(m.M1); f(m.M2); }
@@ -237,7 +245,7 @@ void free_all(gelio_surrogate *s) {
   f(s->Q0); f(s->epi);
   f(s->d_pup); f(s->d_py); f(s->d_pstat);
   if (s->h_pstage) cudaFreeHost(s->h_pstage);
-  if (s->h_order) cudaFreeHost(s->h_order);
+  free_orders(s);
   for (auto &e : s->ev_copy) if (e) cudaEventDestroy(e);
   if (s->ev0) cudaEventDestroy(s->ev0);
   if (s->ev1) cudaEventDestroy(s->ev1);
@@ -312,6 +320,39 @@ int ensure_train(gelio_surrogate *s, int G) {
   if (s->tb.G) SUR_TRY(cudaStreamSynchronize(s->stream));
   free_train(s->tb);
   s->tb = t;
+  return GELIO_OK;
+}
+
+// All that a group of G members needs to train on nrow rows.  The staging of
+// the orders is plain memory where no pinned memory is to be had.
+int ensure_group(gelio_surrogate *s, int G, int steps, size_t nrow) {
+  const int rc = ensure_train(s, G);
+  if (rc != GELIO_OK) return rc;
+  const size_t n_loss = (size_t)G * steps, n_order = G * nrow;
+  if (n_loss > s->step_loss_cap) {
+    if (s->step_loss) cudaFree(s->step_loss);
+    s->step_loss = nullptr;
+    s->step_loss_cap = 0;
+    SUR_TRY(gelio::dev_malloc(&s->step_loss, sizeof(float) * n_loss));
+    s->step_loss_cap = n_loss;
+  }
+  if (n_order > s->order_cap) {
+    if (s->order) cudaFree(s->order);
+    s->order = nullptr;
+    s->order_cap = 0;
+    SUR_TRY(gelio::dev_malloc(&s->order, n_order * sizeof(int)));
+    s->order_cap = n_order;
+  }
+  if (2 * n_order > s->h_order_cap) {
+    free_orders(s);
+    s->h_order_pinned = gelio::pinned_malloc(&s->h_order, 2 * n_order * sizeof(int)) == cudaSuccess;
+    if (!s->h_order_pinned) {
+      (void)cudaGetLastError();
+      s->h_order = static_cast<int *>(std::malloc(2 * n_order * sizeof(int)));
+      if (!s->h_order) return GELIO_ERR_OUT_OF_MEMORY;
+    }
+    s->h_order_cap = 2 * n_order;
+  }
   return GELIO_OK;
 }
 
@@ -765,30 +806,14 @@ int32_t gelio_surrogate_train(gelio_surrogate *s, int32_t epochs, float *last_lo
   }
   const int R = s->rows;
   const int steps = (int)std::max<size_t>(1, nrow / (size_t)R);
-  const int E = (int)s->mem.size(), G = group_size(s);
-  int rc = ensure_train(s, G);
+  // as large a group as the device has memory for
+  const int E = (int)s->mem.size();
+  int G = group_size(s), rc;
+  while ((rc = ensure_group(s, G, steps, nrow)) == GELIO_ERR_OUT_OF_MEMORY && G > 1) {
+    (void)cudaGetLastError();
+    G = (G + 1) / 2;
+  }
   if (rc != GELIO_OK) return rc;
-  if ((size_t)G * steps > s->step_loss_cap) {
-    if (s->step_loss) cudaFree(s->step_loss);
-    s->step_loss = nullptr;
-    s->step_loss_cap = 0;
-    SUR_TRY(gelio::dev_malloc(&s->step_loss, sizeof(float) * G * steps));
-    s->step_loss_cap = (size_t)G * steps;
-  }
-  if (G * nrow > s->order_cap) {
-    if (s->order) cudaFree(s->order);
-    s->order = nullptr;
-    s->order_cap = 0;
-    SUR_TRY(gelio::dev_malloc(&s->order, G * nrow * sizeof(int)));
-    s->order_cap = G * nrow;
-  }
-  if (2 * G * nrow > s->h_order_cap) {
-    if (s->h_order) cudaFreeHost(s->h_order);
-    s->h_order = nullptr;
-    s->h_order_cap = 0;
-    SUR_TRY(gelio::pinned_malloc(&s->h_order, 2 * G * nrow * sizeof(int)));
-    s->h_order_cap = 2 * G * nrow;
-  }
   const long long total = (long long)epochs * steps;
   std::vector<float> sl((size_t)G * steps);
   for (int m0 = 0; m0 < E; m0 += G) {

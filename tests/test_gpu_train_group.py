@@ -45,3 +45,34 @@ def test_gradient_at_small_batches(engine, oracle, batch, n):
         m = int(np.prod(shape))
         a, b = g[off:off + m].astype(np.float64), g_o[off:off + m]
         assert np.linalg.norm(a - b) < 1e-2 * max(np.linalg.norm(b), 1e-30), k
+
+
+@pytest.mark.parametrize("largest", [2 * 4096 * 256 * 2 - 1, 5 * 4096 * 256 * 2 - 1])
+def test_training_where_the_whole_group_does_not_fit(engine, largest):
+    """Allocations above `largest` (less than two members' activations of a
+    4096-row batch, or than five's) and all pinned memory refused: smaller groups
+    train, the same bits."""
+    x, t = data(9000, seed=9)
+    out = []
+    for refuse in (False, True):
+        s = sg.Surrogate(engine, members=6, batch_rows=4096, seed=4)
+        s.add_rows(x, t)
+        refused = []
+
+        def hook(kind, nbytes, user):
+            no = kind == abi.GELIO_ALLOC_PINNED_HOST or nbytes > largest
+            refused.append(no)
+            return int(no)
+
+        fn = abi.ALLOC_HOOK(hook)
+        if refuse:
+            assert engine.lib.gelio_set_alloc_hook(fn, None) == abi.GELIO_OK
+        try:
+            loss = s.train(2)
+        finally:
+            engine.lib.gelio_set_alloc_hook(abi.ALLOC_HOOK(), None)
+        assert any(refused) == refuse
+        out.append([loss] + [s.get_params(m) for m in range(6)])
+        s.close()
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
