@@ -389,9 +389,29 @@ int train_step(gelio_surrogate *s, int m0, int G, int n_valid, UpdateArgs &u) {
   k_head_backward<<<dim3(R / kHeadRows, G), 256, 0, s->stream>>>(t.yhat, t.y, n_valid, R, a, t.Z[3], t.dH[3], t.dy,
                                                                  t.loss_part);
   SUR_TRY(cudaGetLastError());
+  // 64 inputs a tile while that is one item an SM or fewer (26 a member)
+  const int n_tile = 26 * G <= s->sm_count ? 64 : 128;
+  const int items = G * 2 * (3 * (kWidth / n_tile) + 1), dw_grid = std::min(items, s->sm_count);
+  // The class sums start as their sources come where the weight gradients leave
+  // them fewer than a third of the SMs (5 members of 16,384 rows, 24 steps:
+  // 10.49 -> 9.71 ms), else all at once beside those (a member of 4,096 rows,
+  // 48 steps, is bound by its launches: 5.87 ms, 6.05 with three more a step)
+  const bool early = 3 * dw_grid > 2 * s->sm_count;
+  ClassSources c{};
+  for (int li = 0; li < 4; ++li) c.src[li] = t.dH[li];
+  c.src[4] = t.X[3];
+  c.dy = t.dy;
+  auto class_sums = [&](int k, int n) -> int {
+    SUR_TRY(cudaEventRecord(s->ev_fork, s->stream));
+    SUR_TRY(cudaStreamWaitEvent(s->side, s->ev_fork, 0));
+    k_class_sums<<<dim3(kClasses / kClassBlock, kWidth / 64, n * G), 256, 0, s->side>>>(c, k, n, R, t.cls);
+    return cuda_status(cudaGetLastError());
+  };
+  if (early && (rc = class_sums(3, 2)) != GELIO_OK) return rc;
   for (int li = 3; li > 0; --li) {
     a.K = kWidth; a.z_prev = t.Z[li - 1]; a.dh_out = t.dH[li - 1];
     if ((rc = launch_train<DX>(s, t.adH[li], s->tWT[li - 1], a)) != GELIO_OK) return rc;
+    if (early && li > 1 && (rc = class_sums(li - 1, 1)) != GELIO_OK) return rc;
   }
   u.rows = R; u.G = G; u.m0 = m0;
   for (int li = 0; li < 4; ++li) {
@@ -406,17 +426,10 @@ int train_step(gelio_surrogate *s, int m0, int G, int n_valid, UpdateArgs &u) {
   u.timeout_ns = a.timeout_ns;
   SUR_TRY(cudaEventRecord(s->ev_fork, s->stream));
   SUR_TRY(cudaStreamWaitEvent(s->side, s->ev_fork, 0));
-  ClassSources c{};
-  for (int li = 0; li < 4; ++li) c.src[li] = t.dH[li];
-  c.src[4] = t.X[3];
-  c.dy = t.dy;
-  // 64 inputs a tile while that is one item an SM or fewer (26 a member: 5
-  // members of 16,384 rows 128 us; at 128 inputs 70 of the SMs work, 190 us)
-  const int n_tile = 26 * G <= s->sm_count ? 64 : 128;
-  const int items = G * 2 * (3 * (kWidth / n_tile) + 1);
-  k_train_dw<<<std::min(items, s->sm_count), kTrainThreads, kDwSmem, s->stream>>>(t.dw, u, n_tile);
+  k_train_dw<<<dw_grid, kTrainThreads, kDwSmem, s->stream>>>(t.dw, u, n_tile);
   SUR_TRY(cudaGetLastError());
-  k_class_sums<<<dim3(kClasses / kClassBlock, kWidth / 64, 5 * G), 256, 0, s->side>>>(c, R, t.cls);
+  const int left = early ? 1 : 5;
+  k_class_sums<<<dim3(kClasses / kClassBlock, kWidth / 64, left * G), 256, 0, s->side>>>(c, 0, left, R, t.cls);
   k_update_biases<<<dim3(41, G), 256, 0, s->side>>>(u);
   SUR_TRY(cudaGetLastError());
   SUR_TRY(cudaEventRecord(s->ev_join, s->side));
@@ -699,6 +712,9 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
     }
   }
   if (rc != GELIO_OK) return fail(rc);
+  // one member's training memory is taken here: its allocations were 0.3 of the
+  // 1.3 ms of a first short training; a group's comes with its first training
+  if (group_size(s) == 1 && (rc = ensure_train(s, 1)) != GELIO_OK) return fail(rc);
   bool ok = make_map(&s->mQ0, s->Q0, kInPad, kQueryBatch, kTileM);
   ok = ok && make_map3(&s->tW1, s->W1, kInPad, kWidth, E, kWidth);
   for (int i = 0; i < 3; ++i)

@@ -286,14 +286,20 @@ __device__ __forceinline__ int layer_bias(int li) {
   return li == 0 ? kOffB1 : li == 1 ? kOffB2 : li == 2 ? kOffB3 : kOffB4;
 }
 
-// Adam (bias-corrected) on one FP32 master parameter; returns its new value.
+// Adam (bias-corrected) on one FP32 master parameter p and its moments;
+// returns its new value.
+__device__ __forceinline__ float adam_step(const UpdateArgs &u, int slot, float gi, float p, float &m1, float &m2) {
+  m1 = fmaf(1.0f - u.b1, gi, __fmul_rn(u.b1, m1));
+  m2 = fmaf(__fmul_rn(1.0f - u.b2, gi), gi, __fmul_rn(u.b2, m2));
+  return p - u.lr[slot] * (m1 / u.c1[slot]) / (sqrtf(m2 / u.c2[slot]) + u.eps);
+}
+
 __device__ __forceinline__ float adam(const UpdateArgs &u, int slot, int i, float gi) {
   float *p = u.P[slot], *m1 = u.M1[slot], *m2 = u.M2[slot];
-  const float a = fmaf(1.0f - u.b1, gi, __fmul_rn(u.b1, m1[i]));
-  const float b = fmaf(__fmul_rn(1.0f - u.b2, gi), gi, __fmul_rn(u.b2, m2[i]));
+  float a = m1[i], b = m2[i];
+  const float v = adam_step(u, slot, gi, p[i], a, b);
   m1[i] = a;
   m2[i] = b;
-  const float v = p[i] - u.lr[slot] * (a / u.c1[slot]) / (sqrtf(b / u.c2[slot]) + u.eps);
   p[i] = v;
   return v;
 }
@@ -313,16 +319,20 @@ __device__ __forceinline__ float adam(const UpdateArgs &u, int slot, int i, floa
 //   warp 1  (one lane)  MMA issuer
 //   warps 2-9           epilogue: warp w TMEM lanes 32 (w % 4) .. +31 (output
 //           features), half (w - 2) / 4 of the tile's columns
-// Bound by the operands' way from L2 (6 MB an item at N = 64, 130 items for five
-// members of 16,384 rows: 128 us, 6 TB/s; through partials in HBM and an update
-// kernel of their own, 250 us).  With many members N = 128 halves the items.
+// The update goes through shared memory (a lane an input, 128-byte rows): with a
+// feature a lane its scattered accesses were 57 of 135 us.  Now 78 us for five
+// members of 16,384 rows: the products (390 cycles a chunk of 64 rows) and the
+// operands' way from L2 (6 MB an item at N = 64, 130 items) take about as long
+// and overlap.  Through partials in HBM and an update kernel it was 250 us.
+// With many members N = 128 halves the items.
 // ----------------------------------------------------------------------------
 constexpr int kDwStages = 6;
 constexpr uint32_t kDwBox = kChunk * 128;               // 8 KiB: 64 columns of 64 rows
 constexpr uint32_t kDwStage = 4 * kDwBox;               // 128 features, up to 128 inputs
 constexpr int kDwBuffers = 4;
 constexpr int kDwCols = 128;
-constexpr size_t kDwSmem = 1024 + (size_t)kDwStages * kDwStage + 256;
+constexpr int kDwPitch = 33;                            // floats a row of a warp's 32 x 32 piece
+constexpr size_t kDwSmem = 1024 + (size_t)kDwStages * kDwStage + 256 + (size_t)kEpiWarps * 32 * kDwPitch * 4;
 
 struct DwMaps {
   CUtensorMap dh[4], x[4];          // boxes of {64 columns, 64 rows, 1 slot}
@@ -458,6 +468,7 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
   } else {
     const int q = warp & 3;                       // TMEM lane quarter of this warp
     const int h = (warp - 2) / 4;                 // column half of this warp
+    float *tile = reinterpret_cast<float *>(base + kDwStages * kDwStage + 256) + (warp - 2) * 32 * kDwPitch;
     uint32_t count = 0;
     bool ok = true;
     for (int w = blockIdx.x; w < items && ok; w += gridDim.x) {
@@ -489,24 +500,54 @@ __global__ void __launch_bounds__(kTrainThreads, 1)
         if (lane == 0) atomicExch(u.error, 6u);
         break;
       }
-      // output feature o, inputs i0 .. i0 + mine - 1
-      const int o = t.m * kTileM + q * 32 + lane, i0 = t.n0 + h * mine;
+      // features o0 .. o0 + 31 of this warp, 32 inputs at a time through the
+      // warp's piece of shared memory: a lane holds one feature's sums and
+      // updates one input's parameters of every feature
+      const int o0 = t.m * kTileM + q * 32;
       const int fan_in = t.li == 0 ? kFeatures : kWidth, ld = t.li == 0 ? kInPad : kWidth;
-      const int off = layer_weights(t.li) + o * fan_in;
-      __nv_bfloat16 *wr = u.w[t.li] + ((size_t)(u.m0 + t.slot) * kWidth + o) * ld;
-      __nv_bfloat16 *wc = u.wt[t.li] ? u.wt[t.li] + (size_t)(u.m0 + t.slot) * kWidth * kWidth + o : nullptr;
+      float *P = u.P[t.slot], *M1 = u.M1[t.slot], *M2 = u.M2[t.slot];
+      __nv_bfloat16 *wr = u.w[t.li] + (size_t)(u.m0 + t.slot) * kWidth * ld;
+      __nv_bfloat16 *wc = u.wt[t.li] ? u.wt[t.li] + (size_t)(u.m0 + t.slot) * kWidth * kWidth : nullptr;
 #pragma unroll
-      for (int j = 0; j < 64; ++j) {
-        const int i = i0 + j;
-        if (j < mine && i < fan_in) {
+      for (int part = 0; part < 2; ++part) {
+        if (part * 32 >= mine) break;
+        const int i0 = t.n0 + h * mine + part * 32, i = i0 + lane;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 32; ++j) tile[lane * kDwPitch + j] = s[part * 32 + j];
+        __syncwarp();
+        if (i < fan_in) {
+          const int off = layer_weights(t.li) + o0 * fan_in + i;
           if (u.grad) {
-            u.grad[off + i] = s[j];
+            for (int r = 0; r < 32; ++r) u.grad[off + r * fan_in] = tile[r * kDwPitch + lane];
           } else {
-            const __nv_bfloat16 b = __float2bfloat16_rn(adam(u, t.slot, off + i, s[j]));
-            wr[i] = b;
-            if (wc) wc[(size_t)i * kWidth] = b;
+            for (int r0 = 0; r0 < 32; r0 += 8) {
+              float v[8], m1[8], m2[8];
+#pragma unroll
+              for (int r = 0; r < 8; ++r) {
+                const int k = off + (r0 + r) * fan_in;
+                v[r] = P[k];
+                m1[r] = M1[k];
+                m2[r] = M2[k];
+              }
+#pragma unroll
+              for (int r = 0; r < 8; ++r) {
+                const int k = off + (r0 + r) * fan_in;
+                float &g = tile[(r0 + r) * kDwPitch + lane];
+                v[r] = adam_step(u, t.slot, g, v[r], m1[r], m2[r]);
+                P[k] = v[r];
+                M1[k] = m1[r];
+                M2[k] = m2[r];
+                wr[(size_t)(o0 + r0 + r) * ld + i] = __float2bfloat16_rn(v[r]);
+                g = v[r];
+              }
+            }
           }
         }
+        __syncwarp();
+        if (wc && !u.grad)
+          for (int j = 0; j < 32; ++j)
+            wc[(size_t)(i0 + j) * kWidth + o0 + lane] = __float2bfloat16_rn(tile[lane * kDwPitch + j]);
       }
     }
   }
@@ -589,16 +630,16 @@ __global__ void __launch_bounds__(256) k_head_backward(const float *__restrict__
 // the rows c = t, t + 256, ..., in that order, to out[g][k][t][f]: k = 0..3 dH_1
 // .. dH_4, k = 4 X4 weighted by dy.  A block takes 16 classes x 64 columns of one
 // source, a thread 4 columns of a class (8-byte loads, two rows of 128 bytes a
-// warp, 16 rows in flight).  HBM-bound; it runs beside the weight gradients.
-// Read from transposed copies by one block a column it took 32 us a source and
-// member.
+// warp, 16 rows in flight).  HBM-bound.  It runs beside the backward products, a
+// source as soon as it is there, or beside the weight gradients: the n sources
+// from k0 on (all of five members 42 us alone, 135 us beside those).
 constexpr int kClassBlock = 16;
 struct ClassSources {
   const __nv_bfloat16 *src[5];
   const float *dy;
 };
-__global__ void __launch_bounds__(256) k_class_sums(const ClassSources a, int rows, float *__restrict__ out) {
-  const int k = blockIdx.z % 5, slot = blockIdx.z / 5;
+__global__ void __launch_bounds__(256) k_class_sums(const ClassSources a, int k0, int n, int rows, float *__restrict__ out) {
+  const int k = k0 + blockIdx.z % n, slot = blockIdx.z / n;
   const int f0 = blockIdx.y * 64 + (threadIdx.x & 15) * 4;
   const int t = blockIdx.x * kClassBlock + (threadIdx.x >> 4);
   const size_t base = (size_t)slot * rows;
@@ -613,7 +654,7 @@ __global__ void __launch_bounds__(256) k_class_sums(const ClassSources a, int ro
 #pragma unroll
     for (int j = 0; j < 4; ++j) s[j] = fmaf(__bfloat162float(x[j]), wc, s[j]);
   }
-  *reinterpret_cast<float4 *>(out + ((size_t)blockIdx.z * kClasses + t) * kWidth + f0) =
+  *reinterpret_cast<float4 *>(out + (((size_t)slot * 5 + k) * kClasses + t) * kWidth + f0) =
       make_float4(s[0], s[1], s[2], s[3]);
 }
 

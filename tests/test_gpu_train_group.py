@@ -17,7 +17,7 @@ pytestmark = pytest.mark.gpu
 def test_member_does_not_depend_on_its_group(engine, batch, rows):
     x, t = data(rows, seed=rows)
     out = []
-    for members in (1, 3, 16):
+    for members in (1, 3, 5, 16):
         s = sg.Surrogate(engine, members=members, batch_rows=batch, seed=23)
         s.set_params(0, init_params(seed=1))
         s.add_rows(x, t)
