@@ -835,6 +835,7 @@ static int enqueue_run(gelio_ctx *c, int n, const gelio_run_opts *o, double *d_o
     if (rc != GELIO_OK) return rc;
     a.smem_slots = s.smem_slots;
     a.refill = s.refill;
+    a.ctas_per_sm = s.blocks_per_sm;
     GELIO_TRY(launch_model(m, true, variant, s.grid, s.block, s.smem, st, a));
     if (!have_first) { first = s; have_first = true; }
   }

@@ -86,6 +86,7 @@ struct KArgs {
   unsigned long long time_limit_ns; // 0 = no watchdog
   int smem_slots;                 // >0: histograms of the group's first smem_slots sims in shared memory
   int refill;                     // steps between refills (multiple of 4)
+  int ctas_per_sm;                // the grid is as many CTAs for each SM
   // plain / replay kernel
   int plain_sim;                  // simulation index of a plain launch
   unsigned long long plain_first, plain_count;
@@ -532,18 +533,59 @@ __device__ __forceinline__ int find_group_index(const unsigned long long *prefix
   return lo;
 }
 
-// Lanes that each warp of the launch opens.  A run of fewer trajectories than
-// the launch has lanes ends with its longest chains, and a chain is slowed by
-// the warps it shares its SM with and by the other lanes of its warp (their
-// branches are its own).  Handed out 32 to the warp that asks first, 4,096
-// trajectories sat in 128 warps on 16 of the 152 SMs.  Such a run is spread over
-// all warps, as many lanes in each as it needs: few enough, often, that the warp
-// draws their normals (kCoopLanes).  4,096 2D Geliosphere trajectories 19.7 ->
-// 16.3 ms, 4,001 1D B-p trajectories in FP64 steps 1,205 -> 849 ms; on half of
-// the warps 5,000 B-p trajectories took 10% longer.
-__device__ __forceinline__ unsigned spread_lanes(unsigned long long total, unsigned ctas, unsigned warps_per_cta) {
-  const unsigned long long w = (unsigned long long)ctas * warps_per_cta;
-  return total < w * 32u ? (unsigned)((total + w - 1) / w) : 32u;
+// Which warps of the launch work, and how many lanes each opens.  A run ends with
+// its longest chains, and a chain is slowed by the warps it shares its SM with and
+// by the other lanes of its warp (their branches are its own).
+//  * Few trajectories are spread over all warps, as many lanes in each as it
+//    needs: while that is so few that a warp draws their normals together
+//    (kCoopLanes).  4,096 2D Geliosphere trajectories 19.7 -> 16.3 ms (handed out
+//    32 to the warp that asked first they sat on 16 SMs), 4,001 1D B-p
+//    trajectories in FP64 steps 1,205 -> 849 ms; 5,000 in FP32 steps 47 ms, on a
+//    quarter of the warps 58.
+//  * From there on, FP32 steps take as few warps of each SM, in fours (one a
+//    scheduler), as leave a lane 6 trajectories or fewer: the long chains, which
+//    start first, run alone for longer, and a lane's later trajectories fill the
+//    time.  On 4 / 8 / 12 / 16 warps an SM, ms: 1D B-p 50,000 62.9 / 72 / 74 / 77,
+//    100,000 80 / 83 / 86 / 90, 200,000 135 / 101 / 98 / 109, 300,000 192 / 132 /
+//    121 / 126, 800,000 488 / 314 / 267 / 256; 2D Geliosphere 150,000 29.7 / 30.7 /
+//    31.5 / 34.6, 300,000 40.9 / 33.0 / 34.7 / 36.0.
+struct Placement {
+  unsigned warps, lanes;          // of each CTA; of each of those warps
+  unsigned long long dealt;       // first tickets, one a lane
+};
+template <class R>
+__device__ __forceinline__ Placement place(unsigned long long total, unsigned ctas, unsigned warps, unsigned ctas_per_sm) {
+  Placement p{warps, 32u, 0ull};
+  const unsigned long long all = (unsigned long long)ctas * warps;
+  if (total <= all * kCoopLanes<R>) {
+    p.lanes = (unsigned)((total + all - 1) / all);
+  } else if (sizeof(R) == 4 && ctas_per_sm > 0) {
+    const unsigned long long four = (unsigned long long)(ctas / ctas_per_sm) * 4 * 32;   // lanes of four warps an SM
+    const unsigned long long fours = (total + 6 * four - 1) / (6 * four);
+    const unsigned long long w = (4 * fours + ctas_per_sm - 1) / ctas_per_sm;
+    if (w < warps) p.warps = (unsigned)w;
+  }
+  const unsigned long long n = (unsigned long long)ctas * p.warps;
+  if (total < n * p.lanes) p.lanes = (unsigned)((total + n - 1) / n);
+  p.dealt = n * p.lanes;
+  return p;
+}
+
+// A warp's place among the working warps of its CTA (it works if below `work`).
+// Warp slots of an SM belong to its schedulers in turn, so the CTAs of an SM take
+// different ones: with warps 0 and 1 of both CTAs at work, 100,000 B-p
+// trajectories took 92 ms, 80 with a warp on each scheduler.
+__device__ __forceinline__ unsigned warp_rank(const unsigned *slot, unsigned warp, unsigned warps, unsigned work) {
+  unsigned first = slot[0];
+  for (unsigned w = 1; w < warps; ++w) first = min(first, slot[w]);
+  const unsigned turn = warps - first / warps * work % warps;
+  const unsigned mine = (slot[warp] + turn) % warps;
+  unsigned r = 0;
+  for (unsigned w = 0; w < warps; ++w) {
+    const unsigned k = (slot[w] + turn) % warps;
+    r += (k < mine || (k == mine && w < warp)) ? 1u : 0u;
+  }
+  return r;
 }
 
 // ---------------------------------------------------------------------------
@@ -569,8 +611,16 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   unsigned char *coop_base = reinterpret_cast<unsigned char *>(qbase + warps * kQueue);
   R *coop = reinterpret_cast<R *>(coop_base + warp * coop_bytes(MODEL, sizeof(R)));
   int *qlen = reinterpret_cast<int *>(coop_base + warps * coop_bytes(MODEL, sizeof(R))) + warp;
-  if ((threadIdx.x & 31) == 0) *qlen = 0;
+  __shared__ Placement pl;
+  __shared__ unsigned s_slot[8], s_rank[8];
+  if ((threadIdx.x & 31) == 0) {
+    *qlen = 0;
+    asm volatile("mov.u32 %0, %%warpid;" : "=r"(s_slot[warp]));
+  }
+  if (threadIdx.x == 0) pl = place<R>(gpre[ne], gridDim.x, warps, (unsigned)a.ctas_per_sm);
   __syncthreads();
+  if ((threadIdx.x & 31) == 0) s_rank[warp] = pl.warps < warps ? warp_rank(s_slot, warp, warps, pl.warps) : warp;
+  __syncwarp();
   Sink<MODEL> sink;
   sink.sh = sh_hist;
   sink.smem_slots = slots;
@@ -588,9 +638,9 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   // exhausted (warp-uniform): every ticket is handed out, so no lane of this
   // warp will be refilled again
   {
-    const unsigned lanes = spread_lanes(gpre[ne], gridDim.x, warps);
-    drained = (unsigned)lane >= lanes;
-    exhausted = gpre[ne] <= (unsigned long long)gridDim.x * warps * lanes;
+    const bool works = s_rank[warp] < pl.warps;
+    drained = !works || (unsigned)lane >= pl.lanes;
+    exhausted = !works || gpre[ne] <= pl.dealt;
   }
   int slot = 0;
   unsigned window = 0;
@@ -632,12 +682,13 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
     if (need) {
       const int leader = __ffs(need) - 1;
       const unsigned long long total = gpre[ne];
-      const unsigned lanes = spread_lanes(total, gridDim.x, warps);
-      unsigned long long base = ((unsigned long long)warp * gridDim.x + blockIdx.x) * lanes;
+      unsigned long long base = ((unsigned long long)s_rank[warp] * gridDim.x + blockIdx.x) * pl.lanes;
       if (window > 1u) {
         if (lane == leader) {
-          const unsigned long long dealt = (unsigned long long)gridDim.x * warps * lanes;
-          base = dealt + atomicAdd(&a.ctl->ticket[MODEL], (unsigned long long)__popc(need));
+          // formed anew: kept in shared memory it cost the 2D step loop its registers'
+          // order (4 x 2.5 M 492.7 -> 494 to 497 ms)
+          base = place<R>(total, gridDim.x, warps, (unsigned)a.ctas_per_sm).dealt +
+                 atomicAdd(&a.ctl->ticket[MODEL], (unsigned long long)__popc(need));
         }
         base = __shfl_sync(kFull, base, leader);
       }

@@ -196,6 +196,7 @@ extern "C" int32_t gelio_run_noalloc(const gelio_sim_params *d_sims, int32_t n_s
   const unsigned grid = (unsigned)(s->sm_count * s->occ[variant]);
   for (int m = 0; m < 4; ++m) {
     a.refill = (opts && opts->refill_interval > 0) ? opts->refill_interval : (m == kModelFp ? 4 : 16);
+    a.ctas_per_sm = s->occ[variant];
     if (launch(m, variant, grid, kBlock, kQueueBytes, st, a) != cudaSuccess) return GELIO_ERR_CUDA;
   }
   if (launch_reduce(part, kSlices, (long long)n_sims * kSpecDoubles, reinterpret_cast<double *>(d_out), st) !=

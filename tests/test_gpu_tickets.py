@@ -43,3 +43,14 @@ def test_every_particle_once(engine, model, prec, counts):
 def test_small_runs_at_the_lines_of_the_placement(engine, n):
     sim = make_sim(abi.GELIO_MODEL_2D_SOLARPROP, n, injection=LOG, inj_min=30.0, inj_max=100.0, inj_points=7, seed=3)
     same(engine.run(sim).spectra[0], engine.run(sim, plain=True).spectra[0])
+
+
+# around the lines between one, two, three and four warps a scheduler: 6 trajectories a lane of the fewer
+@pytest.mark.parametrize("model", [abi.GELIO_MODEL_2D_GELIOSPHERE, abi.GELIO_MODEL_1D_BP, abi.GELIO_MODEL_1D_FP])
+@pytest.mark.parametrize("kw", [{}, {"block_size": 96}, {"block_size": 64, "blocks_per_sm": 3}, {"compact": 2}])
+def test_every_particle_once_on_fewer_warps(engine, model, kw):
+    for n in (19456, 19457, 116736, 116737, 233473, 350209):
+        sim = make_sim(model, n, injection=LOG, inj_min=50.0, inj_max=100.0, inj_points=7, seed=n)
+        # the 80-register kernels of the 2D models round differently from the plain one: their own on all warps
+        ref = {"compact": 2, "block_size": 32, "blocks_per_sm": 4} if "compact" in kw else {"plain": True}
+        same(engine.run(sim, **kw).spectra[0], engine.run(sim, **ref).spectra[0])
