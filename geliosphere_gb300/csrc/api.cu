@@ -615,8 +615,11 @@ static int choose_slices(int n_sims) {
 // Steps between refills.  A vote and a refill cost the warp about 100
 // instructions, an ended lane idles half a window: trajectories of thousands of
 // steps want long windows (4 x 2.5 M 2D Geliosphere 502 ms at 16, 498 at 32 and
-// 64; B-p 400,000 155 / 152 / 148), half of the F-p ones end with their first.
-static int default_refill(int model) { return (model == kModelFp) ? 4 : (model == kModelBp) ? 64 : 32; }
+// 64; B-p 400,000 155 / 152 / 148; 3 M SolarProp-like 207.1 / 204.3 / 202.8),
+// half of the F-p ones end with their first.
+static int default_refill(int model) {
+  return (model == kModelFp) ? 4 : (model == kModelGeliosphere) ? 32 : 64;
+}
 
 struct LaunchShape {
   unsigned grid, block;
