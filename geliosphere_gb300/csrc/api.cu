@@ -465,6 +465,7 @@ struct gelio_ctx {
   int device = 0;
   int sm_count = 0;
   int max_smem_optin = 0;
+  std::atomic<int> tuning{0};          // autotunes under way
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr;
   cudaStream_t copy_stream = nullptr, eval_stream = nullptr;   // gelio_evaluate: rows on their way up, every other piece
@@ -838,7 +839,7 @@ static int enqueue_run(gelio_ctx *c, int n, const gelio_run_opts *o, double *d_o
     if (rc != GELIO_OK) return rc;
     a.smem_slots = s.smem_slots;
     a.refill = s.refill;
-    a.ctas_per_sm = s.blocks_per_sm;
+    a.ctas_per_sm = c->tuning > 0 ? 0 : s.blocks_per_sm;
     GELIO_TRY(launch_model(m, true, variant, s.grid, s.block, s.smem, st, a));
     if (!have_first) { first = s; have_first = true; }
   }
@@ -1184,6 +1185,13 @@ int32_t gelio_autotune(gelio_ctx *c, const gelio_sim_params *sims, int32_t n, ge
   static const int compacts[2] = {1, 2};
   double best_rate = -1.0;
   gelio_run_opts bo{};
+  // a sample stands for a larger run: it is timed on all warps (on the few that
+  // a sample of its size would take, the shapes hardly differ)
+  struct Tuning {
+    std::atomic<int> &n;
+    explicit Tuning(std::atomic<int> &n_) : n(n_) { ++n; }
+    ~Tuning() { --n; }
+  } tuning(c->tuning);
   std::vector<gelio_spectra> tmp(n);
   // one untimed run first (lazy allocations), then every shape once
   {
