@@ -4,10 +4,10 @@
 // one trajectory at a time.  Lanes whose particle has ended are refilled at
 // warp level every `refill` steps: a ballot of idle lanes, one 64-bit
 // atomicAdd per warp on the model's ticket counter, and each idle lane takes
-// ticket base + rank.  Tickets run over all particles of all simulations of
-// the model in the launch (a whole batch CSV in one launch), a segment of each
-// simulation in turn; the ticket -> (simulation, particle) map is a binary
-// search of the segments' prefix sums.
+// place base + rank of the queue.  Tickets run over all particles of all
+// simulations of the model in the launch (a whole batch CSV in one launch), a
+// segment of each simulation in turn; the ticket -> (simulation, particle) map
+// is a binary search of the segments' prefix sums.
 // This replaces the reference's host loop of 4,096-particle chunks with three
 // device synchronisations each (GeliosphereModel.cu:426-445), and its
 // warp-wide wait for the slowest particle.
@@ -551,10 +551,10 @@ __device__ __forceinline__ int find_group_index(const unsigned long long *prefix
 //    31.5 / 34.6, 300,000 40.9 / 33.0 / 34.7 / 36.0.
 struct Placement {
   unsigned warps, lanes;          // of each CTA; of each of those warps
-  unsigned long long dealt;       // first tickets, one a lane
+  unsigned long long dealt;       // first places in the queue, one a lane
 };
 template <class R>
-__device__ __forceinline__ Placement place(unsigned long long total, unsigned ctas, unsigned warps, unsigned ctas_per_sm) {
+__host__ __device__ __forceinline__ Placement place(unsigned long long total, unsigned ctas, unsigned warps, unsigned ctas_per_sm) {
   Placement p{warps, 32u, 0ull};
   const unsigned long long all = (unsigned long long)ctas * warps;
   if (total <= all * kCoopLanes<R>) {
@@ -571,6 +571,35 @@ __device__ __forceinline__ Placement place(unsigned long long total, unsigned ct
   return p;
 }
 
+// Ticket of a place in the launch's one queue (what the counter gave).  A CTA's
+// first request is for all its warps, `lanes` places each, and those places are
+// dealt: the w-th warp of the b-th CTA to ask gets chunk w * ctas + b, so that every
+// SM starts with its share of each length of trajectory (32 tickets in a row to
+// each warp that asked, the longest went to the few CTAs that started first: 60,000
+// 2D particles 28.3 ms, dealt 25.0).  A place is taken by whoever asks: a CTA that
+// is not resident yet, because another context's run holds its SM, keeps none of
+// them from the others (tied to the CTAs' numbers, 250,000 2D particles beside a
+// run on half of every SM took 59.8 ms, 43.9 so; 60,000 SolarProp-like ones 46.9 and
+// 32.6).  Where there are more lanes than tickets, some places have none.
+__host__ __device__ __forceinline__ unsigned long long ticket_at(unsigned long long at, const Placement &p, unsigned ctas) {
+  if (at >= p.dealt) return at;
+  const uint32_t chunk = (uint32_t)at / p.lanes, i = (uint32_t)at % p.lanes;
+  return (unsigned long long)(chunk % p.warps * ctas + chunk / p.warps) * p.lanes + i;
+}
+// Out of line and formed anew, for all models but 2D Geliosphere: the division, or
+// the placement read from shared memory, costs their step loops registers
+// (SolarProp-like 20,000 18.5 -> 18.9 ms, F-p 10^6 53.5 -> 54.6); Geliosphere's
+// loop loses by the call (4 x 2.5 M 491.1 -> 498.8).
+template <class R>
+static __device__ __noinline__ unsigned long long first_ticket(unsigned long long at, unsigned long long total,
+                                                               unsigned ctas, unsigned warps, unsigned ctas_per_sm) {
+  return ticket_at(at, place<R>(total, ctas, warps, ctas_per_sm), ctas);
+}
+
+// Refill windows of a warp: at the first (1) its places are asked for already, and
+// no later one counts as the first however long the run.
+__host__ __device__ __forceinline__ unsigned next_window(unsigned window) { return window == 0xffffffffu ? 8u : window + 1u; }
+
 // A warp's place among the working warps of its CTA (it works if below `work`).
 // Warp slots of an SM belong to its schedulers in turn, so the CTAs of an SM take
 // different ones: with warps 0 and 1 of both CTAs at work, 100,000 B-p
@@ -586,6 +615,17 @@ __device__ __forceinline__ unsigned warp_rank(const unsigned *slot, unsigned war
     r += (k < mine || (k == mine && w < warp)) ? 1u : 0u;
   }
   return r;
+}
+
+// A 1D lane's normals of a group, out of line (for a refill in a run's tail).
+template <class R> struct Group4 {
+  R z[4];
+};
+template <class R>
+static __device__ __noinline__ Group4<R> group_of(uint32_t k0, uint32_t k1, uint32_t group, unsigned long long pid) {
+  Group4<R> g;
+  normals4<R>(k0, k1, group, kStreamSde, pid, g.z);
+  return g;
 }
 
 // ---------------------------------------------------------------------------
@@ -613,11 +653,15 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   int *qlen = reinterpret_cast<int *>(coop_base + warps * coop_bytes(MODEL, sizeof(R))) + warp;
   __shared__ Placement pl;
   __shared__ unsigned s_slot[8], s_rank[8];
+  __shared__ unsigned long long s_first;
   if ((threadIdx.x & 31) == 0) {
     *qlen = 0;
     asm volatile("mov.u32 %0, %%warpid;" : "=r"(s_slot[warp]));
   }
-  if (threadIdx.x == 0) pl = place<R>(gpre[ne], gridDim.x, warps, (unsigned)a.ctas_per_sm);
+  if (threadIdx.x == 0) {
+    pl = place<R>(gpre[ne], gridDim.x, warps, (unsigned)a.ctas_per_sm);
+    s_first = atomicAdd(&a.ctl->ticket[MODEL], (unsigned long long)(pl.warps * pl.lanes));
+  }
   __syncthreads();
   if ((threadIdx.x & 31) == 0) s_rank[warp] = pl.warps < warps ? warp_rank(s_slot, warp, warps, pl.warps) : warp;
   __syncwarp();
@@ -630,13 +674,8 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   Lane<R> L;
   Consts<R> K;
   bool active = false, drained, exhausted;
-  // The first tickets are dealt, not asked for: chunk w * CTAs + b to warp w of
-  // CTA b, so that every SM starts with its share of each length of trajectory
-  // (asked for, the longest went to the CTAs that started first: 60,000 2D
-  // particles 28.3 ms, dealt 25.0).  The counter hands out those after.
-  //
-  // exhausted (warp-uniform): every ticket is handed out, so no lane of this
-  // warp will be refilled again
+  // exhausted (warp-uniform): every ticket is handed out, or is by the CTAs' first
+  // requests (those of a CTA that is not resident may yet come to this warp)
   {
     const bool works = s_rank[warp] < pl.warps;
     drained = !works || (unsigned)lane >= pl.lanes;
@@ -677,24 +716,29 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
         drained = true;
       }
     }
-    ++window;
+    window = next_window(window);
     const unsigned need = __ballot_sync(kFull, !active && !drained);
     if (need) {
       const int leader = __ffs(need) - 1;
       const unsigned long long total = gpre[ne];
-      unsigned long long base = ((unsigned long long)s_rank[warp] * gridDim.x + blockIdx.x) * pl.lanes;
+      unsigned long long base = s_first + s_rank[warp] * pl.lanes;
       if (window > 1u) {
-        if (lane == leader) {
-          // formed anew: kept in shared memory it cost the 2D step loop its registers'
-          // order (4 x 2.5 M 492.7 -> 494 to 497 ms)
-          base = place<R>(total, gridDim.x, warps, (unsigned)a.ctas_per_sm).dealt +
-                 atomicAdd(&a.ctl->ticket[MODEL], (unsigned long long)__popc(need));
-        }
+        if (lane == leader) base = atomicAdd(&a.ctl->ticket[MODEL], (unsigned long long)__popc(need));
         base = __shfl_sync(kFull, base, leader);
+      }
+      if constexpr (Prefetch<MODEL>::value) {
+        // the tail's draws leave zq behind: drawn again if a lane gets a ticket after all
+        if (exhausted && base < total && window > 1u) {
+          const Group4<R> z = group_of<R>(L.key0, L.key1, L.steps / 4u, L.pid);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) zq[j] = z.z[j];
+        }
       }
       if (base + (unsigned long long)__popc(need) >= total) exhausted = true;
       if (!active && !drained) {
-        const unsigned long long t = base + __popc(need & lanemask_lt());
+        unsigned long long t = base + __popc(need & lanemask_lt());
+        if constexpr (MODEL == kModelGeliosphere) t = ticket_at(t, pl, gridDim.x);
+        else if (t < (unsigned long long)gridDim.x * blockDim.x) t = first_ticket<R>(t, total, gridDim.x, warps, (unsigned)a.ctas_per_sm);
         if (t < total) {
           const int g = find_group_index(gpre, ne, t);
           const int seg = g / gn;

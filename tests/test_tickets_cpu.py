@@ -1,0 +1,71 @@
+"""The queue of the persistent kernels' tickets, on the host: the kernels' own
+functions compiled into a small program.  Every place of the queue is one ticket
+and every ticket one place, whichever CTAs ask and however late; a CTA's first
+places are its share of each length of trajectory; a warp's count of its windows
+never comes back to its first."""
+import os
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+from geliosphere_gb300 import build
+
+PROGRAM = r"""
+#include <cstdio>
+#include <vector>
+#include "kernels.cuh"
+using namespace gelio;
+
+template <class R> int check(unsigned long long total, unsigned ctas, unsigned warps, unsigned per_sm) {
+  const Placement p = place<R>(total, ctas, warps, per_sm);
+  if (p.warps < 1 || p.warps > warps || p.lanes > 32 || (total && p.lanes < 1)) return 1;
+  const unsigned long long places = total > p.dealt ? total : p.dealt;
+  std::vector<char> seen(total, 0);
+  unsigned long long got = 0;
+  for (unsigned long long at = 0; at < places; ++at) {
+    const unsigned long long t = ticket_at(at, p, ctas);
+    if (t >= places) return 2;
+    if (t >= total) continue;
+    if (seen[t]) return 3;
+    seen[t] = 1;
+    ++got;
+  }
+  if (got != total) return 4;
+  if (ticket_at(places, p, ctas) < total || ticket_at(places + 12345, p, ctas) < total) return 5;
+  // a CTA that asks b-th: warp w starts with chunk w * ctas + b
+  for (unsigned b = 0; b < ctas && total; b += 7)
+    for (unsigned w = 0; w < p.warps; ++w)
+      if (ticket_at((unsigned long long)(b * p.warps + w) * p.lanes, p, ctas) !=
+          (unsigned long long)(w * ctas + b) * p.lanes) return 6;
+  return 0;
+}
+
+int main() {
+  const unsigned shapes[][3] = {{304, 8, 2}, {152, 8, 1}, {456, 3, 3}, {608, 4, 4}, {1216, 1, 8}, {1, 1, 1}, {304, 8, 0}};
+  const unsigned long long totals[] = {0, 1, 2, 151, 152, 303, 305, 500, 2431, 2432, 2433, 9727, 9729, 19456, 19457, 38911,
+                                       38913, 77823, 77824, 77825, 116736, 116737, 233473, 350209, 1000003};
+  for (auto &s : shapes)
+    for (auto n : totals) {
+      const int f = check<float>(n, s[0], s[1], s[2]), d = check<double>(n, s[0], s[1], s[2]);
+      if (f || d) { printf("total %llu ctas %u warps %u per sm %u: %d %d\n", n, s[0], s[1], s[2], f, d); return 1; }
+    }
+  unsigned w = 0;
+  if ((w = next_window(w)) != 1u || (w = next_window(w)) != 2u) return 2;
+  for (w = 0xfffffff0u; w != 9u; w = next_window(w))
+    if (w < 2u) { puts("a late window counts as the first"); return 3; }
+  puts("ok");
+}
+"""
+
+
+def test_every_place_is_a_ticket(tmp_path):
+    src, exe = tmp_path / "tickets.cu", tmp_path / "tickets"
+    src.write_text(PROGRAM)
+    cc = build.nvcc()
+    if subprocess.run([cc, "--version"], capture_output=True).returncode != 0:
+        pytest.skip("no nvcc")
+    subprocess.run([cc, *build.ARCH, "-std=c++17", "-O1", "-I" + build.CSRC, "-I" + os.path.join(ROOT, "include"),
+                    str(src), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout
