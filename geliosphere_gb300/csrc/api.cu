@@ -164,12 +164,15 @@ __global__ void k_prepare(const gelio_sim_params *__restrict__ p, int n, SimDev 
     int *idx = g.sim_idx + (size_t)m * n;
     unsigned long long *pre = g.prefix + (size_t)m * ((size_t)n * g.segs + 1);
     int c = 0;
+    bool alike = false;
     for (int i0 = 0; i0 < n; i0 += 32) {
       const bool mine = i0 + lane < n && p[i0 + lane].model == m;
+      alike |= mine && p[i0 + lane].n_particles > 0 && !lengths_differ(p[i0 + lane]);
       const unsigned b = __ballot_sync(kFull, mine);
       if (mine) idx[c + __popc(b & lanemask_lt())] = i0 + lane;
       c += __popc(b);
     }
+    if (__any_sync(kFull, alike) && lane == 0) ctl->alike[m] = 1u;
     __syncwarp();
     const int ne = c * g.segs;
     unsigned long long acc = 0;

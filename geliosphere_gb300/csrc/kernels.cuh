@@ -41,6 +41,7 @@ struct Control {
   int pad;
   unsigned long long group_count[4];
   unsigned long long t_start;      // %globaltimer when the prepare kernel ran
+  unsigned int alike[4];           // a simulation of the model has trajectories of like lengths
 };
 
 // Simulation grouping by model, written by the prepare kernel.
@@ -66,6 +67,20 @@ inline int ticket_segments(int n_sims) {
   const int s = kMaxSegEntries / n_sims;
   return s > 16 ? 16 : (s < 1 ? 1 : s);
 }
+// Whether a simulation has a few trajectories much longer than most (what place goes
+// by): a wide range of energies, and not only below 0.1 GeV, where lengths hardly
+// depend on them.  A logarithmic grid hands out its lowest ones first; a random
+// injection at any time, so that it takes a wider range.  Speed of 116,000
+// trajectories from 1 AU on four warps an SM, times that on all, 2D Geliosphere and
+// 1D B-p: grid 0.1-3 GeV 1.09 and 1.01, 0.01-0.3 GeV 0.83 and 0.69; log-uniform
+// 0.1-30 GeV 0.88 and 0.97, 0.01-3 GeV 0.83 and 0.74; uniform to 5 GeV 1.05 and
+// 1.12, to 1 GeV 0.96 and 0.82; one energy 0.67 and 0.74.
+__host__ __device__ __forceinline__ bool lengths_differ(const gelio_sim_params &p) {
+  if (p.injection == GELIO_INJ_LOG_GRID) return p.inj_points > 1 && p.inj_max >= 30.0f * fmaxf(p.inj_min, 0.06f);
+  if (p.injection == GELIO_INJ_LOG_UNIFORM) return p.inj_max >= 300.0f * fmaxf(p.inj_min, 0.1f);
+  return p.injection == GELIO_INJ_SOLARPROP_GRID || p.injection_max >= 5.0f;
+}
+
 // First ticket of segment s of a simulation of n particles.
 __host__ __device__ __forceinline__ unsigned long long segment_first(unsigned long long n, int s, int segs) {
   const unsigned long long q = n / (unsigned)segs, r = n % (unsigned)segs;
@@ -542,9 +557,10 @@ __device__ __forceinline__ int find_group_index(const unsigned long long *prefix
 //    32 to the warp that asked first they sat on 16 SMs), 4,001 1D B-p
 //    trajectories in FP64 steps 1,205 -> 849 ms; 5,000 in FP32 steps 47 ms, on a
 //    quarter of the warps 58.
-//  * From there on, FP32 steps take as few warps of each SM, in fours (one a
-//    scheduler), as leave a lane 6 trajectories or fewer: the long chains, which
-//    start first, run alone for longer, and a lane's later trajectories fill the
+//  * From there on, FP32 steps whose simulations all have a few long trajectories
+//    among many (lengths_differ; else ctas_per_sm is 0 here) take as few warps of
+//    each SM, in fours (one a scheduler), as leave a lane 6 trajectories or fewer:
+//    the long chains run alone for longer, and a lane's later trajectories fill the
 //    time.  On 4 / 8 / 12 / 16 warps an SM, ms: 1D B-p 50,000 62.9 / 72 / 74 / 77,
 //    100,000 80 / 83 / 86 / 90, 200,000 135 / 101 / 98 / 109, 300,000 192 / 132 /
 //    121 / 126, 800,000 488 / 314 / 267 / 256; 2D Geliosphere 150,000 29.7 / 30.7 /
@@ -654,12 +670,14 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   __shared__ Placement pl;
   __shared__ unsigned s_slot[8], s_rank[8];
   __shared__ unsigned long long s_first;
+  __shared__ unsigned s_per_sm;
   if ((threadIdx.x & 31) == 0) {
     *qlen = 0;
     asm volatile("mov.u32 %0, %%warpid;" : "=r"(s_slot[warp]));
   }
   if (threadIdx.x == 0) {
-    pl = place<R>(gpre[ne], gridDim.x, warps, (unsigned)a.ctas_per_sm);
+    s_per_sm = a.ctl->alike[MODEL] ? 0u : (unsigned)a.ctas_per_sm;
+    pl = place<R>(gpre[ne], gridDim.x, warps, s_per_sm);
     s_first = atomicAdd(&a.ctl->ticket[MODEL], (unsigned long long)(pl.warps * pl.lanes));
   }
   __syncthreads();
@@ -738,7 +756,7 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
       if (!active && !drained) {
         unsigned long long t = base + __popc(need & lanemask_lt());
         if constexpr (MODEL == kModelGeliosphere) t = ticket_at(t, pl, gridDim.x);
-        else if (t < (unsigned long long)gridDim.x * blockDim.x) t = first_ticket<R>(t, total, gridDim.x, warps, (unsigned)a.ctas_per_sm);
+        else if (t < (unsigned long long)gridDim.x * blockDim.x) t = first_ticket<R>(t, total, gridDim.x, warps, s_per_sm);
         if (t < total) {
           const int g = find_group_index(gpre, ne, t);
           const int seg = g / gn;

@@ -1,0 +1,37 @@
+"""Runs whose trajectories are of like lengths use every warp: on a quarter of
+them, as runs with a few long ones among many do well to take, 116,000 such
+trajectories took longer than 150,000."""
+import pytest
+
+from geliosphere_gb300 import abi, make_sim
+from test_gpu_tickets import same
+
+pytestmark = pytest.mark.gpu
+
+ONE = dict(injection=abi.GELIO_INJ_LOG_GRID, inj_points=1)
+RANDOM = dict(injection=abi.GELIO_INJ_LOG_UNIFORM)
+
+
+@pytest.mark.parametrize("model,kw", [
+    (abi.GELIO_MODEL_2D_GELIOSPHERE, dict(ONE, inj_min=0.1, inj_max=0.1)),
+    (abi.GELIO_MODEL_2D_GELIOSPHERE, dict(RANDOM, inj_min=0.1, inj_max=0.2)),
+    (abi.GELIO_MODEL_1D_BP, dict(ONE, inj_min=1.0, inj_max=1.0)),
+])
+def test_fewer_trajectories_take_no_longer(engine, model, kw):
+    def ms(n):
+        sim = make_sim(model, n, seed=3, **kw)
+        return min(engine.run(sim).stats.kernel_ms for _ in range(4))
+
+    # 0.85 to 0.9 on all warps; 1.16 to 1.19 on four warps an SM against eight
+    assert ms(116_000) <= 1.05 * ms(150_000)
+
+
+# one simulation of like lengths decides for its launch's model, an empty one does not
+@pytest.mark.parametrize("counts", [[30_000, 60_000], [90_000, 0], [0, 60_000]])
+@pytest.mark.parametrize("model", [abi.GELIO_MODEL_2D_GELIOSPHERE, abi.GELIO_MODEL_1D_BP])
+def test_mixed_simulations_run_every_particle(engine, model, counts):
+    sims = [make_sim(model, counts[0], injection=abi.GELIO_INJ_LOG_GRID, inj_min=5.0, inj_max=200.0, inj_points=9, seed=1),
+            make_sim(model, counts[1], seed=2, **dict(ONE, inj_min=20.0, inj_max=20.0))]
+    for n, a, b in zip(counts, engine.run(sims).spectra, engine.run(sims, plain=True).spectra):
+        assert a.n_particles == n
+        same(a, b)

@@ -59,9 +59,37 @@ int main() {
 """
 
 
-def test_every_place_is_a_ticket(tmp_path):
+LENGTHS = r"""
+#include <cstdio>
+#include "kernels.cuh"
+using namespace gelio;
+
+static bool differ(int injection, float lo, float hi, int points) {
+  gelio_sim_params p{};
+  p.injection = injection; p.inj_min = lo; p.inj_max = p.injection_max = hi; p.inj_points = points;
+  return lengths_differ(p);
+}
+
+int main() {
+  const int lg = GELIO_INJ_LOG_GRID, lu = GELIO_INJ_LOG_UNIFORM, ru = GELIO_INJ_REFERENCE_UNIFORM, cu = GELIO_INJ_CPU_UNIFORM;
+  const bool wide = differ(lg, 0.01f, 100, 100) && differ(lg, 0.1f, 3.1f, 33) && differ(lg, 1, 100, 10) && differ(lu, 0.01f, 100, 1) &&
+                    differ(lu, 0.3f, 100, 1) && differ(ru, 0, 101, 1) && differ(cu, 0, 5, 1) && differ(GELIO_INJ_SOLARPROP_GRID, 0, 0, 0);
+  const bool narrow = differ(lg, 0.1f, 0.1f, 1) || differ(lg, 0.01f, 100, 1) || differ(lg, 50, 100, 7) || differ(lg, 0.01f, 0.3f, 33) ||
+                      differ(lg, 0.01f, 1, 33) || differ(lu, 0.01f, 3, 1) || differ(lu, 0.03f, 10, 1) || differ(ru, 0, 1, 1) || differ(cu, 0, 0.2f, 1);
+  // trajectories of like lengths take every warp
+  unsigned fewer = 0;
+  for (unsigned long long n = 1; n < 500000; n += 777) {
+    fewer += place<float>(n, 304, 8, 2).warps < 8;
+    if (place<float>(n, 304, 8, 0).warps != 8 || place<double>(n, 304, 8, 2).warps != 8) return 1;
+  }
+  puts(wide && !narrow && fewer > 0 ? "ok" : "no");
+}
+"""
+
+
+def run_program(tmp_path, text):
     src, exe = tmp_path / "tickets.cu", tmp_path / "tickets"
-    src.write_text(PROGRAM)
+    src.write_text(text)
     cc = build.nvcc()
     if subprocess.run([cc, "--version"], capture_output=True).returncode != 0:
         pytest.skip("no nvcc")
@@ -69,3 +97,12 @@ def test_every_place_is_a_ticket(tmp_path):
                     str(src), "-o", str(exe)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout
+
+
+def test_every_place_is_a_ticket(tmp_path):
+    run_program(tmp_path, PROGRAM)
+
+
+def test_which_simulations_go_on_fewer_warps(tmp_path):
+    """Those with a few trajectories much longer than most, by their injection."""
+    run_program(tmp_path, LENGTHS)
