@@ -557,27 +557,32 @@ __device__ __forceinline__ int find_group_index(const unsigned long long *prefix
 //    32 to the warp that asked first they sat on 16 SMs), 4,001 1D B-p
 //    trajectories in FP64 steps 1,205 -> 849 ms; 5,000 in FP32 steps 47 ms, on a
 //    quarter of the warps 58.
-//  * From there on, FP32 steps whose simulations all have a few long trajectories
-//    among many (lengths_differ; else ctas_per_sm is 0 here) take as few warps of
-//    each SM, in fours (one a scheduler), as leave a lane 6 trajectories or fewer:
-//    the long chains run alone for longer, and a lane's later trajectories fill the
-//    time.  On 4 / 8 / 12 / 16 warps an SM, ms: 1D B-p 50,000 62.9 / 72 / 74 / 77,
-//    100,000 80 / 83 / 86 / 90, 200,000 135 / 101 / 98 / 109, 300,000 192 / 132 /
-//    121 / 126, 800,000 488 / 314 / 267 / 256; 2D Geliosphere 150,000 29.7 / 30.7 /
-//    31.5 / 34.6, 300,000 40.9 / 33.0 / 34.7 / 36.0.
+//  * From there on, FP32 steps take as few warps of each SM, in fours (one a
+//    scheduler), as leave a lane `per_lane` trajectories or fewer, 6 where every
+//    simulation has a few long ones among many (lengths_differ): the long chains run
+//    alone for longer, and a lane's later trajectories fill the time.  On 4 / 8 /
+//    12 / 16 warps an SM, ms: 1D B-p 50,000 62.9 / 72 / 74 / 77, 100,000 80 / 83 /
+//    86 / 90, 200,000 135 / 101 / 98 / 109, 300,000 192 / 132 / 121 / 126, 800,000
+//    488 / 314 / 267 / 256; 2D Geliosphere 150,000 29.7 / 30.7 / 31.5 / 34.6,
+//    300,000 40.9 / 33.0 / 34.7 / 36.0.  2 where lengths are alike, since throughput
+//    decides: at 1 / 2 / 3 / 6, speed times that on all warps, trajectories of 0.1
+//    GeV, 2D Geliosphere 25,000 1.25 / 1.31 / 1.32 / 1.27, 50,000 1.12 / 1.09 / 0.94
+//    / 0.92, 116,000 1.01 / 1.01 / 0.95 / 0.71; B-p 50,000 1.19 / 1.19 / 0.95 / 0.96,
+//    116,000 0.98 / 1.01 / 0.95 / 0.70.
+__host__ __device__ constexpr unsigned trajectories_per_lane(bool alike) { return alike ? 2u : 6u; }
 struct Placement {
   unsigned warps, lanes;          // of each CTA; of each of those warps
   unsigned long long dealt;       // first places in the queue, one a lane
 };
 template <class R>
-__host__ __device__ __forceinline__ Placement place(unsigned long long total, unsigned ctas, unsigned warps, unsigned ctas_per_sm) {
+__host__ __device__ __forceinline__ Placement place(unsigned long long total, unsigned ctas, unsigned warps, unsigned ctas_per_sm, unsigned per_lane) {
   Placement p{warps, 32u, 0ull};
   const unsigned long long all = (unsigned long long)ctas * warps;
   if (total <= all * kCoopLanes<R>) {
     p.lanes = (unsigned)((total + all - 1) / all);
   } else if (sizeof(R) == 4 && ctas_per_sm > 0) {
     const unsigned long long four = (unsigned long long)(ctas / ctas_per_sm) * 4 * 32;   // lanes of four warps an SM
-    const unsigned long long fours = (total + 6 * four - 1) / (6 * four);
+    const unsigned long long fours = (total + per_lane * four - 1) / (per_lane * four);
     const unsigned long long w = (4 * fours + ctas_per_sm - 1) / ctas_per_sm;
     if (w < warps) p.warps = (unsigned)w;
   }
@@ -608,8 +613,9 @@ __host__ __device__ __forceinline__ unsigned long long ticket_at(unsigned long l
 // loop loses by the call (4 x 2.5 M 491.1 -> 498.8).
 template <class R>
 static __device__ __noinline__ unsigned long long first_ticket(unsigned long long at, unsigned long long total,
-                                                               unsigned ctas, unsigned warps, unsigned ctas_per_sm) {
-  return ticket_at(at, place<R>(total, ctas, warps, ctas_per_sm), ctas);
+                                                               unsigned ctas, unsigned warps, unsigned ctas_per_sm,
+                                                               unsigned per_lane) {
+  return ticket_at(at, place<R>(total, ctas, warps, ctas_per_sm, per_lane), ctas);
 }
 
 // Refill windows of a warp: at the first (1) its places are asked for already, and
@@ -670,14 +676,14 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
   __shared__ Placement pl;
   __shared__ unsigned s_slot[8], s_rank[8];
   __shared__ unsigned long long s_first;
-  __shared__ unsigned s_per_sm;
+  __shared__ unsigned s_per_lane;
   if ((threadIdx.x & 31) == 0) {
     *qlen = 0;
     asm volatile("mov.u32 %0, %%warpid;" : "=r"(s_slot[warp]));
   }
   if (threadIdx.x == 0) {
-    s_per_sm = a.ctl->alike[MODEL] ? 0u : (unsigned)a.ctas_per_sm;
-    pl = place<R>(gpre[ne], gridDim.x, warps, s_per_sm);
+    s_per_lane = trajectories_per_lane(a.ctl->alike[MODEL] != 0u);
+    pl = place<R>(gpre[ne], gridDim.x, warps, (unsigned)a.ctas_per_sm, s_per_lane);
     s_first = atomicAdd(&a.ctl->ticket[MODEL], (unsigned long long)(pl.warps * pl.lanes));
   }
   __syncthreads();
@@ -756,7 +762,7 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
       if (!active && !drained) {
         unsigned long long t = base + __popc(need & lanemask_lt());
         if constexpr (MODEL == kModelGeliosphere) t = ticket_at(t, pl, gridDim.x);
-        else if (t < (unsigned long long)gridDim.x * blockDim.x) t = first_ticket<R>(t, total, gridDim.x, warps, s_per_sm);
+        else if (t < (unsigned long long)gridDim.x * blockDim.x) t = first_ticket<R>(t, total, gridDim.x, warps, (unsigned)a.ctas_per_sm, s_per_lane);
         if (t < total) {
           const int g = find_group_index(gpre, ne, t);
           const int seg = g / gn;

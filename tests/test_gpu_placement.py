@@ -1,6 +1,6 @@
-"""Runs whose trajectories are of like lengths use every warp: on a quarter of
-them, as runs with a few long ones among many do well to take, 116,000 such
-trajectories took longer than 150,000."""
+"""Runs whose trajectories are of like lengths use every warp from two a lane on: on
+the quarter of them that runs with a few long ones among many do well to take,
+116,000 such trajectories took longer than 150,000."""
 import pytest
 
 from geliosphere_gb300 import abi, make_sim
@@ -22,7 +22,7 @@ def test_fewer_trajectories_take_no_longer(engine, model, kw):
         sim = make_sim(model, n, seed=3, **kw)
         return min(engine.run(sim).stats.kernel_ms for _ in range(4))
 
-    # 0.85 to 0.9 on all warps; 1.16 to 1.19 on four warps an SM against eight
+    # 0.85 to 0.9; 1.16 to 1.19 on four warps an SM against eight
     assert ms(116_000) <= 1.05 * ms(150_000)
 
 

@@ -17,8 +17,8 @@ PROGRAM = r"""
 #include "kernels.cuh"
 using namespace gelio;
 
-template <class R> int check(unsigned long long total, unsigned ctas, unsigned warps, unsigned per_sm) {
-  const Placement p = place<R>(total, ctas, warps, per_sm);
+template <class R> int check(unsigned long long total, unsigned ctas, unsigned warps, unsigned per_sm, bool alike) {
+  const Placement p = place<R>(total, ctas, warps, per_sm, trajectories_per_lane(alike));
   if (p.warps < 1 || p.warps > warps || p.lanes > 32 || (total && p.lanes < 1)) return 1;
   const unsigned long long places = total > p.dealt ? total : p.dealt;
   std::vector<char> seen(total, 0);
@@ -46,8 +46,8 @@ int main() {
   const unsigned long long totals[] = {0, 1, 2, 151, 152, 303, 305, 500, 2431, 2432, 2433, 9727, 9729, 19456, 19457, 38911,
                                        38913, 77823, 77824, 77825, 116736, 116737, 233473, 350209, 1000003};
   for (auto &s : shapes)
-    for (auto n : totals) {
-      const int f = check<float>(n, s[0], s[1], s[2]), d = check<double>(n, s[0], s[1], s[2]);
+    for (auto n : totals) for (int alike = 0; alike < 2; ++alike) {
+      const int f = check<float>(n, s[0], s[1], s[2], alike), d = check<double>(n, s[0], s[1], s[2], alike);
       if (f || d) { printf("total %llu ctas %u warps %u per sm %u: %d %d\n", n, s[0], s[1], s[2], f, d); return 1; }
     }
   unsigned w = 0;
@@ -76,13 +76,17 @@ int main() {
                     differ(lu, 0.3f, 100, 1) && differ(ru, 0, 101, 1) && differ(cu, 0, 5, 1) && differ(GELIO_INJ_SOLARPROP_GRID, 0, 0, 0);
   const bool narrow = differ(lg, 0.1f, 0.1f, 1) || differ(lg, 0.01f, 100, 1) || differ(lg, 50, 100, 7) || differ(lg, 0.01f, 0.3f, 33) ||
                       differ(lg, 0.01f, 1, 33) || differ(lu, 0.01f, 3, 1) || differ(lu, 0.03f, 10, 1) || differ(ru, 0, 1, 1) || differ(cu, 0, 0.2f, 1);
-  // trajectories of like lengths take every warp
-  unsigned fewer = 0;
-  for (unsigned long long n = 1; n < 500000; n += 777) {
-    fewer += place<float>(n, 304, 8, 2).warps < 8;
-    if (place<float>(n, 304, 8, 0).warps != 8 || place<double>(n, 304, 8, 2).warps != 8) return 1;
-  }
-  puts(wide && !narrow && fewer > 0 ? "ok" : "no");
+  // more than six (two) trajectories a lane only on all warps; FP64 steps and sample runs always
+  unsigned fewer[2] = {0, 0};
+  for (unsigned long long n = 1; n < 500000; n += 777)
+    for (int alike = 0; alike < 2; ++alike) {
+      const unsigned most = trajectories_per_lane(alike);
+      const Placement p = place<float>(n, 304, 8, 2, most);
+      if (p.warps < 8 && n > 304ull * p.warps * 32 * most) return 1;
+      fewer[alike] += p.warps < 8;
+      if (place<float>(n, 304, 8, 0, most).warps != 8 || place<double>(n, 304, 8, 2, most).warps != 8) return 2;
+    }
+  puts(wide && !narrow && fewer[0] > 2 * fewer[1] && fewer[1] > 0 ? "ok" : "no");
 }
 """
 
@@ -104,5 +108,6 @@ def test_every_place_is_a_ticket(tmp_path):
 
 
 def test_which_simulations_go_on_fewer_warps(tmp_path):
-    """Those with a few trajectories much longer than most, by their injection."""
+    """Those with a few trajectories much longer than most, by their injection; others
+    up to two trajectories a lane."""
     run_program(tmp_path, LENGTHS)
