@@ -859,8 +859,11 @@ static void touch_pages(void *p, size_t bytes) {
 // inputs of a batch, every member's layers run on it in one launch and
 // k_ensemble forms mean and std.  Few rows come back through the staging, the
 // error flag with them; many straight into the caller's arrays (through the
-// staging the host's two copies of 3.2 MB took 200 us of an 870 us call).
-int infer_sims(gelio_surrogate *s, const gelio_sim_params *sims, int n, size_t rows, double *ln_ratio,
+// staging the host's two copies of 3.2 MB took 200 us of an 870 us call), after
+// the flag has been looked at: a call that fails leaves the arrays as they were.
+// enqueue_infer_sims may return with work under way that reads or writes host
+// memory; infer_sims does not.
+int enqueue_infer_sims(gelio_surrogate *s, const gelio_sim_params *sims, int n, size_t rows, double *ln_ratio,
                double *ln_std) {
   const int E = (int)s->mem.size();
   const size_t stride = (rows + kTileM - 1) / kTileM * kTileM;
@@ -915,7 +918,8 @@ int infer_sims(gelio_surrogate *s, const gelio_sim_params *sims, int n, size_t r
   }
   SUR_TRY(launch_early(s, k_ensemble, (unsigned)((rows + 127) / 128), 128, 0, (const float *)s->d_py, E, (long long)rows,
                        (long long)stride, s->d_pstat, s->d_pstat + rows, (const unsigned *)s->error,
-                       reinterpret_cast<unsigned *>(s->d_pstat + 2 * rows)));
+                       staged ? reinterpret_cast<unsigned *>(s->d_pstat + 2 * rows)
+                              : reinterpret_cast<unsigned *>(s->h_pstage)));      // pinned: the kernel writes it
   SUR_TRY(cudaEventRecord(s->ev1, s->stream));
   const size_t bytes = rows * sizeof(double);
   if (staged) {
@@ -925,9 +929,6 @@ int infer_sims(gelio_surrogate *s, const gelio_sim_params *sims, int n, size_t r
     // (a copy into pages that no one has touched yet took 1.9 ms instead of 40 us)
     touch_pages(ln_ratio, bytes);
     if (ln_std) touch_pages(ln_std, bytes);
-    SUR_TRY(cudaMemcpyAsync(s->h_pstage, s->d_pstat + 2 * rows, down, cudaMemcpyDeviceToHost, s->stream));
-    SUR_TRY(cudaMemcpyAsync(ln_ratio, s->d_pstat, bytes, cudaMemcpyDeviceToHost, s->stream));
-    if (ln_std) SUR_TRY(cudaMemcpyAsync(ln_std, s->d_pstat + rows, bytes, cudaMemcpyDeviceToHost, s->stream));
   }
   SUR_TRY(cudaStreamSynchronize(s->stream));
   unsigned error = 0;
@@ -936,12 +937,34 @@ int infer_sims(gelio_surrogate *s, const gelio_sim_params *sims, int n, size_t r
   if (staged) {
     std::memcpy(ln_ratio, s->h_pstage, bytes);
     if (ln_std) std::memcpy(ln_std, s->h_pstage + bytes, bytes);
+  } else {
+    SUR_TRY(cudaMemcpyAsync(ln_ratio, s->d_pstat, bytes, cudaMemcpyDeviceToHost, s->stream));
+    if (ln_std) SUR_TRY(cudaMemcpyAsync(ln_std, s->d_pstat + rows, bytes, cudaMemcpyDeviceToHost, s->stream));
+    SUR_TRY(cudaStreamSynchronize(s->stream));
   }
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, s->ev0, s->ev1) == cudaSuccess) {
     s->last_ms = ms;
     s->last_flop = gemm_flop(padded, (size_t)E);
   }
+  return GELIO_OK;
+}
+
+int infer_sims(gelio_surrogate *s, const gelio_sim_params *sims, int n, size_t rows, double *ln_ratio,
+               double *ln_std) {
+  const int rc = enqueue_infer_sims(s, sims, n, rows, ln_ratio, ln_std);
+  if (rc != GELIO_OK) cudaStreamSynchronize(s->stream);
+  return rc;
+}
+
+// For tests of calls that fail: sets the device's error flag, as a kernel does
+// one of whose waits ran out.
+int32_t gelio_internal_surrogate_error(gelio_surrogate *s, uint32_t code) {
+  if (!s) return GELIO_ERR_INVALID_ARGUMENT;
+  std::lock_guard<std::mutex> lock(s->mu);
+  SUR_TRY(cudaSetDevice(s->device));
+  SUR_TRY(cudaMemcpyAsync(s->error, &code, sizeof(code), cudaMemcpyHostToDevice, s->stream));
+  SUR_TRY(cudaStreamSynchronize(s->stream));
   return GELIO_OK;
 }
 
