@@ -468,7 +468,6 @@ struct gelio_ctx {
   int device = 0;
   int sm_count = 0;
   int max_smem_optin = 0;
-  std::atomic<int> tuning{0};          // autotunes under way
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_k0 = nullptr, ev_k1 = nullptr;
   cudaStream_t copy_stream = nullptr, eval_stream = nullptr;   // gelio_evaluate: rows on their way up, every other piece
@@ -784,9 +783,10 @@ int32_t gelio_destroy(gelio_ctx *c) {
 
 // Enqueue one run on `st`.  d_params already holds n sims.  model_mask /
 // counts are known for host runs (mask 0 = unknown: launch all four models).
+// all_warps: at any size (gelio_autotune's samples, which stand for larger runs).
 static int enqueue_run(gelio_ctx *c, int n, const gelio_run_opts *o, double *d_out, cudaStream_t st,
                        unsigned model_mask, const int *model_counts, gelio_exit_record *d_rec,
-                       size_t rec_cap, bool timed) {
+                       size_t rec_cap, bool timed, bool all_warps = false) {
   const int prec = (o && o->precision == GELIO_PREC_FP64) ? 1 : 0;
   const int n_slices = choose_slices(n);
   (void)cudaGetLastError();   // launch checks below must see only this run's errors
@@ -842,7 +842,7 @@ static int enqueue_run(gelio_ctx *c, int n, const gelio_run_opts *o, double *d_o
     if (rc != GELIO_OK) return rc;
     a.smem_slots = s.smem_slots;
     a.refill = s.refill;
-    a.ctas_per_sm = c->tuning > 0 ? 0 : s.blocks_per_sm;
+    a.ctas_per_sm = all_warps ? 0 : s.blocks_per_sm;
     GELIO_TRY(launch_model(m, true, variant, s.grid, s.block, s.smem, st, a));
     if (!have_first) { first = s; have_first = true; }
   }
@@ -869,10 +869,8 @@ static int check_opts(const gelio_run_opts *o) {
   return GELIO_OK;
 }
 
-extern "C" {
-
-int32_t gelio_run(gelio_ctx *c, const gelio_sim_params *sims, int32_t n, const gelio_run_opts *o,
-                  gelio_spectra *out, gelio_run_stats *stats) {
+static int run_sims(gelio_ctx *c, const gelio_sim_params *sims, int32_t n, const gelio_run_opts *o,
+                    gelio_spectra *out, gelio_run_stats *stats, bool all_warps) {
   const auto t0 = std::chrono::steady_clock::now();
   if (!c || (n > 0 && (!sims || !out)) || n < 0 || n > kMaxSims) return GELIO_ERR_INVALID_ARGUMENT;
   int rc = check_opts(o);
@@ -898,7 +896,7 @@ int32_t gelio_run(gelio_ctx *c, const gelio_sim_params *sims, int32_t n, const g
     c->rec_cap = rec_cap;
   }
   cudaStream_t st = c->stream;
-  const bool graph = o && o->use_graph && !(o->plain);
+  const bool graph = o && o->use_graph && !o->plain && !all_warps;   // (the key does not hold all_warps)
   const unsigned long long key[8] = {(unsigned long long)n, mask,
     (unsigned long long)(o ? o->precision : 0) | ((unsigned long long)(o ? o->compact : 0) << 8),
     (unsigned long long)(o ? o->block_size : 0) << 32 | (unsigned)(o ? o->blocks_per_sm : 0),
@@ -943,7 +941,7 @@ int32_t gelio_run(gelio_ctx *c, const gelio_sim_params *sims, int32_t n, const g
     GELIO_TRY(cudaGraphLaunch(c->graph, st));
   } else {
     GELIO_TRY(cudaMemcpyAsync(c->d_params, c->h_params, sizeof(gelio_sim_params) * n, cudaMemcpyHostToDevice, st));
-    rc = enqueue_run(c, n, o, c->d_out, st, mask, counts, rec_cap ? c->d_rec : nullptr, rec_cap, true);
+    rc = enqueue_run(c, n, o, c->d_out, st, mask, counts, rec_cap ? c->d_rec : nullptr, rec_cap, true, all_warps);
     if (rc != GELIO_OK) { cudaStreamSynchronize(st); return rc; }
     GELIO_TRY(cudaMemcpyAsync(out, c->d_out, sizeof(gelio_spectra) * n, cudaMemcpyDeviceToHost, st));
   }
@@ -983,6 +981,13 @@ int32_t gelio_run(gelio_ctx *c, const gelio_sim_params *sims, int32_t n, const g
   if (s.n_records_dropped > 0) return GELIO_WARN_RECORDS_TRUNCATED;
   if (s.n_step_capped > 0) return GELIO_WARN_STEP_CAP;
   return GELIO_OK;
+}
+
+extern "C" {
+
+int32_t gelio_run(gelio_ctx *c, const gelio_sim_params *sims, int32_t n, const gelio_run_opts *o,
+                  gelio_spectra *out, gelio_run_stats *stats) {
+  return run_sims(c, sims, n, o, out, stats, false);
 }
 
 int32_t gelio_run_async(gelio_ctx *c, const gelio_sim_params *d_sims, int32_t n, const gelio_run_opts *o,
@@ -1190,17 +1195,12 @@ int32_t gelio_autotune(gelio_ctx *c, const gelio_sim_params *sims, int32_t n, ge
   gelio_run_opts bo{};
   // a sample stands for a larger run: it is timed on all warps (on the few that
   // a sample of its size would take, the shapes hardly differ)
-  struct Tuning {
-    std::atomic<int> &n;
-    explicit Tuning(std::atomic<int> &n_) : n(n_) { ++n; }
-    ~Tuning() { --n; }
-  } tuning(c->tuning);
   std::vector<gelio_spectra> tmp(n);
   // one untimed run first (lazy allocations), then every shape once
   {
     gelio_run_opts o{};
     gelio_run_stats s{};
-    rc = gelio_run(c, sims, n, &o, tmp.data(), &s);
+    rc = run_sims(c, sims, n, &o, tmp.data(), &s, true);
     if (rc != GELIO_OK && rc < GELIO_WARN_FIRST) return rc;
   }
   for (int ci = 0; ci < 2; ++ci)
@@ -1211,7 +1211,7 @@ int32_t gelio_autotune(gelio_ctx *c, const gelio_sim_params *sims, int32_t n, ge
       o.block_size = blocks[bi];
       o.refill_interval = refills[ri];
       gelio_run_stats s{};
-      rc = gelio_run(c, sims, n, &o, tmp.data(), &s);
+      rc = run_sims(c, sims, n, &o, tmp.data(), &s, true);
       if (rc != GELIO_OK && rc < GELIO_WARN_FIRST) return rc;
       const double rate = (s.kernel_ms > 0.0) ? (double)s.n_steps / s.kernel_ms : 0.0;
       // as fast on the sample, the smaller register budget is faster on more
