@@ -1214,11 +1214,7 @@ int32_t gelio_autotune(gelio_ctx *c, const gelio_sim_params *sims, int32_t n, ge
       rc = run_sims(c, sims, n, &o, tmp.data(), &s, true);
       if (rc != GELIO_OK && rc < GELIO_WARN_FIRST) return rc;
       const double rate = (s.kernel_ms > 0.0) ? (double)s.n_steps / s.kernel_ms : 0.0;
-      // as fast on the sample, the smaller register budget is faster on more
-      // trajectories, once the sample's end no longer hides it (2D Geliosphere
-      // from 1 AU: 4 x 1 M 197.0 and 196.5 to 197.5 ms, 4 x 10 M 1,967 and 1,927)
-      const double bar = (ci == 1 && bo.compact == 1) ? 0.995 * best_rate : best_rate;
-      if (rate > bar) {
+      if (rate > best_rate) {
         best_rate = rate;
         bo = o;
         bo.blocks_per_sm = s.blocks_per_sm;
