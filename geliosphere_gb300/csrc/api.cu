@@ -304,7 +304,8 @@ __global__ void __launch_bounds__(kEvalBlock) k_evaluate_2d(const double *__rest
   __syncthreads();
   if (valid && s_bins[u] != 0u) {
     te = round6(te);
-    const double inv = 1.0 / (te * (te + kTwoT0)), ratio = s_p2[u] * inv;
+    // no momentum (NaN) for an exit energy of 0 and less, unless below -2 T0
+    const double p2 = te * (te + kTwoT0), inv = p2 <= 0.0 ? (double)NAN : 1.0 / p2, ratio = s_p2[u] * inv;
     const int pos = s_first[u] + rank;
     s_w[0][pos] = s_weber[u] * inv;
     s_w[1][pos] = lis_usoskin(te, log(te)) * ratio;
