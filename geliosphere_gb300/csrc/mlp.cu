@@ -324,10 +324,10 @@ int ensure_train(gelio_surrogate *s, int G) {
 }
 
 // All that a group of G members needs to train on nrow rows.  The staging of
-// the orders is plain memory where no pinned memory is to be had.
+// the orders is plain memory where no pinned memory is to be had.  The group's
+// buffers come last: where a part is refused, the smaller group that is tried
+// next has the memory of the larger one's buffers to itself.
 int ensure_group(gelio_surrogate *s, int G, int steps, size_t nrow) {
-  const int rc = ensure_train(s, G);
-  if (rc != GELIO_OK) return rc;
   const size_t n_loss = (size_t)G * steps, n_order = G * nrow;
   if (n_loss > s->step_loss_cap) {
     if (s->step_loss) cudaFree(s->step_loss);
@@ -353,7 +353,7 @@ int ensure_group(gelio_surrogate *s, int G, int steps, size_t nrow) {
     }
     s->h_order_cap = 2 * n_order;
   }
-  return GELIO_OK;
+  return ensure_train(s, G);
 }
 
 template <int MODE>
@@ -712,9 +712,9 @@ int32_t gelio_surrogate_create(gelio_ctx *ctx, const gelio_surrogate_opts *opts,
     }
   }
   if (rc != GELIO_OK) return fail(rc);
-  // one member's training memory is taken here: its allocations were 0.3 of the
-  // 1.3 ms of a first short training; a group's comes with its first training
-  if (group_size(s) == 1 && (rc = ensure_train(s, 1)) != GELIO_OK) return fail(rc);
+  // one member's training memory is taken here, so that a surrogate there is can
+  // be trained; a group's comes with its first training, where it is to be had
+  if ((rc = ensure_train(s, 1)) != GELIO_OK) return fail(rc);
   bool ok = make_map(&s->mQ0, s->Q0, kInPad, kQueryBatch, kTileM);
   ok = ok && make_map3(&s->tW1, s->W1, kInPad, kWidth, E, kWidth);
   for (int i = 0; i < 3; ++i)
