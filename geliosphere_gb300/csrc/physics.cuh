@@ -76,6 +76,13 @@ template <> struct Math<float> {
   __device__ static __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
   __device__ static __forceinline__ float mul_add(float a, float b, float c) { return __fadd_rn(__fmul_rn(a, b), c); }
   __device__ static __forceinline__ float max(float x, float y) { return fmaxf(x, y); }
+  // Sums with the contraction written out (SolarProp-like steps).  FP64 steps leave
+  // it to the compiler, which has one instance of them to make.
+  __device__ static __forceinline__ float sum(float a, float b) { return __fadd_rn(a, b); }            // both rounded before
+  __device__ static __forceinline__ float sum_of(float a, float b, float c) { return fmaf(a, b, c); }  // a b + c
+  // a b + c d, the first product not rounded by itself; the second
+  __device__ static __forceinline__ float sum_first(float a, float b, float c, float d) { return fmaf(a, b, __fmul_rn(c, d)); }
+  __device__ static __forceinline__ float sum_second(float a, float b, float c, float d) { return fmaf(c, d, __fmul_rn(a, b)); }
 };
 
 template <> struct Math<double> {
@@ -95,6 +102,10 @@ template <> struct Math<double> {
   __device__ static __forceinline__ double mul_add(double a, double b, double c) {
     return __dadd_rn(__dmul_rn(a, b), c);
   }
+  __device__ static __forceinline__ double sum(double a, double b) { return a + b; }
+  __device__ static __forceinline__ double sum_of(double a, double b, double c) { return a * b + c; }
+  __device__ static __forceinline__ double sum_first(double a, double b, double c, double d) { return a * b + c * d; }
+  __device__ static __forceinline__ double sum_second(double a, double b, double c, double d) { return a * b + c * d; }
 };
 
 // Kahan-compensated scalar: value v, running compensation c (true ~ v - c).
@@ -458,6 +469,10 @@ __device__ __forceinline__ int step_solarprop(Lane<R> &L, const Consts<R> &k, R 
   // Eq. 44: 2 r sqrt(g1) - r^2 tmp / (2 sqrt(g1)) = (2 r g1 - r^2 tmp / 2) / sqrt(g1) (and
   // the g1^1.5 form likewise); Eq. 18: T (T + 2 T0) / (T + T0) = P beta; dt and 1 / r applied
   // once to the summed terms of dr and dtheta.
+  //
+  // Which products of a sum are rounded by themselves is written out (M::sum...): left
+  // to the compiler it differed in the kernel of the smaller register budget from one
+  // build to the next, and with it the last bits of its paths.
   using M = Math<R>;
   const R r = L.r.v, T = L.T.v;
   const R th = theta_full(L);
@@ -472,7 +487,7 @@ __device__ __forceinline__ int step_solarprop(Lane<R> &L, const Consts<R> &k, R 
   const R P = M::sqrt(T * (Tp + T0));
   const R beta = P * M::rcp(Tp);
   const R bP = beta * P;
-  const R g1 = R(1) + gamma2;
+  const R g1 = M::sum(R(1), gamma2);
   const R inv_g1 = M::rcp(g1);
   const R sq1 = M::sqrt(g1);
   const R isq1 = M::rcp(sq1);
@@ -485,37 +500,36 @@ __device__ __forceinline__ int step_solarprop(Lane<R> &L, const Consts<R> &k, R 
   const R r2tmp = tr * r2 * k.ov2 * s * s;                                      // r^2 tmp, Eq. 44
   const R trg1 = tr * g1;
   const R kbr = k.K0 * bP * (R)(5.0 / (3.0 * (double)3.4f));                   // K0 beta P 5 / (3 * 3.4)
-  const R dKrr = kbr * (k.ratio * (trg1 - R(0.5) * r2tmp) * inv_g1_15
-                        + k.one_m_ratio * (trg1 - R(1.5) * r2tmp) * inv_g1_25);
+  const R dKrr_kbr = M::sum_first(k.ratio * M::sum_of(R(-0.5), r2tmp, trg1), inv_g1_15,
+                                  k.one_m_ratio * M::sum_of(R(-1.5), r2tmp, trg1), inv_g1_25);   // dKrr / kbr
   const R Pc = (P < (R)0.1f) ? (R)0.1f : P;
   const R Kpar = k.kpar_c * beta * Pc * r2isq;                                  // Eq. 42
   const R Kper = k.ratio * Kpar;                                                // Eq. 43
-  const R Krr = Kper + (Kpar - Kper) * inv_g1;                                  // Eq. 14
+  const R Krr = M::sum_of(M::sum(Kpar, -Kper), inv_g1, Kper);                                 // Eq. 14
   const R Ktt = Kper;                                                           // Eq. 15
   const R dt = k.dt;
   // Wavy current sheet drifts (Eq. 26, 32-37), as in the 2D Geliosphere step
-  const R xarg = k.alphaM + (R)(2.0 * (double)kPi / 180.0 * 0.0225 / (double)kA) * P * (r * isq1);
-  const R q = (R)kPi * M::rcp(M::sin(xarg)) - R(1);
+  const R xarg = M::sum_of((R)(2.0 * (double)kPi / 180.0 * 0.0225 / (double)kA) * P, r * isq1, k.alphaM);
+  const R q = M::sum_of((R)kPi, M::rcp(M::sin(xarg)), R(-1));
   const R alphaH = M::acos(M::rcp(q));
-  const R tanH = M::copysign(M::sqrt(q * q - R(1)), q);                      // tan(acos(1 / q))
+  const R tanH = M::copysign(M::sqrt(M::sum_of(q, q, R(-1))), q);                      // tan(acos(1 / q))
   const R inv_alphaH = M::rcp(alphaH);
-  const R arg = (R(1) + (R)(-2.0 / (double)kPi) * th) * tanH;
+  const R arg = M::sum_of((R)(-2.0 / (double)kPi), th, R(1)) * tanH;
   const R f = M::atan(arg) * inv_alphaH;
-  const R fprime = (R)(-2.0 / (double)kPi) * tanH * inv_alphaH * M::rcp(R(1) + arg * arg);
+  const R fprime = (R)(-2.0 / (double)kPi) * tanH * inv_alphaH * M::rcp(M::sum_of(arg, arg, R(1)));
   const R H = bP * r * gamma * inv_g1;                                          // P beta r gamma / g1
   const R D2 = H * f * inv_g1;
-  const R DriftR = k.drift2 * D2 * cot;                                         // Eq. 35
-  const R DriftSheetR = k.drift1 * H * fprime;                                  // Eq. 37
-  const R DriftTheta = k.dtheta_sp * D2 * (R(2) + gamma2);                      // Eq. 36
-  // Eq. 16-18
-  const R dr = (-k.V + dKrr + DriftR + DriftSheetR + R(2) * Krr * inv_r) * dt
-             + z0 * M::sqrt(R(2) * Krr * dt);
-  const R dth = dt * inv_r * (Ktt * cot * inv_r * inv_g1 + DriftTheta)
-              + z1 * M::sqrt(R(2) * Ktt * dt) * inv_r;
-  const R dT = -k.adv * bP * inv_r;
+  // Eq. 16-18; drifts: Eq. 35 (drift2 D2 cot), 37 (drift1 H fprime), 36 (dtheta_sp D2 (2 + gamma^2))
+  R det_r = M::sum_of(kbr, dKrr_kbr, -k.V);
+  det_r = M::sum_of(k.drift2 * D2, cot, det_r);
+  det_r = M::sum_of(k.drift1 * H, fprime, det_r);
+  det_r = M::sum_of(R(2) * Krr, inv_r, det_r);
+  const R det_th = M::sum_first(Ktt * cot * inv_r, inv_g1, k.dtheta_sp * D2, M::sum(R(2), gamma2));
+  const R dr = M::sum_second(det_r, dt, z0, M::sqrt(R(2) * Krr * dt));
+  const R dth = M::sum_second(dt * inv_r, det_th, z1 * M::sqrt(R(2) * Ktt * dt), inv_r);
   L.r.add(dr);
   theta_update(L, dth);
-  L.T.add(-dT);
+  L.T.add_product(k.adv * bP, inv_r);                                           // Eq. 18
   const bool rneg = L.r.v < R(0);
   L.r.v = rneg ? -L.r.v : L.r.v;
   L.r.c = rneg ? -L.r.c : L.r.c;
