@@ -1075,7 +1075,8 @@ int32_t gelio_evaluate(gelio_ctx *c, int32_t model, const double *rows, int64_t 
   memset(out, 0, sizeof(*out));
   if (n_rows == 0) return GELIO_OK;
   // few rows add straight into the result (a reduction and the clearing of 1 MB
-  // of slices cost more than their contention does)
+  // of slices cost more than their contention does): one / 16 slices, us, 2D 8,000
+  // rows 61 / 73, 32,000 70 / 81, F-p 32,000 81 / 79, 64,000 122 / 98
   const int n_slices = n_rows <= 32768 ? 1 : 16;
   GELIO_TRY(grow(c->d_part, c->part_bytes, (size_t)n_slices * kSpecDoubles * 8));
   GELIO_TRY(grow(c->d_out, c->out_bytes, sizeof(gelio_spectra)));

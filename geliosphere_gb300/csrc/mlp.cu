@@ -393,10 +393,12 @@ int train_step(gelio_surrogate *s, int m0, int G, int n_valid, UpdateArgs &u) {
   const int n_tile = 26 * G <= s->sm_count ? 64 : 128;
   const int items = G * 2 * (3 * (kWidth / n_tile) + 1), dw_grid = std::min(items, s->sm_count);
   // The class sums start as their sources come where the weight gradients leave
-  // them fewer than a third of the SMs (5 members of 16,384 rows, 24 steps:
-  // 10.49 -> 9.71 ms), else all at once beside those (a member of 4,096 rows,
-  // 48 steps, is bound by its launches: 5.87 ms, 6.05 with three more a step)
-  const bool early = 3 * dw_grid > 2 * s->sm_count;
+  // them fewer than three tenths of the SMs, else all at once beside those.  Four
+  // epochs of six batches, early / at once, ms: 5 members of 16,384 rows (130 of
+  // 152 SMs) 8.95 / 9.74, 8 of 4,096 (112) 5.24 / 5.52; 4 of 16,384 and of 4,096
+  // (104) 7.94 / 7.69 and 3.49 / 3.42, 1 of 4,096 (26; bound by its launches, three
+  // more a step) 2.99 / 2.90.
+  const bool early = 10 * dw_grid > 7 * s->sm_count;
   ClassSources c{};
   for (int li = 0; li < 4; ++li) c.src[li] = t.dH[li];
   c.src[4] = t.X[3];
@@ -870,7 +872,8 @@ int enqueue_infer_sims(gelio_surrogate *s, const gelio_sim_params *sims, int n, 
   // the simulations and their row offsets travel in one copy, so they share
   // one allocation (n * 96 bytes keeps the offsets 8-byte aligned)
   const size_t up = (size_t)n * sizeof(gelio_sim_params) + (size_t)(n + 1) * sizeof(long long);
-  constexpr size_t kStagedRows = 8192;
+  // staged / straight, us: 4,000 rows 65 / 77, 8,000 94 / 101, 16,000 118 / 122, 32,000 181 / 170
+  constexpr size_t kStagedRows = 16384;
   const bool staged = rows <= kStagedRows;
   const size_t down = (staged ? 2 * rows * sizeof(double) : 0) + sizeof(double);   // ... and the error flag
   int rc = GELIO_OK;

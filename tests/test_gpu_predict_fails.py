@@ -13,8 +13,8 @@ from test_surrogate_oracle import init_params
 pytestmark = pytest.mark.gpu
 
 
-# rows: through the staging (8,192 and fewer) and straight into the arrays
-@pytest.mark.parametrize("rows", [100, 8192, 8193, 50_000])
+# rows: through the staging (16,384 and fewer) and straight into the arrays
+@pytest.mark.parametrize("rows", [100, 8193, 16_384, 16_385, 50_000])
 def test_arrays_stay_as_they_were(engine, rows):
     s = sg.Surrogate(engine, members=2, batch_rows=256, seed=3)
     for m in range(2):
