@@ -514,7 +514,7 @@ def run_batch256(args, eng, rank, world, local):
             "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": " ".join(workload_batch256.__doc__.split()), "simulations": n,
                        "particles": total, "graph": True,
-                       "tuned": {"block": tune.block_size, "refill": tune.refill_interval} if tune else None,
+                       "tuned": {"block": tune.block_size, "refill": tune.refill_interval, "compact": tune.compact} if tune else None,
                        "l2": "flushed between timed steps (256 MiB write)"},
             "e2e": {"value": persistent, "unit": "trajectories/s",
                     "h2d_bytes_per_step": n * ctypes.sizeof(abi.SimParams),
@@ -604,6 +604,7 @@ def run_surrogate(args, eng, rank, world, local):
     weights, FP32 accumulation) trained on the GPU on MC spectra of random 2D
     simulations, evaluated on held-out draws against high-statistics MC:
     spectra/s of each, median |delta flux| over 0.1-10 GeV, fallback rate."""
+    import ctypes
     import numpy as np
     from geliosphere_gb300 import surrogate as sg
     chunk = 256
@@ -688,12 +689,12 @@ def run_surrogate(args, eng, rank, world, local):
             "train_loss": [float(v) for v in loss], "seconds": {"mc_training_data": t_data, "training": t_train,
                                                                  "mc_test": mc_s, "surrogate_predict": t_pred},
             "e2e": {"value": sur_rate, "unit": "spectra/s",
-                    "h2d_bytes_per_step": len(test) * 100 * 7 * 4,
-                    "d2h_bytes_per_step": len(test) * 100 * 5 * 4},
-            # the per-simulation query inputs; per 65,536-row inference batch the
-            # per-row inputs and the fused network (every member); the ensemble
-            # statistics
-            "gpu_launches": 2 * -(-len(test) * 100 // 65536) + 2,
+                    # the simulations and their row offsets; the ratio and its spread of every row
+                    "h2d_bytes_per_step": len(test) * ctypes.sizeof(abi.SimParams) + (len(test) + 1) * 8,
+                    "d2h_bytes_per_step": len(test) * 100 * 16},
+            # per 262,144-row inference batch the inputs and the fused network
+            # (every member); the ensemble statistics
+            "gpu_launches": 2 * -(-len(test) * 100 // 262144) + 1,
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": bf16_peak, "unit": "TFLOP/s",
                          "frac": achieved / bf16_peak, "traffic": None, "kernel": "k_mlp_infer_fused (tcgen05, all layers and members in one launch)",
                          "device_ms": dev_ms, "flop": flop,
@@ -710,6 +711,7 @@ def run_surrogate_infer(args, eng, rank, world, local):
     x 100 log-grid points, every step.  value = spectra/s of predict through
     the C ABI (host parameters in, host ratios and spread out); the roofline
     is the fused network kernel's FLOP over the device time of each predict."""
+    import ctypes
     import numpy as np
     from geliosphere_gb300 import abi
     from geliosphere_gb300 import surrogate as sg
@@ -755,9 +757,10 @@ def run_surrogate_infer(args, eng, rank, world, local):
             "config": {"workload": " ".join(run_surrogate_infer.__doc__.split()), "members": members,
                        "simulations": n, "rows": rows},
             "device_ms_per_step": dev_ms, "wall_over_device": 1e3 * wall / dev_ms,
-            "e2e": {"value": world * n / wall, "unit": "spectra/s", "h2d_bytes_per_step": n * 96,
+            "e2e": {"value": world * n / wall, "unit": "spectra/s",
+                    "h2d_bytes_per_step": n * ctypes.sizeof(abi.SimParams) + (n + 1) * 8,
                     "d2h_bytes_per_step": rows * 16},
-            "gpu_launches": (2 * -(-rows // 65536) + 2) * args.steps,
+            "gpu_launches": (2 * -(-rows // 262144) + 1) * args.steps,
             "roofline": {"bound": "tensor", "achieved": achieved, "peak": bf16_peak, "unit": "TFLOP/s",
                          "frac": achieved / bf16_peak, "traffic": None,
                          "kernel": "k_mlp_infer_fused (tcgen05, all layers and members in one launch)",
@@ -950,7 +953,7 @@ def main():
         "dtype": "f32",
         "data": "synthetic",
         "config": headline_config(args.particles),
-        "tuned": {"block": tune.block_size, "refill": tune.refill_interval} if tune else None,
+        "tuned": {"block": tune.block_size, "refill": tune.refill_interval, "compact": tune.compact} if tune else None,
         "particle_steps_per_s": steps_per_s,
         "e2e": {"value": e2e_value, "unit": "trajectories/s",
                 "h2d_bytes_per_step": n * ctypes.sizeof(abi.SimParams),
