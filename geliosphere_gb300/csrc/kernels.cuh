@@ -52,8 +52,9 @@ struct Control {
 // its longest trajectories (ticket_particle below), so every simulation's
 // long trajectories start in the first 1 / segs of the run.  One simulation
 // after another, the last one's started when the others were done and the run
-// ended on them: 4 x 250,000 2D Geliosphere particles 75 ms, now 62 (the
-// kernel's full rate needs 51); a batch of 48 uneven rows, 3 M particles, 135 -> 117.
+// ended on them: 4 x 250,000 2D Geliosphere particles 75 -> 62 ms (57 now; the
+// kernel's full rate needs 49); a batch of 48 uneven rows, 3 M particles, 135 -> 117
+// (113 now).
 struct Groups {
   int *sim_idx;                   // [4][n_sims]: simulation indices of model m
   unsigned long long *prefix;     // [4][n_sims * segs + 1]: entry (segment, simulation of the group)
@@ -554,9 +555,9 @@ __device__ __forceinline__ int find_group_index(const unsigned long long *prefix
 //  * Few trajectories are spread over all warps, as many lanes in each as it
 //    needs: while that is so few that a warp draws their normals together
 //    (kCoopLanes).  4,096 2D Geliosphere trajectories 19.7 -> 16.3 ms (handed out
-//    32 to the warp that asked first they sat on 16 SMs), 4,001 1D B-p
-//    trajectories in FP64 steps 1,205 -> 849 ms; 5,000 in FP32 steps 47 ms, on a
-//    quarter of the warps 58.
+//    32 to the warp that asked first they sat on 16 SMs; 11.8 now, with the tail's
+//    draws), 4,001 1D B-p trajectories in FP64 steps 1,205 -> 849 ms (303 now, with
+//    quiet groups); 5,000 in FP32 steps 47 ms, on a quarter of the warps 58.
 //  * From there on, FP32 steps take as few warps of each SM, in fours (one a
 //    scheduler), as leave a lane `per_lane` trajectories or fewer, 6 where every
 //    simulation has a few long ones among many (lengths_differ): the long chains run
@@ -842,8 +843,9 @@ __global__ void __launch_bounds__(256, MINB) k_persistent(const KArgs a) {
     // overlap).  A lane at an event repeats its group while its warp waits:
     // rare, since events are (B-p: ~10^-4 of the steps).  With the energy
     // formed only at a record, kept round keys and B-p's tail drawn by the
-    // warp: B-p 400,000 particles 227 -> 156 ms (258 -> 378 G steps/s), 4,001
-    // in FP64 steps 849 -> 440 ms, F-p 10^6 particles 116 -> 44 ms.
+    // warp: B-p 400,000 particles 227 -> 156 ms (149 now), 4,001 in FP64 steps 849
+    // -> 440 ms (303 now, the bounds off the FP64 pipe and 16 lanes' draws by the
+    // warp), F-p 10^6 particles 116 -> 44 ms (38 now).
     auto group_1d = [&](const R *z) {
       if constexpr (Prefetch<MODEL>::value) {
         if (L.steps + 4u < cap32 && four_quiet_steps<MODEL, R>(L, K, z)) {

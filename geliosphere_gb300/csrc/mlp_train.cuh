@@ -5,8 +5,8 @@
 // m0..m0+G-1 of the ensemble), every activation buffer is [G][rows][256].
 // One member alone fills neither the SMs (128 row tiles of a 16,384-row batch)
 // nor hides the launches: 27 launches and 410 us a step and member at 16,384
-// rows, now 12 launches and 85 us a member for a group of five (200,000 rows,
-// 2 epochs: 49.2 -> 10.8 ms).
+// rows, now 15 launches (12 where the class sums go all at once) and 85 us a member
+// for a group of five (200,000 rows, 2 epochs: 49.2 -> 10.2 ms).
 //
 // All operands are row-major in HBM, written once:
 //   forward   Z_l  = X_{l-1} W_l^T    A = X_{l-1} [rows x in]   (K-major)  B = W_l   [256 x in]

@@ -170,7 +170,7 @@ extern "C" int32_t gelio_run_noalloc(const gelio_sim_params *d_sims, int32_t n_s
   Control *ctl = reinterpret_cast<Control *>(base + kOffCtl);
   SimDev *sims = reinterpret_cast<SimDev *>(base + kOffSims);
   float *tables = reinterpret_cast<float *>(base + kOffTables);
-  Groups g{reinterpret_cast<int *>(base + kOffGsim), reinterpret_cast<unsigned long long *>(base + kOffGpre), 1};   // one segment: the scratch holds n + 1 sums
+  Groups g{reinterpret_cast<int *>(base + kOffGsim), reinterpret_cast<unsigned long long *>(base + kOffGpre), 1};   // one segment: the scratch holds n + 1 sums, so simulation by simulation
   double *part = reinterpret_cast<double *>(base + kOffPart);
   const size_t part_bytes = sizeof(double) * (size_t)kSlices * n_sims * kSpecDoubles;
 
