@@ -599,7 +599,7 @@ __host__ __device__ __forceinline__ Placement place(unsigned long long total, un
 // B-p trajectories took 45.5 to 51 ms from one run to the next, 45.3 to 45.7 so.
 __device__ __forceinline__ void first_of_each_sm_first(unsigned ctas_per_sm) {
   const unsigned wave = ctas_per_sm > 1u ? blockIdx.x * ctas_per_sm / gridDim.x : 0u;
-  if (wave > 0u) __nanosleep(3000u * wave);
+  if (wave > 0u) __nanosleep(wave < 3u ? 3000u * wave : 9000u);      // (small blocks: many to an SM)
 }
 
 // Both out of line for the 2D models, whose step loops keep their registers' order so
